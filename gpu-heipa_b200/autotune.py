@@ -26,10 +26,10 @@ CANDIDATES = {
     "match_coop_max_m": [0, 1 << 19, 1 << 21, 1 << 23],
     "jet_fused_max_n": [0, 2048, 4096, 8192],
     "jet_fused_max_m": [1 << 16, 1 << 18, 1 << 20],
-    "jet_coop_max_n": [0, 16384, 65536],
-    "jet_coop_max_m": [1 << 19, 1 << 21, 1 << 23],
-    "jet_coop_max_deg": [16, 32, 64],
-    "jet_coop_rows": [512, 1024, 2048],
+    "jet_coop_max_n": [0, 65536, 1 << 20, 1 << 24],
+    "jet_coop_max_m": [1 << 21, 1 << 24, 1 << 27],
+    "jet_coop_max_deg": [12, 24, 64],
+    "jet_coop_rows": [256, 512, 1024],
     "jet_hub_deg": [256, 1024, 4096],
     "jet_hub_conn": [0, 1],
     "jet_hub_track_pct": [25, 50, 100],
@@ -38,8 +38,8 @@ CANDIDATES = {
     "jet_chunk_mode": [0, 1],
 }
 DEFAULTS = {"jet_graph_max_m": 1 << 24, "order_small_n": 16384, "match_coop_max_n": 1 << 17,
-            "match_coop_max_m": 1 << 21, "jet_fused_max_n": 4096, "jet_fused_max_m": 1 << 18,
-            "jet_coop_max_n": 65536, "jet_coop_max_m": 1 << 21, "jet_coop_max_deg": 32, "jet_coop_rows": 1024,
+            "match_coop_max_m": 1 << 21, "jet_fused_max_n": 8192, "jet_fused_max_m": 1 << 18,
+            "jet_coop_max_n": 1 << 24, "jet_coop_max_m": 1 << 27, "jet_coop_max_deg": 24, "jet_coop_rows": 512,
             "jet_hub_deg": 1024, "jet_hub_conn": 1, "jet_hub_track_pct": 50, "jet_inval_all_pct": 5,
             "jet_vec_loads": 1, "jet_chunk_mode": 0}
 

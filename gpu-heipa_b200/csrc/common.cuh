@@ -74,30 +74,42 @@ __host__ __device__ __forceinline__ u32 murmur3_u32(u32 key) {
     return h;
 }
 
+// a * 2^k <= b * 3^k for a, b < 2^32, p3 = 3^k < 2^39, k <= 24, in 64-bit words
+__host__ __device__ __forceinline__ bool pow15_reaches(u64 a, u64 b, u32 k, u64 p3) {
+    const u64 lo = b * (p3 & 0xFFFFFFFFull);
+    const u64 hi = b * (p3 >> 32) + (lo >> 32);  // b * p3 = hi * 2^32 + (lo mod 2^32)
+    const u64 x = a << k;
+    return hi > (x >> 32) || (hi == (x >> 32) && (lo & 0xFFFFFFFFull) >= (x & 0xFFFFFFFFull));
+}
+
 // gain_bucket (jet_label_propagation.h:147-180) as an exact integer rule:
 // with g = -gx / vwgt, g >= 1 -> 25 + min{k : 1.5^k >= g} (<= 49), and
-// g < 1 -> 25 - min{k : 1.5^k >= 1/g} (>= 2). 128-bit products keep it exact.
+// g < 1 -> 25 - min{k : 1.5^k >= 1/g} (>= 2). The smallest k is found by
+// bisection (1.5^k grows with k): five comparisons instead of up to 24, each
+// in 64-bit words.
 __host__ __device__ __forceinline__ u32 gain_bucket(s32 gx, s32 vwgt) {
     if (gx > 0) return 0;
     if (gx == 0) return 1;
-    unsigned __int128 a = (unsigned __int128) (u64) (-(s64) gx);
-    unsigned __int128 b = (unsigned __int128) (u64) (vwgt < 1 ? 1 : vwgt);
-    unsigned __int128 p2 = 1, p3 = 1;
+    const u64 a = (u64) (-(s64) gx), b = (u64) (vwgt < 1 ? 1 : vwgt);
+    const bool above = a >= b;
+    const u64 x = above ? a : b, y = above ? b : a;
     u32 k = 0;
-    if (a >= b) {
-        while (k < 24 && a * p2 > b * p3) {
-            ++k;
-            p2 *= 2;
-            p3 *= 3;
+    u64 p3 = 1;
+    // invariant: p3 = 3^k, and k = 0 or 1.5^(k - 1) < x / y; pows[i] = 3^(step - 1)
+    const u64 pows[5] = {14348907ull, 2187ull, 27ull, 3ull, 1ull};
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        const u32 step = 16u >> i;
+        const u32 kk = k + step;
+        if (kk > 24) continue;
+        const u64 q3 = p3 * pows[i];
+        if (!pow15_reaches(x, y, kk - 1, q3)) {
+            k = kk;
+            p3 = 3 * q3;
         }
-        return 25 + k;
     }
-    while (k < 23 && b * p2 > a * p3) {
-        ++k;
-        p2 *= 2;
-        p3 *= 3;
-    }
-    return 25 - k;
+    if (!above && k > 23) k = 23;
+    return above ? 25 + k : 25 - k;
 }
 
 // ---- warp helpers ------------------------------------------------------------

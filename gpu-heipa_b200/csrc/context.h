@@ -130,12 +130,12 @@ struct Tunables {
     u32 order_small_n = 16384;         // single-block rebalance ordering up to this many vertices
     u32 match_coop_max_n = 1u << 17;   // cooperative matching loop up to this many vertices ...
     u64 match_coop_max_m = 1ull << 21; // ... and entries
-    u32 jet_fused_max_n = 4096;        // whole Jet level loop in one block up to this many vertices ...
+    u32 jet_fused_max_n = 8192;        // whole Jet level loop in one thread-block cluster up to this many vertices ...
     u64 jet_fused_max_m = 1ull << 18;  // ... and entries
-    u32 jet_coop_max_n = 65536;        // ... else as a cooperative grid up to this many vertices ...
-    u64 jet_coop_max_m = 1ull << 21;   // ... and entries ...
-    u32 jet_coop_max_deg = 32;         // ... and average degree (dense levels keep the whole GPU)
-    u32 jet_coop_rows = 1024;          // vertices per block of that grid
+    u32 jet_coop_max_n = 1u << 24;     // ... else as a cooperative grid up to this many vertices ...
+    u64 jet_coop_max_m = 1ull << 27;   // ... and entries ...
+    u32 jet_coop_max_deg = 24;         // ... and average degree (smaller levels also above it: jet.cu)
+    u32 jet_coop_rows = 512;           // vertices per block of that grid
     u32 jet_hub_deg = 1024;            // Jet table passes: rows above this length are cut into chunks of it (64..4096)
     u32 jet_chunk_mode = 0;            // chunk kernels: 0 = 4 entries per lane, 1 = 8, 2 = bulk-copy staged rows
     u32 jet_hub_conn = 1;              // per-kernel Jet loop: keep hub-row connectivity up to date (1) or rescan (0)
@@ -163,6 +163,7 @@ struct Ctx {
     // and kept until destroy().
     std::vector<std::unique_ptr<Ctx> > workers;
     Ctx &worker(size_t i);
+    u32 peers = 1;  // contexts that run solves on the device beside this one (itself included)
 
     void init(int dev, size_t arena_bytes);
     void destroy();

@@ -45,6 +45,10 @@ constexpr unsigned long long DL_OLD = 0xFFFFull << DL_OLD_SHIFT;
 constexpr int DL_SLOT_SHIFT = 33;                             // tracked hub slot + 1 (0: not a tracked hub)
 constexpr u32 DL_MAX_HUBS = 0x7FFFFFFEu;
 
+// Direct-indexed block tables: k fits a table and, for the mapping objective
+// (whose candidate scoring loops over pairs of blocks), k is small.
+inline bool direct_tables(u32 k, bool promap) { return k <= JW_SLOTS && (!promap || k <= 256); }
+
 // Block-tier table size: a row never has more distinct blocks than k.
 inline u32 block_slots_for(u32 k) {
     u32 t = 64;
@@ -2034,389 +2038,9 @@ __global__ void __launch_bounds__(OB, 1) k_order_small(JArgs a, RbArgs r, u32 wi
     order_small_body<STRONG>(a, r, width, key_bits, S, max_b_w, sm);
 }
 
-// ---- fused refinement of small and mid-size levels --------------------------------------
+// ---- level loop of small and mid-size levels in one launch -------------------------------
 
-// The whole level loop of jet_refine in one launch of 1024-thread blocks: the
-// iteration control (ratios, weak/strong switching, best-labelling tracking)
-// and per iteration the same steps as the per-kernel path (gain pass, filter,
-// afterburner, weak or strong rebalancing with the one-block ordering,
-// perform). Levels of at most Tunables::jet_fused_max_n vertices run it in a
-// single block (phases separated by __syncthreads()); levels of at most
-// Tunables::jet_coop_max_n vertices run it as a cooperative grid (phases
-// separated by grid barriers; block 0 alone does the ordering). State written
-// in one phase is read in a later phase with plain loads after the barrier
-// (never through the non-coherent path). Every branch of the control flow
-// depends only on values all threads read after the same barrier, so every
-// thread reaches every barrier. The result equals the per-kernel path's (a
-// parity test forces both).
-constexpr int FB = OB;                  // threads per block (= the ordering block)
-constexpr u32 FUSED_MAX_N = 1u << 16;   // upper bound of both vertex thresholds (one-block ordering)
-constexpr u32 FUSED_AB_THREAD = 32;     // afterburner / delta rows handled by one thread
-constexpr int FC_N = 4;  // counters per set: warp rows, block rows, candidates, moves
-constexpr int FS_N = 2;  // sums per set: moved-row entries, objective delta
-
-struct FusedCtl {
-    u32 n_ratios;
-    u32 ratios[17];
-    s32 lmax;
-    u32 promap;
-    long long obj;  // in: objective of the input labelling; out: best objective
-    s32 maxw;       // in / out: maximum block weight
-    u32 iterations; // out: Jet iterations run
-};
-
-struct FusedArgs {
-    RbArgs weak, strong;
-    u32 width;
-    int bits_weak, bits_strong;
-    OrderScratch S;
-    u32 *under;       // writable alias of weak.under
-    u32 *part;        // receives the best labelling
-    u32 *gcnt;        // cooperative grid: 2 sets of FC_N counters (zero on entry)
-    long long *gsum;  // cooperative grid: 2 sets of FS_N sums (zero on entry)
-    u32 *bar;         // cooperative grid: barrier words (zero on entry)
-};
-
-// Barrier of the team: the block, or the cooperative grid (bounded wait;
-// false once a wait gave up).
-template<bool COOP>
-__device__ __forceinline__ bool team_sync(u32 *bar, u32 *err) {
-    if (COOP) return grid_barrier(bar, err);
-    __syncthreads();
-    return true;
-}
-
-// Loads a value that decides the control flow (counts, sums, block weights)
-// after a barrier: from L2 on a grid (global memory), a volatile load within
-// one block (shared or global memory), so every thread sees the same value.
-template<bool COOP, typename T>
-__device__ __forceinline__ T ld_team(const T *p) {
-    return COOP ? __ldcg(p) : *(const volatile T *) p;
-}
-
-__device__ __forceinline__ long long block_sum_ll(long long v, long long *sm) {
-    v = warp_sum<long long>(v);
-    if (lane_id() == 0) sm[warp_in_block()] = v;
-    __syncthreads();
-    long long r = 0;
-    if (threadIdx.x == 0) {
-        for (u32 w = 0; w < (blockDim.x >> 5); ++w) r += sm[w];
-        sm[32] = r;
-    }
-    __syncthreads();
-    r = sm[32];
-    __syncthreads();
-    return r;
-}
-
-// Adds v over all threads into *slot (zero beforehand), synchronises the team
-// and reads the total into out; false once a barrier wait gave up.
-template<bool COOP>
-__device__ __forceinline__ bool team_sum(long long v, long long *slot, long long *sm, u32 *bar, u32 *err,
-                                         long long &out) {
-    v = block_sum_ll(v, sm);
-    if (threadIdx.x == 0 && v) atomicAdd((unsigned long long *) slot, (unsigned long long) v);
-    if (!team_sync<COOP>(bar, err)) return false;
-    out = ld_team<COOP>(slot);
-    return true;
-}
-
-#define TEAM_SYNC()                                          \
-    do {                                                     \
-        if (!team_sync<COOP>(F.bar, &a.st->err)) goto finish; \
-    } while (0)
-
-template<bool COOP>
-__global__ void __launch_bounds__(FB, 1) k_jet_loop(JArgs a, FusedArgs F, FusedCtl *ctl) {
-    extern __shared__ s32 fsm[];
-    const u32 tid = threadIdx.x, lane = lane_id(), warp = warp_in_block(), n = a.g.n, k = a.k;
-    s32 *wtab = fsm + warp * k;  // per-warp direct table
-    s32 *btab = fsm + 32u * k;   // block table
-    s32 *sbd = fsm + 33u * k;    // block-weight changes of this block's moves
-    __shared__ u32 scnt[2 * FC_N];
-    __shared__ long long ssum[2 * FS_N];
-    __shared__ long long sl[33];
-    __shared__ unsigned long long smu[33];
-    __shared__ long long sms[33];
-    __shared__ s32 smx[32];
-    __shared__ OrderSmem osm;
-    for (u32 i = tid; i < 34u * k; i += FB) fsm[i] = 0;
-    if (!COOP && tid < 2 * FC_N) scnt[tid] = 0;
-    if (!COOP && tid < 2 * FS_N) ssum[tid] = 0;
-    __syncthreads();
-    u32 *const cnt_base = COOP ? F.gcnt : scnt;
-    long long *const sum_base = COOP ? F.gsum : ssum;
-    const u32 nthreads = gridDim.x * FB;
-    const u32 wbase0 = blockIdx.x * FB + warp * 32u;  // first row of this warp in grid-stride loops
-    const u32 gwarps = gridDim.x * (FB / 32), gw = blockIdx.x * (FB / 32) + warp;
-    const ConnTable<false, true, false> WT{nullptr, wtab, 0, k};
-    const ConnTable<true, true, false> BT{nullptr, btab, 0, k};
-    const bool promap = ctl->promap != 0;
-    const s32 lmax = ctl->lmax;
-    const u32 n_ratios = ctl->n_ratios;
-    long long obj = ctl->obj, best_obj = obj;
-    s32 maxw = ctl->maxw, best_max = maxw;
-    u32 iterations = 0, it = 0;
-    for (u32 ri = 0; ri < n_ratios; ++ri) {
-        const u32 ratio = ctl->ratios[ri];
-        u32 balance_iteration = 0, iteration = 0;
-        while (iteration < JET_MAX_ITERATIONS) {
-            iteration += 1;
-            ++iterations;
-            // counter set of this iteration (zero); the other set is cleared
-            // after the first barrier, when every thread is done reading it
-            const u32 set = it & 1u;
-            ++it;
-            u32 *const cnt = cnt_base + set * FC_N;
-            long long *const sum = sum_base + set * FS_N;
-            const bool clears = blockIdx.x == 0 && tid < (u32) FC_N;
-            bool lp_iter = false;
-            int step;
-            if (maxw <= lmax) {
-                step = 0;
-                lp_iter = true;
-                balance_iteration = 0;
-            } else if (!promap) {
-                step = balance_iteration < JET_MAX_WEAK_ITERATIONS ? 1 : 2;
-            } else {
-                balance_iteration++;
-                step = balance_iteration < JET_MAX_WEAK_ITERATIONS ? 1 : 2;
-            }
-            u32 nm;
-            if (step == 0) {
-                // gain pass (jet_lp :193-238): cached targets, else recompute
-                for (u32 wb = wbase0; wb < n; wb += nthreads) {
-                    const u32 u = wb + lane;
-                    int cls = -1;
-                    if (u < n) {
-                        const u32 dc = a.dest_cache[u];
-                        if (dc != NULL_PART) {
-                            a.dest_part[u] = dc;
-                        } else {
-                            cls = table_tier(a.g.rowlen[u], k);
-                            if (cls == 0) lp_thread<false>(a, u, ratio);
-                        }
-                    }
-                    const u32 s1 = warp_append(&cnt[0], cls == 1);
-                    if (cls == 1) a.heavy[s1] = u;
-                    const u32 s2 = warp_append(&cnt[1], cls == 2);
-                    if (cls == 2) a.heavy2[s2] = u;
-                }
-                TEAM_SYNC();
-                if (clears) cnt_base[(set ^ 1u) * FC_N + tid] = 0;
-                if (clears && tid < (u32) FS_N) sum_base[(set ^ 1u) * FS_N + tid] = 0;
-                const u32 n1 = ld_team<COOP>(&cnt[0]), n2 = ld_team<COOP>(&cnt[1]);
-                for (u32 i = gw; i < n1; i += gwarps) lp_group<false, true, false>(a, a.heavy[i], ratio, WT, nullptr, nullptr);
-                for (u32 i = blockIdx.x; i < n2; i += gridDim.x) lp_group<true, true, false>(a, a.heavy2[i], ratio, BT, smu, sms);
-                TEAM_SYNC();
-                // filter (:247-258)
-                for (u32 wb = wbase0; wb < n; wb += nthreads) {
-                    const u32 u = wb + lane;
-                    bool c = false;
-                    if (u < n) {
-                        c = a.dest_part[u] != NO_MOVE && a.lock[u] == 0;
-                        if (c) {
-                            a.gain1[u] = a.gain_cache[u];
-                        } else {
-                            a.gain1[u] = GAIN_MIN;
-                            a.lock[u] = 0;
-                        }
-                    }
-                    const u32 s3 = warp_append(&cnt[2], c);
-                    if (c) a.cand[s3] = u;
-                }
-                TEAM_SYNC();
-                // afterburner: short rows by a thread, longer ones by the whole warp
-                const u32 nc = ld_team<COOP>(&cnt[2]);
-                for (u32 wb = wbase0; wb < nc; wb += nthreads) {
-                    const u32 i = wb + lane;
-                    u32 u = 0, len = 0;
-                    bool lock = false;
-                    if (i < nc) {
-                        u = a.cand[i];
-                        len = a.g.rowlen[u];
-                        if (len <= FUSED_AB_THREAD) {
-                            const s32 ug = a.gain1[u];
-                            lock = wadd(ug, ab_range<false>(a, u, ug, a.map[u], a.dest_part[u], 0, len, 0, 1)) >= 0;
-                        }
-                    }
-                    unsigned longer = __ballot_sync(FULL, i < nc && len > FUSED_AB_THREAD);
-                    while (longer) {
-                        const int src = __ffs(longer) - 1;
-                        longer &= longer - 1;
-                        const u32 v = __shfl_sync(FULL, u, src), lv = __shfl_sync(FULL, len, src);
-                        const s32 vg = a.gain1[v];
-                        const s32 change = (s32) warp_sum<u32>(
-                            (u32) ab_range<false>(a, v, vg, a.map[v], a.dest_part[v], 0, lv, lane, 32));
-                        if (lane == (u32) src) lock = wadd(vg, change) >= 0;
-                    }
-                    if (lock) a.lock[u] = 1;
-                    const u32 s4 = warp_append(&cnt[3], lock);
-                    if (lock) a.moves[s4] = u;
-                }
-                TEAM_SYNC();
-                nm = ld_team<COOP>(&cnt[3]);
-            } else {
-                // rebalancing picks (rebalance_weak :592-751 / rebalance_strong :356-590)
-                const bool strong = step == 2;
-                const RbArgs &r = strong ? F.strong : F.weak;
-                if (blockIdx.x == 0) {
-                    if (strong) maxv_block(a.bw, k, r.max_b_w, &a.st->imax[1]);
-                    else under_block(a.bw, k, r.max_b_w, F.under, &a.st->cnt[ST_AUX]);
-                }
-                TEAM_SYNC();
-                if (clears) cnt_base[(set ^ 1u) * FC_N + tid] = 0;
-                if (clears && tid < (u32) FS_N) sum_base[(set ^ 1u) * FS_N + tid] = 0;
-                const s32 maxv = ld_team<COOP>(&a.st->imax[1]);
-                for (u32 wb = wbase0; wb < n; wb += nthreads) {
-                    const u32 u = wb + lane;
-                    int cls = -1;
-                    if (u < n) {
-                        const u32 o = a.map[u];
-                        const bool q = strong ? rb_qualifies<true>(a, r, o, g_vw(a.g, u), maxv)
-                                              : rb_qualifies<false>(a, r, o, g_vw(a.g, u), maxv);
-                        if (!q) {
-                            if (!strong) a.dest_part[u] = o;
-                            r.keys[u] = NOKEY;
-                        } else {
-                            cls = table_tier(a.g.rowlen[u], k);
-                            if (cls == 0) {
-                                if (strong) rb_thread<true, false>(a, r, u, o);
-                                else rb_thread<false, false>(a, r, u, o);
-                            }
-                        }
-                    }
-                    const u32 s1 = warp_append(&cnt[0], cls == 1);
-                    if (cls == 1) a.heavy[s1] = u;
-                    const u32 s2 = warp_append(&cnt[1], cls == 2);
-                    if (cls == 2) a.heavy2[s2] = u;
-                }
-                TEAM_SYNC();
-                const u32 n1 = ld_team<COOP>(&cnt[0]), n2 = ld_team<COOP>(&cnt[1]);
-                for (u32 i = gw; i < n1; i += gwarps) {
-                    if (strong) rb_group<true, false, true, false>(a, r, a.heavy[i], WT, nullptr, nullptr);
-                    else rb_group<false, false, true, false>(a, r, a.heavy[i], WT, nullptr, nullptr);
-                }
-                for (u32 i = blockIdx.x; i < n2; i += gridDim.x) {
-                    if (strong) rb_group<true, true, true, false>(a, r, a.heavy2[i], BT, smu, sms);
-                    else rb_group<false, true, true, false>(a, r, a.heavy2[i], BT, smu, sms);
-                }
-                TEAM_SYNC();
-                if (blockIdx.x == 0) {
-                    if (strong) order_small_body<true>(a, r, F.width, F.bits_strong, F.S, r.max_b_w, osm);
-                    else order_small_body<false>(a, r, F.width, F.bits_weak, F.S, r.max_b_w, osm);
-                }
-                TEAM_SYNC();
-                nm = ld_team<COOP>(&a.st->cnt[ST_MOVES]);
-            }
-            // perform_moves (:753-924): labels with the moved bit, block weights
-            long long entries = 0;
-            for (u32 i = blockIdx.x * FB + tid; i < nm; i += nthreads) {
-                const u32 u = a.moves[i];
-                const u32 ou = a.map[u], nu = a.dest_part[u];
-                const s32 w = g_vw(a.g, u);
-                if (ou != nu) {
-                    atomicSub(&sbd[ou], w);
-                    atomicAdd(&sbd[nu], w);
-                }
-                a.map[u] = ou != nu ? (nu | MOVED) : nu;
-                a.dest_part[u] = ou;
-                a.dest_cache[u] = NULL_PART;
-                entries += a.g.rowlen[u];
-            }
-            __syncthreads();
-            for (u32 b = tid; b < k; b += FB)
-                if (sbd[b]) {
-                    atomicAdd(&a.bw[b], sbd[b]);
-                    sbd[b] = 0;
-                }
-            long long ent = 0;
-            if (!team_sum<COOP>(entries, &sum[0], sl, F.bar, &a.st->err, ent)) goto finish;
-            const bool inval = (unsigned long long) ent < a.inval_all_min;
-            s32 m = 0;
-            for (u32 b = tid; b < k; b += FB) {
-                const s32 x = ld_team<COOP>(&a.bw[b]);
-                m = x > m ? x : m;
-            }
-            m = __reduce_max_sync(FULL, m);
-            if (lane == 0) smx[warp] = m;
-            __syncthreads();
-            s32 new_maxw = 0;
-            for (u32 w = 0; w < FB / 32; ++w) new_maxw = smx[w] > new_maxw ? smx[w] : new_maxw;
-            // exact objective change and the neighbours' cache resets
-            long long acc = 0;
-            for (u32 wb = wbase0; wb < nm; wb += nthreads) {
-                const u32 i = wb + lane;
-                u32 u = 0, len = 0;
-                if (i < nm) {
-                    u = a.moves[i];
-                    len = a.g.rowlen[u];
-                    if (len <= FUSED_AB_THREAD) acc += delta_range<false>(a, u, 0, len, 0, 1, inval);
-                }
-                unsigned longer = __ballot_sync(FULL, i < nm && len > FUSED_AB_THREAD);
-                while (longer) {
-                    const int src = __ffs(longer) - 1;
-                    longer &= longer - 1;
-                    const u32 v = __shfl_sync(FULL, u, src), lv = __shfl_sync(FULL, len, src);
-                    acc += delta_range<false>(a, v, 0, lv, lane, 32, inval);
-                }
-            }
-            long long d = 0;
-            if (!team_sum<COOP>(acc, &sum[1], sl, F.bar, &a.st->err, d)) goto finish;
-            if (!inval)
-                for (u32 u = blockIdx.x * FB + tid; u < n; u += nthreads) a.dest_cache[u] = NULL_PART;
-            for (u32 i = blockIdx.x * FB + tid; i < nm; i += nthreads) a.map[a.moves[i]] &= ~MOVED;
-            // control (jet_label_propagation.h:966-1030, promap :1250-1305):
-            // 1 = next iteration, 2 = next ratio
-            int action = 0;
-            if (!promap) {
-                if (nm == 0) {
-                    if (lp_iter) {
-                        action = 2;
-                    } else if (balance_iteration < JET_MAX_WEAK_ITERATIONS) {
-                        balance_iteration = JET_MAX_WEAK_ITERATIONS;
-                        action = 1;
-                    } else {
-                        action = 2;
-                    }
-                } else if (!lp_iter) {
-                    balance_iteration++;
-                }
-            } else if (nm == 0) {
-                action = 1;
-            }
-            bool copy = false;
-            if (action == 0) {
-                obj += promap ? d : d / 2;
-                maxw = new_maxw;
-                const bool leq = promap ? (maxw < best_max) : (maxw <= best_max);
-                if (best_max > lmax && maxw < best_max) {
-                    copy = true;
-                    iteration = 0;
-                } else if (obj < best_obj && (maxw <= lmax || leq)) {
-                    if (1000 * obj < 999 * best_obj) iteration = 0;  // PHI = 0.999
-                    copy = true;
-                }
-                if (copy) {
-                    best_obj = obj;
-                    best_max = maxw;
-                }
-            }
-            if (copy)  // the moved bits may still be set here: mask them
-                for (u32 u = blockIdx.x * FB + tid; u < n; u += nthreads) F.part[u] = a.map[u] & ~MOVED;
-            TEAM_SYNC();
-            if (action == 2) break;
-        }
-    }
-    if (blockIdx.x == 0 && tid == 0) {
-        ctl->obj = best_obj;
-        ctl->maxw = best_max;
-        ctl->iterations = iterations;
-    }
-finish:;
-}
-
-#undef TEAM_SYNC
+#include "jet_loop.cuh"
 
 // ---- objectives ------------------------------------------------------------------
 
@@ -2508,10 +2132,6 @@ void set_big_smem() {
     HP_CUDA(cudaFuncSetAttribute(k_lp_block, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     HP_CUDA(cudaFuncSetAttribute(k_rb_block<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     HP_CUDA(cudaFuncSetAttribute(k_rb_block<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    HP_CUDA(cudaFuncSetAttribute(k_jet_loop<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int) (34 * JW_SLOTS * sizeof(s32))));
-    HP_CUDA(cudaFuncSetAttribute(k_jet_loop<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int) (34 * JW_SLOTS * sizeof(s32))));
     // staged chunk kernels: the full shared-memory carveout, so that
     // STAGE_BLOCKS_PER_SM blocks of stage_smem() bytes fit on an SM
     HP_CUDA(cudaFuncSetAttribute(k_delta_staged, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
@@ -2617,7 +2237,7 @@ void JetLevel::setup(Ctx &c, const DGraph &gr, u32 kk, s32 lm, const DistOracle 
     // warp tier: direct-indexed table of k values when k is small enough
     // (for the mapping objective the candidate scoring loops over the table,
     // so only up to 256 blocks), else a hashed table of JW_SLOTS slots
-    warp_direct = k <= JW_SLOTS && (d == nullptr || k <= 256);
+    warp_direct = direct_tables(k, d != nullptr);
     warp_slots = warp_direct ? k : JW_SLOTS;
     warp_smem = (JW_BLOCK / 32) * (warp_direct ? 1u : 2u) * warp_slots * (u32) sizeof(u32);
     // chunk items (afterburner candidates, delta moves, hub chunks; each
@@ -3070,136 +2690,221 @@ void JetLevel::run_step(int kind, u32 ratio_pct) {
     c.sync();
 }
 
-// The whole level loop in one k_jet_loop launch (warp_direct levels of at
-// most FUSED_MAX_N vertices): one block, or a cooperative grid of `blocks`
-// blocks; writes the best labelling to part.
-static void jet_refine_fused(Ctx &ctx, JetLevel &L, const std::vector<u32> &ratios, bool promap, u32 *part,
-                             s64 &obj, s32 &maxw, u32 blocks) {
-    const u32 n = L.g.n, k = L.k;
-    const s32 opt = (L.g_weight + (s32) (k - 1)) / (s32) k;
-    u32 sections, width;
-    sections_of(n, k, sections, width);
-    FusedArgs F{};
-    F.weak.opt = F.strong.opt = opt;
-    F.weak.max_b_w = std::max<s32>(L.lmax - 100, (s32) ((99 * (s64) L.lmax) / 100));
-    F.strong.max_b_w = std::max<s32>(opt + 1, (s32) ((99 * (s64) L.lmax) / 100));
-    F.weak.sections = F.strong.sections = sections;
-    F.under = ctx.balloc<u32>(k);
-    F.weak.under = F.under;
-    F.weak.keys = F.strong.keys = ctx.balloc<u32>(n);
-    F.width = width;
-    F.bits_weak = bits_for((u64) MAX_BUCKETS * k * sections + 1);
-    F.bits_strong = bits_for((u64) MAX_BUCKETS * k * sections + 2);
-    OrderScratch &S = F.S;
-    S.cands = ctx.balloc<u32>(n);
-    S.ck = ctx.balloc<u32>(n);
-    S.cands2 = ctx.balloc<u32>(n);
-    S.ck2 = ctx.balloc<u32>(n);
-    S.prefix = ctx.balloc<long long>((u64) n + 1);
-    S.B = ctx.balloc<long long>((u64) k + 1);
-    S.ea = ctx.balloc<long long>(k);
-    S.es = ctx.balloc<long long>((u64) k + 1);
-    S.mpre = ctx.balloc<long long>((u64) n + 1);
-    S.fail = ctx.balloc<u32>(n);
-    S.fail2 = ctx.balloc<u32>(n);
-    F.part = part;
-    F.gcnt = ctx.balloc<u32>(2 * FC_N);
-    F.gsum = ctx.balloc<long long>(2 * FS_N);
-    F.bar = ctx.balloc<u32>(2);
-    HP_CUDA(cudaMemsetAsync(F.bar, 0, 2 * sizeof(u32), ctx.stream));
-    HP_CUDA(cudaMemsetAsync(F.gcnt, 0, 2 * FC_N * sizeof(u32), ctx.stream));
-    HP_CUDA(cudaMemsetAsync(F.gsum, 0, 2 * FS_N * sizeof(long long), ctx.stream));
-    FusedCtl h{};
-    h.n_ratios = (u32) ratios.size();
-    for (size_t i = 0; i < ratios.size() && i < 17; ++i) h.ratios[i] = ratios[i];
-    h.lmax = L.lmax;
-    h.promap = promap ? 1u : 0u;
-    h.obj = obj;
-    h.maxw = maxw;
-    FusedCtl *d = ctx.balloc<FusedCtl>(1);
-    HP_CUDA(cudaMemcpyAsync(d, &h, sizeof(FusedCtl), cudaMemcpyHostToDevice, ctx.stream));
-    ctx.zero_counters();
-    const size_t smem = 34 * (size_t) k * sizeof(s32);
-    JArgs a = make_args(L);
-    std::optional<CoopGuard> coop;  // cooperative budget (grid blocks), until the kernel has completed
-    if (blocks <= 1) {
-        KernTimer kt(ctx, "k_jet_fused");
-        k_jet_loop<false><<<1, FB, smem, ctx.stream>>>(a, F, d); note_launch();
-    } else {
-        coop.emplace(ctx.device, ctx.stream, blocks, (u32) ctx.sm_count);
-        KernTimer kt(ctx, "k_jet_coop");
-        void *args[] = {&a, &F, &d};
-        HP_CUDA(cudaLaunchCooperativeKernel((const void *) k_jet_loop<true>, dim3(blocks), dim3(FB), args, smem,
-                                            ctx.stream));
-        note_launch();
-    }
-    HP_LAUNCH_CHECK();
-    HP_CUDA(cudaMemcpyAsync(&h, d, sizeof(FusedCtl), cudaMemcpyDeviceToHost, ctx.stream));
-    const DevStatus &st = ctx.read_status();
-    if (st.err & DEV_ERR_SPIN) throw CoopSpin{};
-    if (st.err) throw HpError{HP_ERR_DEVICE, "Jet kernel reported error bits " + std::to_string(st.err)};
-    obj = h.obj;
-    maxw = h.maxw;
+// ---- host side of the single-launch level loop ------------------------------------------
+
+constexpr u32 TEAM_CLUSTER_THREADS = 512;
+constexpr u32 TEAM_GRID_THREADS = 1024;
+// vertices per block of a cluster team (up to its largest size): 4 rows per warp
+constexpr u32 TEAM_CLUSTER_ROWS = 64;
+constexpr u32 TEAM_CLUSTER_MAX_N = 1u << 16;  // upper bound of Tunables::jet_fused_max_n
+constexpr u32 TEAM_PEER_BLOCKS = 40;
+// Levels above Tunables::jet_coop_max_deg entries per vertex run as a grid
+// team up to these sizes. Barriers dominate small levels whatever their
+// degree (ultra R-MAT 65k, levels of up to 600 entries per vertex: 302 ms with
+// a limit of 32, 221 ms with none); on larger dense levels the rows dominate,
+// which the per-kernel loop cuts into chunks and sums hub rows once (R-MAT 4M:
+// 278 ms with a limit of 128 entries per vertex, 293 ms with none; its top
+// level, 31 entries per vertex and 1.3e8 entries, 285 ms as a team).
+constexpr u64 TEAM_ANY_DEG_M = 1ull << 21;
+constexpr u64 TEAM_MID_DEG_M = 1ull << 26, TEAM_MID_DEG = 128;
+
+template<bool CLUSTER>
+static const void *team_kernel(u32 k, bool promap) {
+    if (promap) return (const void *) k_jet_team<CLUSTER, 8, true>;
+    return k <= 256 ? (const void *) k_jet_team<CLUSTER, 8, false> : (const void *) k_jet_team<CLUSTER, 32, false>;
 }
 
-// Blocks of the cooperative level loop for a level of n vertices (0 when it
-// does not apply): one per Tunables::jet_coop_rows vertices, at least two, at
-// most as many as fit on the GPU at once.
-static u32 coop_blocks(Ctx &ctx, u32 n, u32 k) {
+static cudaLaunchConfig_t team_config(u32 blocks, u32 threads, size_t smem, cudaStream_t stream,
+                                      cudaLaunchAttribute &attr, bool cluster) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    if (cluster) {
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = blocks;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+    } else {
+        attr.id = cudaLaunchAttributeCooperative;
+        attr.val.cooperative = 1;
+    }
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Per device, once: shared-memory and cluster-size limits of the team
+// kernels; returns the largest cluster that the device can run with the
+// largest tables.
+static u32 team_limits(int device) {
+    static std::mutex mu;
+    static std::vector<std::pair<int, u32> > done;
+    std::lock_guard<std::mutex> lock(mu);
+    for (const auto &d: done)
+        if (d.first == device) return d.second;
+    u32 best = TEAM_CLUSTER_MAX;
+    for (int i = 0; i < 3; ++i) {
+        const bool promap = i == 2;
+        const u32 k = i == 0 ? JW_SLOTS : 256;
+        const void *kc = team_kernel<true>(k, promap), *kg = team_kernel<false>(k, promap);
+        const size_t sc = team_smem(k, TEAM_CLUSTER_THREADS / 32, promap);
+        const size_t sg = team_smem(k, TEAM_GRID_THREADS / 32, promap);
+        HP_CUDA(cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sc));
+        HP_CUDA(cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sg));
+        HP_CUDA(cudaFuncSetAttribute(kc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        for (; best > 1; best /= 2) {
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = team_config(best, TEAM_CLUSTER_THREADS, sc, nullptr, attr, true);
+            int fits = 0;
+            if (cudaOccupancyMaxActiveClusters(&fits, kc, &cfg) == cudaSuccess && fits > 0) break;
+            cudaGetLastError();
+        }
+    }
+    done.emplace_back(device, best);
+    return best;
+}
+
+// Runs the level loop in one k_jet_team launch (direct-indexed tables): part
+// receives the best labelling. `saved` receives the input labels. Throws
+// CoopSpin when the loop gave up (barrier wait, or too many evictions to
+// rank); part is then to be restored from saved.
+static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const std::vector<u32> &ratios,
+                            const DistOracle *D, unsigned long long inval_all_min, u32 *part, u32 *saved, s64 &obj,
+                            s32 &maxw, bool cluster, u32 blocks) {
+    const u32 n = g.n;
+    const bool promap = D != nullptr;
+    TeamArgs a{};
+    a.g = g;
+    a.k = k;
+    a.lmax = lmax;
+    a.opt = ((s32) g.total_vw + (s32) (k - 1)) / (s32) k;
+    a.weak_max = std::max<s32>(lmax - 100, (s32) ((99 * (s64) lmax) / 100));
+    a.strong_max = std::max<s32>(a.opt + 1, (s32) ((99 * (s64) lmax) / 100));
+    sections_of(n, k, a.sections, a.width);
+    a.promap = promap ? 1u : 0u;
+    a.code = promap ? D->code : nullptr;
+    a.bitdist = promap ? D->bitdist : nullptr;
+    a.inval_all_min = inval_all_min;
+    a.part = part;
+    a.saved = saved;
+    a.tw = ctx.balloc<unsigned long long>(n);
+    a.abrec = ctx.balloc<unsigned long long>(n);
+    a.dest_cache = ctx.balloc<u32>(n);
+    a.gain_cache = ctx.balloc<s32>(n);
+    a.lock = ctx.balloc<u32>(n);
+    a.dest = ctx.balloc<u32>(n);
+    a.keys = ctx.balloc<u32>(n);
+    a.cand = ctx.balloc<u32>(n);
+    a.moves = ctx.balloc<u32>(n);
+    a.hubs = ctx.balloc<u32>(n);
+    a.mcomp = ctx.balloc<unsigned long long>(n);
+    a.mow = ctx.balloc<unsigned long long>(n);
+    a.tsum = ctx.balloc<s32>((u64) k * blocks);
+    a.ea = ctx.balloc<s32>(k);
+    // zeroed words in one allocation: outcome, sums, counters, barrier, block
+    // weights, bins
+    const size_t bins = (size_t) k * a.width + 2;
+    const size_t zero_bytes = sizeof(TeamOut) + 2 * TS_N * sizeof(long long) + (2 * TC_N + 2 + k + bins) * sizeof(u32);
+    char *z = ctx.balloc<char>(zero_bytes);
+    HP_CUDA(cudaMemsetAsync(z, 0, zero_bytes, ctx.stream));
+    a.out = (TeamOut *) z;
+    a.sum = (long long *) (a.out + 1);
+    a.cnt = (u32 *) (a.sum + 2 * TS_N);
+    a.bar = a.cnt + 2 * TC_N;
+    a.bw = (s32 *) (a.bar + 2);
+    a.hist = (u32 *) (a.bw + k);
+    TeamCtl ctl{};
+    ctl.n_ratios = (u32) ratios.size();
+    for (size_t i = 0; i < ratios.size() && i < 17; ++i) ctl.ratios[i] = ratios[i];
+    ctl.obj = obj;
+    ctl.maxw = maxw;
+    const u32 threads = cluster ? TEAM_CLUSTER_THREADS : TEAM_GRID_THREADS;
+    const size_t smem = team_smem(k, threads / 32, promap);
+    const void *kern = cluster ? team_kernel<true>(k, promap) : team_kernel<false>(k, promap);
+    std::optional<CoopGuard> coop;  // cooperative budget (grid blocks), until the kernel has completed
+    if (!cluster) coop.emplace(ctx.device, ctx.stream, blocks, (u32) ctx.sm_count);
+    {
+        KernTimer kt(ctx, cluster ? "k_jet_fused" : "k_jet_coop");
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = team_config(blocks, threads, smem, ctx.stream, attr, cluster);
+        void *args[] = {&a, &ctl};
+        HP_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
+        note_launch();
+    }
+    static_assert(sizeof(TeamOut) <= sizeof(DevStatus), "the outcome is read through the pinned status mirror");
+    HP_CUDA(cudaMemcpyAsync(ctx.h_status, a.out, sizeof(TeamOut), cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    const TeamOut o = *(const TeamOut *) ctx.h_status;
+    if ((o.err & DEV_ERR_SPIN) || o.gave_up) throw CoopSpin{};
+    if (o.err) throw HpError{HP_ERR_DEVICE, "Jet kernel reported error bits " + std::to_string(o.err)};
+    obj = o.obj;
+    maxw = o.maxw;
+}
+
+// Blocks of the cooperative level loop for a level of n vertices and m
+// entries (0 when it does not apply): one per Tunables::jet_coop_rows vertices
+// or 16 times as many entries, at least two, at most as many as fit on the GPU
+// at once. 512 rows against 1024 / 2048 (one B200): ultra R-MAT 65k 222 / 229
+// / 253 ms, RGG 200k 20.5 / 20.7 / 21.8 ms. Beside other solves (HM sub-solves,
+// batch and server workers) a grid takes a share of the SMs, so that grids run
+// side by side instead of one after another at full width: HM RGG 8M 403 ms
+// uncapped, 342 / 359 ms with at least 32 / 64 blocks each.
+static u32 coop_blocks(Ctx &ctx, u32 n, u64 m, u32 k, bool promap) {
     int per_sm = 0;
-    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_jet_loop<true>, FB,
-                                                          34 * (size_t) k * sizeof(s32)));
+    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, team_kernel<false>(k, promap), TEAM_GRID_THREADS,
+                                                          team_smem(k, TEAM_GRID_THREADS / 32, promap)));
     if (per_sm <= 0) return 0;
     const u64 rows = std::max<u32>(1, ctx.tune.jet_coop_rows);
-    const u64 want = ((u64) n + rows - 1) / rows;
-    return (u32) std::max<u64>(2, std::min<u64>(want, (u64) per_sm * ctx.sm_count));
+    const u64 want = (std::max<u64>(n, m / 16) + rows - 1) / rows;
+    u64 cap = (u64) per_sm * ctx.sm_count;
+    if (ctx.peers > 1) cap = std::min<u64>(cap, std::max<u64>(TEAM_PEER_BLOCKS, 2 * (u64) ctx.sm_count / ctx.peers));
+    return (u32) std::max<u64>(2, std::min<u64>(want, cap));
 }
 
 void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultra, u32 level, s64 &obj, s32 &maxw,
                 const DistOracle *D) {
     if (g.n == 0 || k <= 1) return;
     ScratchScope ss(ctx.arena);
-    JetLevel L;
-    L.setup(ctx, g, k, lmax, D, part);
     const bool promap = D != nullptr;
     // one filter ratio per level (or none for the mapping objective): a
     // recomputed gain then equals a still-valid cached one
-    L.cache_pure = promap || !ultra;
-    L.graphs = g.m <= ctx.tune.jet_graph_max_m && !ctx.prof.enabled;
-    s64 best_obj = obj;
-    s32 best_max = maxw;
+    const bool cache_pure = promap || !ultra;
     std::vector<u32> ratios;
     if (ultra && !promap) ratios = {85, 80, 75, 70, 65, 60, 55, 50, 45, 40, 35, 30, 25, 20, 15, 10, 5};
     else ratios = {level == 0 ? 25u : 75u};
-    if (L.warp_direct && !ctx.prof.enabled) {
-        if (g.n <= std::min<u32>(ctx.tune.jet_fused_max_n, FUSED_MAX_N) && g.m <= ctx.tune.jet_fused_max_m) {
-            jet_refine_fused(ctx, L, ratios, promap, part, obj, maxw, 1);
-            return;
-        }
-        if (g.n <= std::min<u32>(ctx.tune.jet_coop_max_n, FUSED_MAX_N) && g.m <= ctx.tune.jet_coop_max_m &&
-            g.m <= (u64) ctx.tune.jet_coop_max_deg * g.n) {
-            set_big_smem();
-            const u32 blocks = coop_blocks(ctx, g.n, k);
-            if (blocks) {
-                // the level's input labelling, kept for the per-kernel path
-                // should the cooperative loop give up at a grid barrier
-                u32 *saved = ctx.balloc<u32>(g.n);
-                HP_CUDA(cudaMemcpyAsync(saved, part, sizeof(u32) * g.n, cudaMemcpyDeviceToDevice, ctx.stream));
-                const s64 obj0 = obj;
-                const s32 maxw0 = maxw;
-                try {
-                    jet_refine_fused(ctx, L, ratios, promap, part, obj, maxw, blocks);
-                    return;
-                } catch (const CoopSpin &) {
-                    HP_CUDA(cudaMemcpyAsync(part, saved, sizeof(u32) * g.n, cudaMemcpyDeviceToDevice, ctx.stream));
-                    ctx.zero_status();
-                    obj = obj0;
-                    maxw = maxw0;
-                    L.setup(ctx, g, k, lmax, D, part);
-                }
+    // small and mid-size levels: the whole loop in one launch
+    if (direct_tables(k, promap) && !ctx.prof.enabled) {
+        u32 blocks = 0;
+        const bool cluster = g.n <= std::min<u32>(ctx.tune.jet_fused_max_n, TEAM_CLUSTER_MAX_N) && g.m <= ctx.tune.jet_fused_max_m;
+        const u32 max_cluster = team_limits(ctx.device);
+        if (cluster)
+            blocks = std::max<u32>(1, std::min<u32>(max_cluster, (g.n + TEAM_CLUSTER_ROWS - 1) / TEAM_CLUSTER_ROWS));
+        else if (g.n <= ctx.tune.jet_coop_max_n && g.m <= ctx.tune.jet_coop_max_m &&
+                 (g.m <= (u64) ctx.tune.jet_coop_max_deg * g.n || g.m <= TEAM_ANY_DEG_M ||
+                  (g.m <= TEAM_MID_DEG_M && g.m <= TEAM_MID_DEG * g.n)))
+            blocks = coop_blocks(ctx, g.n, g.m, k, promap);
+        if (blocks) {
+            ScratchScope ss2(ctx.arena);
+            u32 *saved = ctx.balloc<u32>(g.n);
+            const unsigned long long inval = cache_pure ? (g.m * ctx.tune.jet_inval_all_pct + 99) / 100 : ~0ull;
+            try {
+                jet_refine_team(ctx, g, k, lmax, ratios, D, inval, part, saved, obj, maxw, cluster, blocks);
+                return;
+            } catch (const CoopSpin &) {
+                // the per-kernel loop redoes the level from its input labels
+                HP_CUDA(cudaMemcpyAsync(part, saved, sizeof(u32) * g.n, cudaMemcpyDeviceToDevice, ctx.stream));
+                ctx.sync();  // saved is released here
             }
         }
     }
+    JetLevel L;
+    L.setup(ctx, g, k, lmax, D, part);
+    L.cache_pure = cache_pure;
+    L.graphs = g.m <= ctx.tune.jet_graph_max_m && !ctx.prof.enabled;
+    s64 best_obj = obj;
+    s32 best_max = maxw;
     L.prepare_kernel_loop();
     for (u32 ratio: ratios) {
         u32 balance_iteration = 0, iteration = 0;

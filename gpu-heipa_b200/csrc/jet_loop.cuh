@@ -1,0 +1,1202 @@
+// The whole Jet level loop of one level in one launch (included by jet.cu).
+//
+// A team of blocks runs every iteration of jet_refine: the iteration control
+// (ratios, weak / strong switching, best-labelling tracking) and the steps of
+// the per-kernel path, with the same result. The team is a thread-block
+// cluster on small levels (hardware barrier, co-scheduled by the hardware) or
+// a cooperative grid on larger ones (bounded grid barrier).
+//
+// What bounds it: the latency of one iteration (levels of a few thousand to a
+// few million vertices, tens to hundreds of iterations, everything in L2), so
+// the design minimises barriers and dependent loads per iteration:
+//  * a label-propagation iteration has three barriers: gains and filter, then
+//    afterburner and moves, then the objective change. A vertex word holds
+//    label, previous label and the iteration that changed it, so moves are
+//    applied while other blocks still read the previous labels, and nothing
+//    has to be unmarked afterwards;
+//  * a rebalance iteration sorts nothing. Candidates add their weight to a
+//    histogram over the mini-bucket keys; per overloaded block the histogram
+//    gives the mini-bucket in which the limit falls, and only the candidates
+//    of that one need their order (ascending vertex id): per-warp weight sums
+//    over contiguous vertex ranges, prefix sums over them and a prefix within
+//    32 vertices. Strong rebalancing needs the exact prefix of every evicted
+//    vertex: the few evicted ones are ranked among each other;
+//  * rows are evaluated by 8 lanes (32 lanes for k > 256) with a
+//    direct-indexed block table in shared memory: an entry costs one add and
+//    one exchange, which collects each distinct block once and clears the
+//    table; no pass over all k blocks.
+// Measured (one B200, mean time of one iteration): against one 1024-thread
+// block that ran the same steps, levels of up to 4096 vertices of an RGG with
+// 3001 vertices 27 -> 14 us; against a cooperative grid whose block 0 sorted
+// the candidates, levels of up to 65536 vertices of a 256x256 grid 62 -> 21 us,
+// of an R-MAT graph with 65536 vertices 280 -> 71 us. Between two barriers
+// about 3 us remain when there is little work: the barrier, the list length,
+// the list entry, the row bounds, the row and the neighbours' words are read
+// one after the other.
+#pragma once
+
+constexpr u32 TEAM_HUB = 1024;         // rows above this length are evaluated by a whole block
+constexpr u32 TEAM_LONG = 64;          // afterburner / delta rows above this length take a whole warp
+constexpr u32 TEAM_LIST = 128;         // distinct-block list slots per warp (mapping objective; at least k)
+constexpr u32 TEAM_RANK_MAX = 32768;   // evicted vertices ranked by counting; more are left to the per-kernel path
+constexpr u32 TEAM_CLUSTER_MAX = 16;   // blocks of a cluster team
+
+enum TeamCnt { TC_HUB = 0, TC_CAND = 1, TC_MOVES = 2, TC_FAIL = 3, TC_N = 4 };
+enum TeamSum { TS_ENTRIES = 0, TS_DELTA = 1, TS_N = 2 };
+
+// Vertex word: label (16 bits), previous label (16 bits), iteration that
+// changed the label (32 bits).
+__device__ __forceinline__ u32 tw_label(unsigned long long x) { return (u32) x & 0xFFFFu; }
+__device__ __forceinline__ u32 tw_old(unsigned long long x) { return ((u32) x >> 16); }
+__device__ __forceinline__ u32 tw_stamp(unsigned long long x) { return (u32) (x >> 32); }
+
+struct TeamCtl {
+    u32 n_ratios;
+    u32 ratios[17];
+    long long obj;   // objective of the input labelling
+    s32 maxw;        // its maximum block weight
+};
+
+// Outcome, written by the kernel.
+struct TeamOut {
+    long long obj;   // best objective
+    s32 maxw;        // its maximum block weight
+    u32 iterations;
+    u32 gave_up;     // 1: more than TEAM_RANK_MAX evicted vertices in one step, nothing was decided
+    u32 err;         // DevErr bits
+};
+
+struct TeamArgs {
+    DGraph g;
+    u32 k;
+    s32 lmax;
+    s32 opt;
+    s32 weak_max, strong_max;
+    u32 sections, width;
+    u32 promap;
+    const u32 *code;
+    const s32 *bitdist;
+    unsigned long long inval_all_min;
+    u32 *part;                  // in: labels; out: best labelling
+    u32 *saved;                 // receives a copy of the input labels
+    unsigned long long *tw;     // vertex words
+    unsigned long long *abrec;  // afterburner records: gain, target (16 bits), label (16 bits)
+    u32 *dest_cache;
+    s32 *gain_cache;
+    u32 *lock;
+    u32 *dest;                  // rebalance targets
+    u32 *keys;                  // mini-bucket keys
+    u32 *cand, *moves, *hubs;
+    unsigned long long *mcomp;  // strong: (key, vertex) of every evicted vertex
+    unsigned long long *mow;    // strong: (block, vertex weight)
+    s32 *bw;                    // zero on entry
+    u32 *hist;                  // k * width + 2 weights, zero on entry
+    s32 *tsum;                  // k * blocks
+    s32 *ea;                    // k
+    u32 *cnt;                   // 2 sets of TC_N counters, zero on entry
+    long long *sum;             // 2 sets of TS_N sums, zero on entry
+    u32 *bar;                   // grid barrier word, zero on entry
+    TeamOut *out;  // zero on entry
+};
+
+// Shared-memory arrays (dynamic): per warp the block tables, then k-word
+// arrays of the block.
+struct TeamSm {
+    s32 *tab;      // this warp's tables
+    s32 *tab0;     // the block's first table
+    u32 stride;    // words between the tables of two warps
+    unsigned long long *list;  // this warp's distinct-block list (mapping objective)
+    s32 *bw, *bd, *cutbase, *tot, *spill, *toff;
+    u32 *under, *olist, *cutkey;
+    long long *es, *pre;
+    u32 *code;
+    s32 *dist;
+};
+
+// Bytes of dynamic shared memory of a team block of `warps` warps.
+inline size_t team_smem(u32 k, u32 warps, bool promap) {
+    const size_t groups = k <= 256 ? 4 : 1;
+    size_t b = (size_t) warps * groups * k * 4;
+    b = (b + 15) & ~(size_t) 15;
+    if (promap) b += (size_t) warps * std::max<u32>(TEAM_LIST, k) * 8;
+    b += ((size_t) k + 2) * 8 * 2 + (size_t) k * 4 * 10 + 32 * 4;
+    return (b + 15) & ~(size_t) 15;
+}
+
+template<int GL>
+__device__ __forceinline__ TeamSm team_carve(unsigned char *base, u32 k, u32 warps, u32 warp, bool promap) {
+    TeamSm S;
+    S.stride = (32 / GL) * k;
+    S.tab0 = (s32 *) base;
+    S.tab = S.tab0 + warp * S.stride;
+    size_t off = ((size_t) warps * S.stride * 4 + 15) & ~(size_t) 15;
+    const u32 ln = k > TEAM_LIST ? k : TEAM_LIST;
+    S.list = nullptr;
+    if (promap) {
+        S.list = (unsigned long long *) (base + off) + (size_t) warp * ln;
+        off += (size_t) warps * ln * 8;
+    }
+    S.es = (long long *) (base + off);
+    S.pre = S.es + k + 2;
+    s32 *p = (s32 *) (S.pre + k + 2);
+    S.bw = p;
+    S.bd = p + k;
+    S.cutbase = p + 2 * k;
+    S.tot = p + 3 * k;
+    S.spill = p + 4 * k;
+    S.toff = p + 5 * k;
+    S.under = (u32 *) (p + 6 * k);
+    S.olist = (u32 *) (p + 7 * k);
+    S.cutkey = (u32 *) (p + 8 * k);
+    S.code = (u32 *) (p + 9 * k);
+    S.dist = p + 10 * k;
+    return S;
+}
+
+// ---- team barrier ----------------------------------------------------------------------
+
+// Cluster: the hardware barrier (release / acquire at cluster scope). Grid:
+// one counter that only grows; thread 0 of every block adds one and waits for
+// it to reach a multiple of the grid size. The wait is bounded: after
+// TEAM_SPINS polls a block adds TEAM_POISON, which ends every wait, and all
+// blocks leave (the host redoes the level).
+constexpr u32 TEAM_POISON = 0x80000000u;
+constexpr u32 TEAM_SPINS = 1u << 21;
+
+template<bool CLUSTER>
+__device__ __forceinline__ bool team_barrier(u32 *bar, u32 &target, u32 *err) {
+    if (CLUSTER) {
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        return true;
+    }
+    __shared__ u32 s_ok;
+    target += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        u32 v;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(bar) : "memory");
+        v += 1;
+        u32 spins = 0;
+        while (v < target) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if (++spins > TEAM_SPINS) {
+                set_error(err, DEV_ERR_SPIN);
+                atomicOr(bar, TEAM_POISON);
+                v = TEAM_POISON;
+            }
+        }
+        s_ok = v < TEAM_POISON ? 1u : 0u;
+    }
+    __syncthreads();
+    return s_ok != 0u;
+}
+
+// ---- row evaluation --------------------------------------------------------------------
+
+enum TeamOp { OP_CUT = 0, OP_MAP = 1, OP_WEAK = 2, OP_STRONG = 3 };
+
+struct RowOut {
+    unsigned long long bk;  // best block key
+    s32 own;                // connection to the own block
+    s32 sum, count;         // strong: connection to and number of the eligible blocks
+};
+
+__device__ __forceinline__ s32 team_dist(const TeamSm &S, u32 x, u32 y) {
+    if (x == y) return 0;
+    return S.dist[31 - __clz(S.code[x] ^ S.code[y])];
+}
+
+// One distinct neighbour block b with connection c of a row of block o.
+template<int OP>
+__device__ __forceinline__ void row_take(const TeamSm &S, u32 o, s32 max_b_w, u32 b, s32 c, RowOut &r) {
+    if (b == o) {
+        r.own = c;
+        return;
+    }
+    if (OP == OP_STRONG) {
+        if (S.bw[b] < max_b_w) {
+            r.sum = wadd(r.sum, c);
+            ++r.count;
+        }
+    } else if (OP == OP_CUT || S.bw[b] < max_b_w) {
+        const unsigned long long key = cut_key(c, b);
+        r.bk = key > r.bk ? key : r.bk;
+    }
+}
+
+// Mapping objective: scores the distinct blocks list[0, cnt) (block in the
+// high word, connection in the low word) of a row of block o; lanes first,
+// first + step, ... of the list.
+__device__ __forceinline__ void row_score(const TeamSm &S, const unsigned long long *list, u32 cnt, u32 o, u32 first,
+                                          u32 step, RowOut &r) {
+    for (u32 i = first; i < cnt; i += step) {
+        const u32 b = (u32) (list[i] >> 32);
+        if (b == o) continue;
+        s32 d = 0;
+        for (u32 t = 0; t < cnt; ++t) {
+            const unsigned long long e = list[t];
+            const u32 id = (u32) (e >> 32);
+            d = wadd(d, wmul((s32) (u32) e, wsub(team_dist(S, o, id), team_dist(S, b, id))));
+        }
+        const unsigned long long key = delta_key(d, b);
+        r.bk = key > r.bk ? key : r.bk;
+    }
+}
+
+// Reduces a row result over groups of GL lanes (every lane of a group
+// receives it).
+template<int OP, int GL>
+__device__ __forceinline__ void row_reduce(RowOut &r) {
+#pragma unroll
+    for (int d = GL / 2; d > 0; d >>= 1) {
+        if (OP != OP_MAP) r.own += __shfl_xor_sync(FULL, r.own, d);  // one lane holds it
+        if (OP == OP_STRONG) {
+            r.sum = wadd(r.sum, __shfl_xor_sync(FULL, r.sum, d));
+            r.count += __shfl_xor_sync(FULL, r.count, d);
+        } else {
+            const unsigned long long y = __shfl_xor_sync(FULL, r.bk, d);
+            r.bk = y > r.bk ? y : r.bk;
+        }
+    }
+}
+
+__device__ __forceinline__ u32 label_of(const TeamArgs &a, u32 v) { return ((const u32 *) a.tw)[2 * (u64) v] & 0xFFFFu; }
+
+// Evaluates the rows of the lanes in `need` (beg, len <= 4 * GL, own block o
+// of each lane's row), 32 / GL rows at a time, GL lanes per row; every lane
+// receives its row's result. All lanes of the warp call this.
+template<int OP, int GL>
+__device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u32 need, u32 beg, u32 len, u32 o,
+                                           s32 max_b_w, RowOut &out) {
+    constexpr int NG = 32 / GL;
+    const u32 lane = lane_id(), g = lane / GL, gl = lane % GL;
+    s32 *tv = S.tab + g * a.k;
+    while (need) {
+        u32 m = need, rest = need;
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            if (i < (int) g) m &= m - 1;
+            rest &= rest - 1;
+        }
+        const int src = m ? __ffs(m) - 1 : 0;
+        const u32 rb = __shfl_sync(FULL, beg, src);
+        u32 rl = __shfl_sync(FULL, len, src);
+        const u32 ro = __shfl_sync(FULL, o, src);
+        if (!m) rl = 0;
+        u32 b[4];
+        s32 w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const u32 t = gl + j * GL;
+            b[j] = t < rl ? __ldg(&a.g.adj[(u64) rb + t]) : EMPTY;
+            w[j] = t < rl ? g_ew(a.g, (u64) rb + t) : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (b[j] != EMPTY) b[j] = label_of(a, b[j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (b[j] != EMPTY) atomicAdd(&tv[b[j]], w[j]);
+        __syncwarp();
+        // the exchange returns a block's connection to one of its entries and
+        // clears the table
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = b[j] != EMPTY ? atomicExch(&tv[b[j]], 0) : 0;
+        __syncwarp();
+        RowOut r{0, 0, 0, 0};
+        if (OP == OP_MAP) {
+            unsigned long long *list = S.list + g * (4 * GL);
+            u32 cnt = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const u32 mask = (__ballot_sync(FULL, w[j] != 0) >> (g * GL)) & (GL == 32 ? FULL : (1u << GL) - 1u);
+                if (w[j] != 0) list[cnt + __popc(mask & ((1u << gl) - 1u))] = ((unsigned long long) b[j] << 32) | (u32) w[j];
+                cnt += __popc(mask);
+            }
+            __syncwarp();
+            row_score(S, list, cnt, ro, gl, GL, r);
+            __syncwarp();
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (w[j] != 0) row_take<OP>(S, ro, max_b_w, b[j], w[j], r);
+        }
+        row_reduce<OP, GL>(r);
+        // back to the lanes that own the rows
+        const u32 rank = __popc(need & ((1u << lane) - 1u));
+        const bool mine = (need >> lane & 1u) && rank < (u32) NG;
+        const int from = (mine ? rank : 0) * GL;
+        const unsigned long long bk = __shfl_sync(FULL, r.bk, from);
+        const s32 own = __shfl_sync(FULL, r.own, from);
+        const s32 sum = OP == OP_STRONG ? __shfl_sync(FULL, r.sum, from) : 0;
+        const s32 count = OP == OP_STRONG ? __shfl_sync(FULL, r.count, from) : 0;
+        if (mine) out = RowOut{bk, own, sum, count};
+        need = rest;
+    }
+}
+
+// Adds entries first, first + step, ... of a row to the direct table tv.
+__device__ __forceinline__ void row_add(const TeamArgs &a, u32 beg, u32 len, u32 first, u32 step, s32 *tv) {
+    for (u32 t0 = first; t0 < len; t0 += 4 * step) {
+        u32 b[4];
+        s32 w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const u32 t = t0 + j * step;
+            b[j] = t < len ? __ldg(&a.g.adj[(u64) beg + t]) : EMPTY;
+            w[j] = t < len ? g_ew(a.g, (u64) beg + t) : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (b[j] != EMPTY) b[j] = label_of(a, b[j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (b[j] != EMPTY) atomicAdd(&tv[b[j]], w[j]);
+    }
+}
+
+// Result of a filled table (one warp; clears it).
+template<int OP>
+__device__ __forceinline__ RowOut row_finish(const TeamArgs &a, const TeamSm &S, s32 *tv, u32 o, s32 max_b_w) {
+    const u32 lane = lane_id();
+    RowOut r{0, 0, 0, 0};
+    if (OP == OP_MAP) {
+        u32 cnt = 0;
+        for (u32 s0 = 0; s0 < a.k; s0 += 32) {
+            const u32 s = s0 + lane;
+            const s32 c = s < a.k ? tv[s] : 0;
+            const u32 mask = __ballot_sync(FULL, c != 0);
+            if (c != 0) {
+                S.list[cnt + __popc(mask & ((1u << lane) - 1u))] = ((unsigned long long) s << 32) | (u32) c;
+                tv[s] = 0;
+            }
+            cnt += __popc(mask);
+        }
+        __syncwarp();
+        row_score(S, S.list, cnt, o, lane, 32, r);
+    } else {
+        for (u32 s = lane; s < a.k; s += 32) {
+            const s32 c = tv[s];
+            if (c != 0) {
+                tv[s] = 0;
+                row_take<OP>(S, o, max_b_w, s, c, r);
+            }
+        }
+    }
+    __syncwarp();
+    row_reduce<OP, 32>(r);
+    return r;
+}
+
+// Evaluates the rows of the lanes in `need`, one at a time by the whole warp.
+template<int OP>
+__device__ __forceinline__ void rows_long(const TeamArgs &a, const TeamSm &S, u32 need, u32 beg, u32 len, u32 o,
+                                          s32 max_b_w, RowOut &out) {
+    while (need) {
+        const int src = __ffs(need) - 1;
+        need &= need - 1;
+        const u32 rb = __shfl_sync(FULL, beg, src), rl = __shfl_sync(FULL, len, src), ro = __shfl_sync(FULL, o, src);
+        row_add(a, rb, rl, lane_id(), 32, S.tab);
+        __syncwarp();
+        const RowOut r = row_finish<OP>(a, S, S.tab, ro, max_b_w);
+        if (lane_id() == src) out = r;
+    }
+}
+
+// Target and gain of a row (jet_lp :193-238 / ProMap_jet_lp :219-263).
+template<bool MAP>
+__device__ __forceinline__ void lp_decide(const RowOut &r, u32 ratio, u32 &best, s32 &gain) {
+    best = NO_MOVE;
+    gain = 0;
+    if (!r.bk) return;
+    if (MAP) {
+        const s32 d = (s32) ((u32) (r.bk >> 32) ^ 0x80000000u);
+        if (d >= 0) {
+            best = ~(u32) r.bk;
+            gain = d;
+        }
+    } else {
+        const s32 bc = (s32) (u32) (r.bk >> 32);
+        if (bc >= r.own || (s64) r.own - (s64) bc < ((s64) ratio * (s64) r.own) / 100) {
+            best = ~(u32) r.bk;
+            gain = wsub(bc, r.own);
+        }
+    }
+}
+
+// Filter of one vertex (:247-258): its afterburner record; true when it is a
+// candidate.
+__device__ __forceinline__ bool lp_filter_one(const TeamArgs &a, u32 u, u32 o, u32 dest, s32 gain, u32 lock) {
+    const bool c = dest != NO_MOVE && lock == 0;
+    if (!c && lock) a.lock[u] = 0;
+    a.abrec[u] = (unsigned long long) (u32) (c ? gain : GAIN_MIN) | ((unsigned long long) (dest & 0xFFFFu) << 32) |
+                 ((unsigned long long) o << 48);
+    return c;
+}
+
+// Moves u from ou to nu (perform_moves :753-924).
+__device__ __forceinline__ void team_move(const TeamArgs &a, const TeamSm &S, u32 u, u32 ou, u32 nu, s32 vw, u32 stamp) {
+    if (ou != nu) {
+        atomicSub(&S.bd[ou], vw);
+        atomicAdd(&S.bd[nu], vw);
+    }
+    a.tw[u] = (unsigned long long) nu | ((unsigned long long) ou << 16) |
+              ((unsigned long long) (ou != nu ? stamp : 0u) << 32);
+    a.dest_cache[u] = NULL_PART;
+}
+
+// Afterburner terms of up to four loaded entries (ab_batch over abrec).
+template<bool MAP>
+__device__ __forceinline__ s32 team_ab(const TeamArgs &a, const TeamSm &S, u32 u, s32 ug, u32 ou, u32 nu, u32 beg,
+                                       u32 len, u32 first, u32 step) {
+    s32 change = 0;
+    for (u32 t0 = first; t0 < len; t0 += 4 * step) {
+        u32 v[4];
+        s32 w[4];
+        unsigned long long x[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const u32 t = t0 + j * step;
+            v[j] = t < len ? __ldg(&a.g.adj[(u64) beg + t]) : SENTINEL;
+            w[j] = t < len ? g_ew(a.g, (u64) beg + t) : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[j] = v[j] != SENTINEL ? a.abrec[v[j]] : 0ull;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const s32 vg = (s32) (u32) x[j];
+            if (v[j] == SENTINEL || !(vg > ug || (vg == ug && v[j] < u))) continue;
+            const u32 nv = (u32) (x[j] >> 32) & 0xFFFFu, ov = (u32) (x[j] >> 48);
+            s32 t;
+            if (!MAP) {
+                t = wmul(w[j], (s32) (nv == nu) - (s32) (nv == ou) + (s32) (ov == ou) - (s32) (ov == nu));
+            } else {
+                const s32 before_u = wsub(team_dist(S, ou, ov), team_dist(S, nu, ov));
+                const s32 after_u = wsub(team_dist(S, ou, nv), team_dist(S, nu, nv));
+                t = wmul(w[j], wsub(after_u, before_u));
+            }
+            change = wadd(change, t);
+        }
+    }
+    return change;
+}
+
+// Objective change and cache resets over a moved row (delta_batch).
+template<bool MAP>
+__device__ __forceinline__ long long team_delta(const TeamArgs &a, const TeamSm &S, u32 ou, u32 nu, bool moved,
+                                                u32 stamp, u32 beg, u32 len, u32 first, u32 step, bool inval) {
+    long long acc = 0;
+    for (u32 t0 = first; t0 < len; t0 += 4 * step) {
+        u32 v[4];
+        s32 w[4];
+        unsigned long long x[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const u32 t = t0 + j * step;
+            v[j] = t < len ? __ldg(&a.g.adj[(u64) beg + t]) : SENTINEL;
+            w[j] = t < len ? g_ew(a.g, (u64) beg + t) : 0;
+        }
+        if (moved) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = v[j] != SENTINEL ? a.tw[v[j]] : 0ull;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (v[j] == SENTINEL) continue;
+                const bool mv = tw_stamp(x[j]) == stamp;
+                const u32 nv = tw_label(x[j]), ov = mv ? tw_old(x[j]) : nv;
+                long long c;
+                if (!MAP) c = (long long) w[j] * ((long long) (nu != nv) - (long long) (ou != ov));
+                else c = (long long) w[j] * ((long long) team_dist(S, nu, nv) - (long long) team_dist(S, ou, ov));
+                acc += mv ? c : 2 * c;
+            }
+        }
+        if (inval) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (v[j] != SENTINEL) a.dest_cache[v[j]] = NULL_PART;
+        }
+    }
+    return acc;
+}
+
+// Exclusive prefix (p) and total (t) of v over the lanes of `mask` (this
+// lane's peers). All lanes of the warp call this.
+__device__ __forceinline__ void peer_prefix(u32 mask, s32 v, s32 &p, s32 &t) {
+    const u32 lane = lane_id();
+    p = 0;
+    t = 0;
+#pragma unroll
+    for (u32 i = 0; i < 32; ++i) {
+        const s32 x = __shfl_sync(FULL, v, i);
+        if (mask >> i & 1u) {
+            t += x;
+            if (i < lane) p += x;
+        }
+    }
+}
+
+// Adds v over all threads to *slot with one atomic per block. No block
+// barrier follows: the team barrier does.
+__device__ __forceinline__ void team_add(long long v, long long *slot, long long *sm) {
+    v = warp_sum<long long>(v);
+    if (lane_id() == 0) sm[warp_in_block()] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        long long r = 0;
+        for (u32 w = 0; w < (blockDim.x >> 5); ++w) r += sm[w];
+        if (r) atomicAdd((unsigned long long *) slot, (unsigned long long) r);
+    }
+}
+
+// Adds the block's weight changes to the block weights (after a
+// __syncthreads() that follows the last team_move).
+__device__ __forceinline__ void team_flush_bw(const TeamArgs &a, const TeamSm &S) {
+    for (u32 b = threadIdx.x; b < a.k; b += blockDim.x)
+        if (S.bd[b]) {
+            atomicAdd(&a.bw[b], S.bd[b]);
+            S.bd[b] = 0;
+        }
+}
+
+// Copies the block weights to shared memory and returns their maximum (at
+// least 0). All threads call this.
+__device__ __forceinline__ s32 team_load_bw(const TeamArgs &a, const TeamSm &S, s32 *smx) {
+    s32 m = 0;
+    for (u32 b = threadIdx.x; b < a.k; b += blockDim.x) {
+        const s32 x = __ldcg(&a.bw[b]);
+        S.bw[b] = x;
+        m = x > m ? x : m;
+    }
+    m = __reduce_max_sync(FULL, m);
+    if (lane_id() == 0) smx[warp_in_block()] = m;
+    __syncthreads();
+    s32 r = 0;
+    for (u32 w = 0; w < (blockDim.x >> 5); ++w) r = smx[w] > r ? smx[w] : r;
+    __syncthreads();
+    return r;
+}
+
+#define TEAM_SYNC()                                                         \
+    do {                                                                    \
+        if (!team_barrier<CLUSTER>(a.bar, bar_target, &a.out->err)) return;  \
+    } while (0)
+
+// CLUSTER: the team is one cluster (gridDim.x blocks), else a cooperative
+// grid. GL: lanes per short row. MAP: process-mapping objective.
+template<bool CLUSTER, int GL, bool MAP>
+__global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ TeamArgs a,
+                                                        const __grid_constant__ TeamCtl ctl) {
+    extern __shared__ __align__(16) unsigned char team_dsm[];
+    __shared__ long long sl[33];
+    __shared__ u32 su[33];
+    __shared__ s32 smx[32];
+    const u32 tid = threadIdx.x, lane = lane_id(), warp = warp_in_block(), nw = blockDim.x >> 5;
+    const u32 n = a.g.n, k = a.k, G = gridDim.x;
+    TeamSm S = team_carve<GL>(team_dsm, k, nw, warp, MAP);
+    u32 bar_target = 0;
+    for (u32 i = tid; i < nw * S.stride; i += blockDim.x) S.tab0[i] = 0;
+    for (u32 b = tid; b < k; b += blockDim.x) {
+        S.bd[b] = 0;
+        if (MAP) S.code[b] = a.code[b];
+    }
+    if (MAP && tid < 32) S.dist[tid] = a.bitdist[tid];
+    __syncthreads();
+    // contiguous vertex range of every warp (ascending with block and warp)
+    const u32 gwarps = G * nw, gw = blockIdx.x * nw + warp;
+    const u32 per = (n + gwarps - 1) / gwarps;
+    const u32 r0 = (u32) min((u64) n, (u64) gw * per), r1 = (u32) min((u64) n, (u64) r0 + per);
+    for (u32 u = r0 + lane; u < r1; u += 32) {
+        const u32 o = a.part[u];
+        a.saved[u] = o;
+        a.tw[u] = o;
+        a.dest_cache[u] = NULL_PART;
+        a.lock[u] = 0;
+        atomicAdd(&S.bd[o], g_vw(a.g, u));
+    }
+    __syncthreads();
+    team_flush_bw(a, S);
+    TEAM_SYNC();
+    team_load_bw(a, S, smx);
+    long long obj = ctl.obj, best_obj = obj;
+    s32 maxw = ctl.maxw, best_max = maxw;
+    u32 iterations = 0;
+    for (u32 ri = 0; ri < ctl.n_ratios; ++ri) {
+        const u32 ratio = ctl.ratios[ri];
+        u32 balance_iteration = 0, iteration = 0;
+        while (iteration < JET_MAX_ITERATIONS) {
+            iteration += 1;
+            ++iterations;
+            const u32 stamp = iterations;
+            // counter set of this iteration (zero); block 0 clears the other
+            // one after the first barrier, when every thread has read it
+            u32 *const cnt = a.cnt + (iterations & 1u) * TC_N;
+            long long *const sum = a.sum + (iterations & 1u) * TS_N;
+            u32 *const cnt_o = a.cnt + ((iterations & 1u) ^ 1u) * TC_N;
+            long long *const sum_o = a.sum + ((iterations & 1u) ^ 1u) * TS_N;
+            bool lp_iter = false;
+            int step;
+            if (maxw <= a.lmax) {
+                step = 0;
+                lp_iter = true;
+                balance_iteration = 0;
+            } else if (!MAP) {
+                step = balance_iteration < JET_MAX_WEAK_ITERATIONS ? 1 : 2;
+            } else {
+                balance_iteration++;
+                step = balance_iteration < JET_MAX_WEAK_ITERATIONS ? 1 : 2;
+            }
+            long long entries = 0;
+            if (step == 0) {
+                // gains (cached targets, else recomputed) and filter
+                constexpr int OP = MAP ? OP_MAP : OP_CUT;
+                for (u32 base = r0; base < r1; base += 32) {
+                    const u32 u = base + lane;
+                    const bool act = u < r1;
+                    u32 dest = NO_MOVE, lock = 0, o = 0, len = 0, beg = 0;
+                    s32 gain = 0;
+                    if (act) {
+                        dest = a.dest_cache[u];
+                        lock = a.lock[u];
+                        gain = a.gain_cache[u];
+                        o = label_of(a, u);
+                    }
+                    const bool need = act && dest == NULL_PART;
+                    if (need) {
+                        len = __ldg(&a.g.rowlen[u]);
+                        beg = __ldg(&a.g.rowptr[u]);
+                    }
+                    const bool hub = need && len > TEAM_HUB;
+                    RowOut r{0, 0, 0, 0};
+                    rows_short<OP, GL>(a, S, __ballot_sync(FULL, need && len <= 4 * GL), beg, len, o, 0, r);
+                    rows_long<OP>(a, S, __ballot_sync(FULL, need && len > 4 * GL && !hub), beg, len, o, 0, r);
+                    if (need && !hub) {
+                        lp_decide<MAP>(r, ratio, dest, gain);
+                        a.dest_cache[u] = dest;
+                        a.gain_cache[u] = gain;
+                    }
+                    const u32 sh = warp_append(&cnt[TC_HUB], hub);
+                    if (hub) a.hubs[sh] = u;
+                    const bool c = act && !hub && lp_filter_one(a, u, o, dest, gain, lock);
+                    const u32 sc = warp_append(&cnt[TC_CAND], c);
+                    if (c) a.cand[sc] = u;
+                }
+                TEAM_SYNC();
+                if (blockIdx.x == 0 && tid < TC_N) cnt_o[tid] = 0;
+                if (blockIdx.x == 0 && tid < TS_N) sum_o[tid] = 0;
+                const u32 nhub = __ldcg(&cnt[TC_HUB]);
+                if (nhub) {
+                    for (u32 i = blockIdx.x; i < nhub; i += G) {
+                        const u32 u = a.hubs[i], o = label_of(a, u);
+                        row_add(a, __ldg(&a.g.rowptr[u]), __ldg(&a.g.rowlen[u]), tid, blockDim.x, S.tab0);
+                        __syncthreads();
+                        if (warp == 0) {
+                            const RowOut r = row_finish<OP>(a, S, S.tab0, o, 0);
+                            if (lane == 0) {
+                                u32 dest;
+                                s32 gain;
+                                lp_decide<MAP>(r, ratio, dest, gain);
+                                a.dest_cache[u] = dest;
+                                a.gain_cache[u] = gain;
+                                if (lp_filter_one(a, u, o, dest, gain, a.lock[u])) a.cand[atomicAdd(&cnt[TC_CAND], 1u)] = u;
+                            }
+                        }
+                        __syncthreads();
+                    }
+                    TEAM_SYNC();
+                }
+                // afterburner and moves: 8 lanes per candidate, long rows by the warp
+                const u32 nc = __ldcg(&cnt[TC_CAND]);
+                const u32 g = lane >> 3, gl = lane & 7;
+                for (u32 base = gw * 4; base < nc; base += gwarps * 4) {
+                    const u32 i = base + g;
+                    const bool act = i < nc;
+                    u32 u = 0, len = 0, beg = 0;
+                    unsigned long long rec = 0;
+                    if (act) {
+                        u = a.cand[i];
+                        len = __ldg(&a.g.rowlen[u]);
+                        beg = __ldg(&a.g.rowptr[u]);
+                        rec = a.abrec[u];
+                    }
+                    const s32 ug = (s32) (u32) rec;
+                    const u32 nu = (u32) (rec >> 32) & 0xFFFFu, ou = (u32) (rec >> 48);
+                    s32 ch = 0;
+                    if (act && len <= TEAM_LONG) ch = team_ab<MAP>(a, S, u, ug, ou, nu, beg, len, gl, 8);
+                    __syncwarp();
+#pragma unroll
+                    for (int d = 4; d > 0; d >>= 1) ch = wadd(ch, __shfl_xor_sync(FULL, ch, d));
+                    u32 lng = __ballot_sync(FULL, gl == 0 && len > TEAM_LONG);
+                    while (lng) {
+                        const int src = __ffs(lng) - 1;
+                        lng &= lng - 1;
+                        const u32 xu = __shfl_sync(FULL, u, src), xl = __shfl_sync(FULL, len, src),
+                                  xb = __shfl_sync(FULL, beg, src), xo = __shfl_sync(FULL, ou, src),
+                                  xn = __shfl_sync(FULL, nu, src);
+                        const s32 xg = __shfl_sync(FULL, ug, src);
+                        const s32 c = (s32) warp_sum<u32>((u32) team_ab<MAP>(a, S, xu, xg, xo, xn, xb, xl, lane, 32));
+                        if ((int) lane == src) ch = c;
+                    }
+                    const bool mv = act && gl == 0 && wadd(ug, ch) >= 0;
+                    if (mv) {
+                        a.lock[u] = 1;
+                        team_move(a, S, u, ou, nu, g_vw(a.g, u), stamp);
+                        entries += len;
+                    }
+                    const u32 sm_ = warp_append(&cnt[TC_MOVES], mv);
+                    if (mv) a.moves[sm_] = u;
+                }
+                team_add(entries, &sum[TS_ENTRIES], sl);
+                team_flush_bw(a, S);
+                TEAM_SYNC();
+            } else {
+                const bool strong = step == 2;
+                const s32 max_b_w = strong ? a.strong_max : a.weak_max;
+                const u32 sft = strong ? 1u : 0u;  // own keys of block o: [o * width + sft, (o + 1) * width + sft)
+                // blocks with room (weak) or the largest room (strong), and
+                // the overloaded blocks, from the block weights in shared memory
+                u32 n_under = 0, n_over = 0;
+                s32 maxv = INT32_MIN;
+                for (u32 b0 = 0; b0 < k; b0 += blockDim.x) {
+                    const u32 b = b0 + tid;
+                    const s32 x = b < k ? S.bw[b] : INT32_MAX;
+                    const bool un = b < k && x < max_b_w, ov = b < k && x > a.lmax;
+                    if (un && max_b_w - x > maxv) maxv = max_b_w - x;
+                    u32 tot;
+                    const u32 p = block_exclusive_scan<u32>((un ? 1u : 0u) | (ov ? 0x10000u : 0u), tot, su);
+                    if (un) S.under[n_under + (p & 0xFFFFu)] = b;
+                    if (ov) S.olist[n_over + (p >> 16)] = b;
+                    n_under += tot & 0xFFFFu;
+                    n_over += tot >> 16;
+                }
+                maxv = __reduce_max_sync(FULL, maxv);
+                if (lane == 0) smx[warp] = maxv;
+                __syncthreads();
+                for (u32 w = 0; w < nw; ++w) maxv = smx[w] > maxv ? smx[w] : maxv;
+                if (strong && blockIdx.x == 0)
+                    for (u32 b = tid; b < k; b += blockDim.x) a.ea[b] = 0;
+                // picks: target and mini-bucket key of every candidate, whose
+                // weight goes to the key's bin
+                auto finish = [&](u32 u, u32 o, s32 vw, const RowOut &r) -> u32 {
+                    if (strong) {
+                        const s32 gain = wsub(r.sum / (r.count ? r.count : 1), r.own);
+                        const s32 excess = S.bw[o] - a.lmax;
+                        return (MAX_BUCKETS * o + gain_bucket(gain, vw < excess ? vw : excess)) * a.sections +
+                               (u % a.sections) + 1;
+                    }
+                    u32 best = o;
+                    s32 gain = 0;
+                    const s32 best_w = r.bk ? (s32) (u32) (r.bk >> 32) : 0;
+                    if (best_w <= 0) {
+                        if (n_under > 0) best = S.under[u % n_under];
+                        gain = -r.own;
+                    } else {
+                        best = ~(u32) r.bk;
+                        gain = wsub(best_w, r.own);
+                    }
+                    a.dest[u] = best;
+                    return o != best ? (MAX_BUCKETS * o + gain_bucket(gain, vw)) * a.sections + (u % a.sections) : NOKEY;
+                };
+                for (u32 base = r0; base < r1; base += 32) {
+                    const u32 u = base + lane;
+                    const bool act = u < r1;
+                    u32 o = 0, len = 0, beg = 0;
+                    s32 vw = 0;
+                    if (act) {
+                        o = label_of(a, u);
+                        vw = g_vw(a.g, u);
+                    }
+                    bool need = false;
+                    if (act) {
+                        const s64 ow = S.bw[o];
+                        if (ow > a.lmax)
+                            need = strong ? ((s64) vw <= 2 * (s64) maxv && (s64) vw < 2 * (ow - a.opt))
+                                          : 2 * (s64) vw < 3 * (ow - a.opt);
+                    }
+                    if (need) {
+                        len = __ldg(&a.g.rowlen[u]);
+                        beg = __ldg(&a.g.rowptr[u]);
+                    }
+                    const bool hub = need && len > TEAM_HUB;
+                    RowOut r{0, 0, 0, 0};
+                    const u32 ms = __ballot_sync(FULL, need && len <= 4 * GL);
+                    const u32 ml = __ballot_sync(FULL, need && len > 4 * GL && !hub);
+                    if (strong) {
+                        rows_short<OP_STRONG, GL>(a, S, ms, beg, len, o, max_b_w, r);
+                        rows_long<OP_STRONG>(a, S, ml, beg, len, o, max_b_w, r);
+                    } else {
+                        rows_short<OP_WEAK, GL>(a, S, ms, beg, len, o, max_b_w, r);
+                        rows_long<OP_WEAK>(a, S, ml, beg, len, o, max_b_w, r);
+                    }
+                    u32 key = NOKEY;
+                    if (need && !hub) key = finish(u, o, vw, r);
+                    if (act && !hub) a.keys[u] = key;
+                    // one add per distinct key of the warp
+                    const u32 peers = __match_any_sync(FULL, key);
+                    if (__any_sync(FULL, key != NOKEY)) {
+                        s32 p, t;
+                        peer_prefix(peers, vw, p, t);
+                        if (key != NOKEY && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(&a.hist[key], (u32) t);
+                    }
+                    const u32 sh = warp_append(&cnt[TC_HUB], hub);
+                    if (hub) a.hubs[sh] = u;
+                }
+                TEAM_SYNC();
+                if (blockIdx.x == 0 && tid < TC_N) cnt_o[tid] = 0;
+                if (blockIdx.x == 0 && tid < TS_N) sum_o[tid] = 0;
+                const u32 nhub = __ldcg(&cnt[TC_HUB]);
+                if (nhub) {
+                    for (u32 i = blockIdx.x; i < nhub; i += G) {
+                        const u32 u = a.hubs[i], o = label_of(a, u);
+                        row_add(a, __ldg(&a.g.rowptr[u]), __ldg(&a.g.rowlen[u]), tid, blockDim.x, S.tab0);
+                        __syncthreads();
+                        if (warp == 0) {
+                            const RowOut r = strong ? row_finish<OP_STRONG>(a, S, S.tab0, o, max_b_w)
+                                                    : row_finish<OP_WEAK>(a, S, S.tab0, o, max_b_w);
+                            if (lane == 0) {
+                                const s32 vw = g_vw(a.g, u);
+                                const u32 key = finish(u, o, vw, r);
+                                a.keys[u] = key;
+                                if (key != NOKEY) atomicAdd(&a.hist[key], (u32) vw);
+                            }
+                        }
+                        __syncthreads();
+                    }
+                    TEAM_SYNC();
+                }
+                // per overloaded block: the bin in which the limit falls, by 8
+                // lanes over contiguous shares of the block's bins
+                for (u32 b = tid; b < k; b += blockDim.x) {
+                    S.tot[b] = 0;
+                    S.spill[b] = 0;
+                }
+                __syncthreads();
+                const u32 g = lane >> 3, gl = lane & 7;
+                for (u32 i0 = warp * 4; i0 < n_over; i0 += nw * 4) {
+                    const u32 i = i0 + g;
+                    const bool act = i < n_over;
+                    const u32 o = act ? S.olist[i] : 0;
+                    const u32 share = (a.width + 7) / 8;
+                    const u32 b0 = min(gl * share, a.width), b1 = min(b0 + share, a.width);
+                    const u32 *h = a.hist + (u64) o * a.width + sft;
+                    s32 mine = 0, last = 0;
+                    if (act) {
+#pragma unroll 8
+                        for (u32 x = b0; x < b1; ++x) mine += (s32) __ldcg(&h[x]);
+                        last = (s32) __ldcg(&h[a.width - 1]);
+                    }
+                    const s32 spill = act && strong ? (s32) __ldcg(&h[-1]) : 0;
+                    s32 inc = mine;
+#pragma unroll
+                    for (int d = 1; d < 8; d <<= 1) {
+                        const s32 y = __shfl_up_sync(FULL, inc, d, 8);
+                        if ((int) gl >= d) inc += y;
+                    }
+                    const s32 total = __shfl_sync(FULL, inc, 7, 8) + spill;
+                    s32 run = spill + inc - mine;
+                    const s32 limit = act ? S.bw[o] - a.lmax : 0;
+                    if (act && gl == 0) {
+                        // all bins but the last one of strong keys, which the
+                        // next block's range starts with (key = (o + 1) * width)
+                        S.tot[o] = strong ? total - last : total;
+                        S.spill[o] = spill;
+                        // no bin reaches the limit: all are taken; the bin of
+                        // the previous block reaches it: none is
+                        if (total < limit || spill >= limit) {
+                            S.cutkey[o] = total < limit ? NOKEY : 0u;
+                            S.cutbase[o] = 0;
+                        }
+                    }
+                    if (act && run < limit && limit <= run + mine) {
+                        u32 x = b0;
+                        for (; x < b1; ++x) {
+                            const s32 c = (s32) __ldcg(&h[x]);
+                            if (limit <= run + c) break;
+                            run += c;
+                        }
+                        S.cutkey[o] = o * a.width + sft + x;
+                        S.cutbase[o] = run;
+                    }
+                }
+                __syncthreads();
+                if (strong)
+                    // a block after an overloaded one whose own weight is
+                    // within the limit holds only that block's last bin
+                    for (u32 i = tid; i < n_over; i += blockDim.x) {
+                        const u32 o = S.olist[i];
+                        if (o + 1 < k && S.bw[o + 1] <= a.lmax) S.tot[o + 1] = (s32) __ldcg(&a.hist[(u64) (o + 1) * a.width]);
+                    }
+                // weight of each warp's candidates in the cut bins
+                for (u32 base = r0; base < r1; base += 32) {
+                    const u32 u = base + lane;
+                    if (u < r1) {
+                        const u32 key = a.keys[u];
+                        if (key != NOKEY) {
+                            const u32 o = (key - sft) / a.width;
+                            if (key == S.cutkey[o]) atomicAdd(&S.tab[o], g_vw(a.g, u));
+                        }
+                    }
+                }
+                __syncthreads();
+                for (u32 i = tid; i < n_over; i += blockDim.x) {
+                    const u32 o = S.olist[i];
+                    s32 run = 0;
+                    for (u32 w = 0; w < nw; ++w) {
+                        s32 *p = S.tab0 + w * S.stride + o;
+                        const s32 x = *p;
+                        *p = run;
+                        run += x;
+                    }
+                    a.tsum[(u64) o * G + blockIdx.x] = run;
+                }
+                TEAM_SYNC();
+                // weight before this block's share of the cut bins
+                for (u32 i0 = warp * 4; i0 < n_over; i0 += nw * 4) {
+                    const u32 i = i0 + g;
+                    const bool act = i < n_over;
+                    const u32 o = act ? S.olist[i] : 0;
+                    s32 x = 0;
+                    if (act)
+                        for (u32 b = gl; b < blockIdx.x; b += 8) x += __ldcg(&a.tsum[(u64) o * G + b]);
+#pragma unroll
+                    for (int d = 4; d > 0; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
+                    if (act && gl == 0) S.toff[o] = x;
+                }
+                // the bins are not read any more in this step: clear them
+                for (u32 i = blockIdx.x; i < n_over; i += G) {
+                    u32 *h = a.hist + (u64) S.olist[i] * a.width;
+                    for (u32 x = tid; x <= a.width; x += blockDim.x) h[x] = 0;
+                }
+                __syncthreads();
+                // selection in ascending vertex id
+                for (u32 base = r0; base < r1; base += 32) {
+                    const u32 u = base + lane;
+                    const u32 key = u < r1 ? a.keys[u] : NOKEY;
+                    if (__ballot_sync(FULL, key != NOKEY) == 0) continue;
+                    u32 o = 0;
+                    s32 vw = 0;
+                    bool take = false, cut = false;
+                    if (key != NOKEY) {
+                        o = (key - sft) / a.width;
+                        vw = g_vw(a.g, u);
+                        cut = key == S.cutkey[o];
+                        take = key < S.cutkey[o];
+                    }
+                    if (__any_sync(FULL, cut)) {
+                        const u32 peers = __match_any_sync(FULL, cut ? o : EMPTY);
+                        s32 p, t;
+                        peer_prefix(peers, vw, p, t);
+                        s32 before = 0;
+                        if (cut) before = S.tab[o];
+                        __syncwarp();
+                        if (cut) {
+                            if ((peers & ((1u << lane) - 1u)) == 0) S.tab[o] = before + t;
+                            const s32 score = S.cutbase[o] + S.toff[o] + before + p;
+                            const s32 limit = S.bw[o] - a.lmax;
+                            take = score < limit;
+                            if (strong && take && score + vw >= limit) a.ea[o] = score + vw;
+                        }
+                        __syncwarp();
+                    }
+                    if (take && !strong) {
+                        const u32 nu = a.dest[u];
+                        team_move(a, S, u, o, nu, vw, stamp);
+                        entries += __ldg(&a.g.rowlen[u]);
+                    }
+                    const u32 s = warp_append(&cnt[TC_MOVES], take);
+                    if (take) {
+                        a.moves[s] = u;
+                        if (strong) {
+                            a.mcomp[s] = ((unsigned long long) key << 32) | u;
+                            a.mow[s] = ((unsigned long long) o << 32) | (u32) vw;
+                        }
+                    }
+                }
+                __syncwarp();
+                for (u32 i = lane; i < n_over; i += 32) S.tab[S.olist[i]] = 0;
+                if (strong) {
+                    TEAM_SYNC();
+                    const u32 ns = __ldcg(&cnt[TC_MOVES]);
+                    if (ns > TEAM_RANK_MAX) {
+                        if (blockIdx.x == 0 && tid == 0) a.out->gave_up = 1;
+                        return;
+                    }
+                    // cookie cutter (:524-551): evicted weight before each
+                    // block and free capacity up to each block
+                    long long c1 = 0, c2 = 0;
+                    for (u32 b0 = 0; b0 < k; b0 += blockDim.x) {
+                        const u32 b = b0 + tid;
+                        long long add = 0, cap = 0;
+                        if (b < k) {
+                            add = __ldcg(&a.ea[b]);
+                            if (add == 0) add = S.tot[b];
+                            cap = max_b_w > S.bw[b] ? (long long) max_b_w - S.bw[b] : 0;
+                        }
+                        long long t1, t2;
+                        const long long p1 = block_exclusive_scan<long long>(add, t1, sl);
+                        const long long p2 = block_exclusive_scan<long long>(cap, t2, sl);
+                        if (b < k) {
+                            S.pre[b] = c1 + p1;
+                            S.es[b + 1] = c2 + p2 + cap;
+                        }
+                        c1 += t1;
+                        c2 += t2;
+                    }
+                    if (tid == 0) S.es[0] = 0;
+                    __syncthreads();
+                    // exact prefix of each evicted vertex among its block's
+                    // and the first slot attempt (adjust_scores :560-584)
+                    for (u32 j0 = gw * 4; j0 < ns; j0 += gwarps * 4) {
+                        const u32 j = j0 + g;
+                        const bool act = j < ns;
+                        unsigned long long comp = 0, ow = 0;
+                        if (act) {
+                            comp = a.mcomp[j];
+                            ow = a.mow[j];
+                        }
+                        const u32 o = (u32) (ow >> 32);
+                        s32 x = 0;
+                        if (act) {
+#pragma unroll 4
+                            for (u32 i = gl; i < ns; i += 8) {
+                                const unsigned long long ci = a.mcomp[i], wi = a.mow[i];
+                                if ((u32) (wi >> 32) == o && ci < comp) x += (s32) (u32) wi;
+                            }
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int d = 4; d > 0; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
+                        if (act && gl == 0) {
+                            const u32 u = (u32) comp;
+                            const s32 vw = (s32) (u32) ow;
+                            const long long tg = (long long) S.spill[o] + x + S.pre[o];
+                            const s32 id = chunk_of(S.es, k, tg);
+                            const bool fits = id < (s32) k && (long long) (vw / 2) <= S.es[id + 1] - tg;
+                            if (!fits && id < (s32) k) {
+                                a.cand[atomicAdd(&cnt[TC_FAIL], 1u)] = u;
+                            } else {
+                                team_move(a, S, u, o, fits ? (u32) id : o, vw, stamp);
+                            }
+                            entries += __ldg(&a.g.rowlen[u]);
+                        }
+                        __syncwarp();
+                    }
+                    team_add(entries, &sum[TS_ENTRIES], sl);
+                    team_flush_bw(a, S);
+                    TEAM_SYNC();
+                    const u32 nf = __ldcg(&cnt[TC_FAIL]);
+                    if (nf) {
+                        // fallback slots in ascending vertex id (block 0)
+                        if (blockIdx.x == 0) {
+                            for (u32 j = tid; j < nf; j += blockDim.x) {
+                                const u32 u = a.cand[j];
+                                u32 p = 0;
+                                for (u32 i = 0; i < nf; ++i) p += a.cand[i] < u;
+                                a.hubs[p] = u;
+                            }
+                            __syncthreads();
+                            if (tid == 0) {
+                                long long mv = c1;
+                                for (u32 j = 0; j < nf; ++j) {
+                                    const u32 u = a.hubs[j];
+                                    const u32 o = label_of(a, u);
+                                    const s32 vw = g_vw(a.g, u);
+                                    u32 dest = o;
+                                    for (u32 guard = 0; guard < 2 * k + 4; ++guard) {
+                                        const long long tg = mv;
+                                        mv += vw;
+                                        const s32 id = chunk_of(S.es, k, tg);
+                                        if (id >= (s32) k) break;
+                                        if ((long long) (vw / 2) <= S.es[id + 1] - tg) {
+                                            dest = (u32) id;
+                                            break;
+                                        }
+                                    }
+                                    team_move(a, S, u, o, dest, vw, stamp);
+                                }
+                            }
+                            __syncthreads();
+                            team_flush_bw(a, S);
+                        }
+                        TEAM_SYNC();
+                    }
+                } else {
+                    team_add(entries, &sum[TS_ENTRIES], sl);
+                    team_flush_bw(a, S);
+                    TEAM_SYNC();
+                }
+            }
+            // exact objective change and the neighbours' cache resets
+            const u32 nm = __ldcg(&cnt[TC_MOVES]);
+            const bool inval = (unsigned long long) __ldcg(&sum[TS_ENTRIES]) < a.inval_all_min;
+            const s32 new_maxw = team_load_bw(a, S, smx);
+            long long acc = 0;
+            {
+                const u32 g = lane >> 3, gl = lane & 7;
+                for (u32 base = gw * 4; base < nm; base += gwarps * 4) {
+                    const u32 i = base + g;
+                    u32 u = 0, len = 0, beg = 0;
+                    unsigned long long x = 0;
+                    if (i < nm) {
+                        u = a.moves[i];
+                        len = __ldg(&a.g.rowlen[u]);
+                        beg = __ldg(&a.g.rowptr[u]);
+                        x = a.tw[u];
+                    }
+                    if (len <= TEAM_LONG)
+                        acc += team_delta<MAP>(a, S, tw_old(x), tw_label(x), tw_stamp(x) == stamp, stamp, beg, len, gl, 8,
+                                               inval);
+                    __syncwarp();
+                    u32 lng = __ballot_sync(FULL, gl == 0 && len > TEAM_LONG);
+                    while (lng) {
+                        const int src = __ffs(lng) - 1;
+                        lng &= lng - 1;
+                        const u32 xl = __shfl_sync(FULL, len, src), xb = __shfl_sync(FULL, beg, src);
+                        const unsigned long long xx = __shfl_sync(FULL, x, src);
+                        acc += team_delta<MAP>(a, S, tw_old(xx), tw_label(xx), tw_stamp(xx) == stamp, stamp, xb, xl, lane,
+                                               32, inval);
+                    }
+                }
+            }
+            if (!inval)
+                for (u32 u = r0 + lane; u < r1; u += 32) a.dest_cache[u] = NULL_PART;
+            team_add(acc, &sum[TS_DELTA], sl);
+            TEAM_SYNC();
+            const long long d = __ldcg(&sum[TS_DELTA]);
+            // control (jet_label_propagation.h:966-1030, promap :1250-1305)
+            if (!MAP) {
+                if (nm == 0) {
+                    if (lp_iter || balance_iteration >= JET_MAX_WEAK_ITERATIONS) break;
+                    balance_iteration = JET_MAX_WEAK_ITERATIONS;
+                    continue;
+                }
+                if (!lp_iter) balance_iteration++;
+            } else if (nm == 0) {
+                continue;
+            }
+            obj += MAP ? d : d / 2;
+            maxw = new_maxw;
+            bool copy = false;
+            const bool leq = MAP ? (maxw < best_max) : (maxw <= best_max);
+            if (best_max > a.lmax && maxw < best_max) {
+                copy = true;
+                iteration = 0;
+            } else if (obj < best_obj && (maxw <= a.lmax || leq)) {
+                if (1000 * obj < 999 * best_obj) iteration = 0;  // PHI = 0.999
+                copy = true;
+            }
+            if (copy) {
+                best_obj = obj;
+                best_max = maxw;
+                // labels change again after the next barrier at the earliest
+                for (u32 u = r0 + lane; u < r1; u += 32) a.part[u] = label_of(a, u);
+            }
+        }
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        a.out->obj = best_obj;
+        a.out->maxw = best_max;
+        a.out->iterations = iterations;
+    }
+}
+
+#undef TEAM_SYNC

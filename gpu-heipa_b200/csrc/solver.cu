@@ -209,6 +209,7 @@ void run_hm_tasks(Ctx &ctx, std::vector<HmTask> &tasks, Fn fn) {
     std::vector<Ctx *> wc(W);
     for (size_t w = 0; w < W; ++w) {
         wc[w] = &ctx.worker(w);
+        wc[w]->peers = ctx.peers * (u32) W;
         wc[w]->arena.attach(slab + w * slice, slice);
     }
     std::atomic<size_t> next{0};

@@ -1,0 +1,80 @@
+"""The single-launch Jet level loop (cluster and cooperative-grid teams) against the oracle at the sizes where it can go
+wrong: levels of one to a few vertices, row lengths around the tiers (8 lanes x 4 entries, a warp, 64-entry and 1024-entry
+limits), block counts around the table layouts (256 / 257, 1024), several mini-buckets per gain bucket, one overloaded
+block, and evictions that need fallback slots. Integer results: equality."""
+import numpy as np
+import pytest
+
+import gpu_heipa as H
+import oracle as O
+from helpers import isolated_plus_path, star, to_oracle
+
+pytestmark = pytest.mark.gpu
+
+TEAMS = {"cluster": {"jet_fused_max_n": 65536, "jet_fused_max_m": 1 << 30, "jet_coop_max_n": 0},
+         "grid": {"jet_fused_max_n": 0, "jet_coop_max_n": 1 << 24, "jet_coop_max_deg": 1 << 20, "jet_coop_rows": 64}}
+
+
+def wheel(lens):
+    """Hubs of the given row lengths over one shared ring of vertices."""
+    n_ring = max(lens)
+    edges = {(i, (i + 1) % n_ring) for i in range(n_ring)} if n_ring > 2 else set()
+    for h, ln in enumerate(lens):
+        edges |= {(j, n_ring + h) for j in range(ln)}
+    e = np.array(sorted({(min(a, b), max(a, b)) for a, b in edges}), np.int64)
+    both = np.concatenate([e, e[:, ::-1]])
+    both = both[np.lexsort((both[:, 1], both[:, 0]))]
+    n = n_ring + len(lens)
+    xadj = np.concatenate([[0], np.cumsum(np.bincount(both[:, 0], minlength=n))])
+    lo, hi = both.min(1), both.max(1)
+    return H.Graph(xadj, both[:, 1], (lo * 7 + hi * 3) % 9 + 1)
+
+
+def weighted(g, seed):
+    return H.Graph(g.xadj, g.adj, g.ew, np.random.default_rng(seed).integers(1, 40, g.n).astype(np.int32))
+
+
+CASES = {
+    "one_vertex": (isolated_plus_path(1, 0), 4, None),
+    "path": (isolated_plus_path(3, 30), 2, None),
+    "tier_rows": (wheel([1, 8, 31, 32, 33, 63, 64, 65, 127, 128, 129]), 5, None),
+    "hub_rows": (wheel([1023, 1024, 1025, 1500, 2100]), 64, None),
+    "star": (star(3000), 3, None),
+    "k256": (H.Graph.rmat(12, 12, seed=4), 256, None),
+    "k257": (H.Graph.rmat(12, 12, seed=5), 257, None),
+    "k1024": (weighted(H.Graph.rmat(13, 8, seed=6), 1), 1024, None),
+    "sections": (weighted(H.Graph.rgg3d(30011, 9.0, 1, 9, seed=2), 3), 2, None),
+    "heavy_vertices": (weighted(H.Graph.grid(61, 67, 1, 5, seed=3), 5), 24, None),
+    "map256": (H.Graph.rgg3d(6007, 30.0, 1, 50, seed=7), 256, ([4, 8, 8], [1, 10, 100])),
+    "map_hubs": (wheel([40, 64, 65, 1024, 1030, 1300]), 24, ([2, 4, 3], [1, 10, 100])),
+}
+
+
+@pytest.mark.parametrize("team", sorted(TEAMS))
+@pytest.mark.parametrize("start", ["spread", "one_block"])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_team_loop_equals_oracle(name, start, team):
+    g, k, hd = CASES[name]
+    og = to_oracle(g)
+    rng = np.random.default_rng(11)
+    part = rng.integers(0, k, g.n).astype(np.uint32)
+    if start == "one_block":  # most of the weight in the last block
+        part[rng.random(g.n) < 0.6] = k - 1
+    vw = np.ones(g.n, np.int64) if g.vw is None else g.vw
+    lmax = O.lmax(g.total_weight(), k, 0.03)
+    maxw = int(np.bincount(part, weights=vw, minlength=k).max())
+    hier, dist = hd if hd else (None, None)
+    obj = O.comm_cost(og, part, hier, dist) if hd else O.edge_cut(og, part)
+    c = H.Context(0, 512 << 20)
+    try:
+        for t, v in TEAMS[team].items():
+            c.tune(t, v)
+        dg = c.upload(g)
+        for ultra in ((False,) if hd else (False, True)):
+            got = c.jet_refine(dg, k, lmax, part, obj, maxw, ultra=ultra, level=0, hierarchy=hier, distance=dist)
+            want = O.jet_refine(og, k, lmax, ultra, 0, part, obj, maxw, hier, dist)
+            assert got[1:] == want[1:]
+            np.testing.assert_array_equal(got[0], want[0])
+        dg.free()
+    finally:
+        c.close()
