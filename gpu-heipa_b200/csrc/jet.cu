@@ -2692,12 +2692,18 @@ void JetLevel::run_step(int kind, u32 ratio_pct) {
 
 // ---- host side of the single-launch level loop ------------------------------------------
 
+constexpr u32 TEAM_BLOCK_THREADS = 512;
 constexpr u32 TEAM_CLUSTER_THREADS = 512;
 constexpr u32 TEAM_GRID_THREADS = 1024;
+constexpr size_t TEAM_BLOCK_SMEM = 226 * 1024;  // dynamic shared memory of a block team
 // vertices per block of a cluster team (up to its largest size): 4 rows per warp
 constexpr u32 TEAM_CLUSTER_ROWS = 64;
 constexpr u32 TEAM_CLUSTER_MAX_N = 1u << 16;  // upper bound of Tunables::jet_fused_max_n
 constexpr u32 TEAM_PEER_BLOCKS = 40;
+// Block teams: what fits in shared memory. The cluster took 14.7 us per
+// iteration on the levels of up to 1700 vertices of an RGG with 3001 vertices,
+// one block with the level in shared memory 10.5 us.
+constexpr u32 TEAM_BLOCK_MAX_N = 4096;
 // Levels above Tunables::jet_coop_max_deg entries per vertex run as a grid
 // team up to these sizes. Barriers dominate small levels whatever their
 // degree (ultra R-MAT 65k, levels of up to 600 entries per vertex: 302 ms with
@@ -2708,20 +2714,28 @@ constexpr u32 TEAM_PEER_BLOCKS = 40;
 constexpr u64 TEAM_ANY_DEG_M = 1ull << 21;
 constexpr u64 TEAM_MID_DEG_M = 1ull << 26, TEAM_MID_DEG = 128;
 
-template<bool CLUSTER>
-static const void *team_kernel(u32 k, bool promap) {
-    if (promap) return (const void *) k_jet_team<CLUSTER, 8, true>;
-    return k <= 256 ? (const void *) k_jet_team<CLUSTER, 8, false> : (const void *) k_jet_team<CLUSTER, 32, false>;
+static const void *team_kernel(int team, u32 k, bool promap) {
+    if (team == TEAM_BLOCK) {
+        if (promap) return (const void *) k_jet_block<8, true>;
+        return k <= 256 ? (const void *) k_jet_block<8, false> : (const void *) k_jet_block<32, false>;
+    }
+    if (team == TEAM_CLUSTER) {
+        if (promap) return (const void *) k_jet_team<TEAM_CLUSTER, 8, true>;
+        return k <= 256 ? (const void *) k_jet_team<TEAM_CLUSTER, 8, false>
+                        : (const void *) k_jet_team<TEAM_CLUSTER, 32, false>;
+    }
+    if (promap) return (const void *) k_jet_team<TEAM_GRID, 8, true>;
+    return k <= 256 ? (const void *) k_jet_team<TEAM_GRID, 8, false> : (const void *) k_jet_team<TEAM_GRID, 32, false>;
 }
 
 static cudaLaunchConfig_t team_config(u32 blocks, u32 threads, size_t smem, cudaStream_t stream,
-                                      cudaLaunchAttribute &attr, bool cluster) {
+                                      cudaLaunchAttribute &attr, int team) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    if (cluster) {
+    if (team == TEAM_CLUSTER) {
         attr.id = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = blocks;
         attr.val.clusterDim.y = 1;
@@ -2731,7 +2745,7 @@ static cudaLaunchConfig_t team_config(u32 blocks, u32 threads, size_t smem, cuda
         attr.val.cooperative = 1;
     }
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = team == TEAM_BLOCK ? 0 : 1;
     return cfg;
 }
 
@@ -2748,15 +2762,17 @@ static u32 team_limits(int device) {
     for (int i = 0; i < 3; ++i) {
         const bool promap = i == 2;
         const u32 k = i == 0 ? JW_SLOTS : 256;
-        const void *kc = team_kernel<true>(k, promap), *kg = team_kernel<false>(k, promap);
+        const void *kc = team_kernel(TEAM_CLUSTER, k, promap), *kg = team_kernel(TEAM_GRID, k, promap);
         const size_t sc = team_smem(k, TEAM_CLUSTER_THREADS / 32, promap);
         const size_t sg = team_smem(k, TEAM_GRID_THREADS / 32, promap);
         HP_CUDA(cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sc));
         HP_CUDA(cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sg));
+        HP_CUDA(cudaFuncSetAttribute(team_kernel(TEAM_BLOCK, k, promap), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int) TEAM_BLOCK_SMEM));
         HP_CUDA(cudaFuncSetAttribute(kc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         for (; best > 1; best /= 2) {
             cudaLaunchAttribute attr;
-            const cudaLaunchConfig_t cfg = team_config(best, TEAM_CLUSTER_THREADS, sc, nullptr, attr, true);
+            const cudaLaunchConfig_t cfg = team_config(best, TEAM_CLUSTER_THREADS, sc, nullptr, attr, TEAM_CLUSTER);
             int fits = 0;
             if (cudaOccupancyMaxActiveClusters(&fits, kc, &cfg) == cudaSuccess && fits > 0) break;
             cudaGetLastError();
@@ -2766,74 +2782,94 @@ static u32 team_limits(int device) {
     return best;
 }
 
-// Runs the level loop in one k_jet_team launch (direct-indexed tables): part
-// receives the best labelling. `saved` receives the input labels. Throws
-// CoopSpin when the loop gave up (barrier wait, or too many evictions to
-// rank); part is then to be restored from saved.
+// Offset of a block team's level arrays in its shared memory.
+static size_t team_level_offset(u32 k, bool promap) { return team_smem(k, TEAM_BLOCK_THREADS / 32, promap); }
+
+// Runs the level loop in one launch (direct-indexed tables): part receives
+// the best labelling. `saved` receives the input labels (cluster and grid
+// teams). Throws CoopSpin when the loop gave up (barrier wait, or too many
+// evictions to rank); part is then to be restored from saved.
 static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const std::vector<u32> &ratios,
                             const DistOracle *D, unsigned long long inval_all_min, u32 *part, u32 *saved, s64 &obj,
-                            s32 &maxw, bool cluster, u32 blocks) {
+                            s32 &maxw, int team, u32 blocks) {
     const u32 n = g.n;
     const bool promap = D != nullptr;
     TeamArgs a{};
-    a.g = g;
+    a.n = n;
+    a.rowptr = g.rowptr;
+    a.rowlen = g.rowlen;
+    a.adj = g.adj;
+    a.ew = g.ew;
+    a.vw = g.vw;
     a.k = k;
     a.lmax = lmax;
     a.opt = ((s32) g.total_vw + (s32) (k - 1)) / (s32) k;
     a.weak_max = std::max<s32>(lmax - 100, (s32) ((99 * (s64) lmax) / 100));
     a.strong_max = std::max<s32>(a.opt + 1, (s32) ((99 * (s64) lmax) / 100));
     sections_of(n, k, a.sections, a.width);
-    a.promap = promap ? 1u : 0u;
     a.code = promap ? D->code : nullptr;
     a.bitdist = promap ? D->bitdist : nullptr;
     a.inval_all_min = inval_all_min;
     a.part = part;
-    a.saved = saved;
-    a.tw = ctx.balloc<unsigned long long>(n);
-    a.abrec = ctx.balloc<unsigned long long>(n);
-    a.dest_cache = ctx.balloc<u32>(n);
-    a.gain_cache = ctx.balloc<s32>(n);
-    a.lock = ctx.balloc<u32>(n);
-    a.dest = ctx.balloc<u32>(n);
-    a.keys = ctx.balloc<u32>(n);
-    a.cand = ctx.balloc<u32>(n);
-    a.moves = ctx.balloc<u32>(n);
-    a.hubs = ctx.balloc<u32>(n);
-    a.mcomp = ctx.balloc<unsigned long long>(n);
-    a.mow = ctx.balloc<unsigned long long>(n);
-    a.tsum = ctx.balloc<s32>((u64) k * blocks);
-    a.ea = ctx.balloc<s32>(k);
-    // zeroed words in one allocation: outcome, sums, counters, barrier, block
-    // weights, bins
-    const size_t bins = (size_t) k * a.width + 2;
-    const size_t zero_bytes = sizeof(TeamOut) + 2 * TS_N * sizeof(long long) + (2 * TC_N + 2 + k + bins) * sizeof(u32);
-    char *z = ctx.balloc<char>(zero_bytes);
-    HP_CUDA(cudaMemsetAsync(z, 0, zero_bytes, ctx.stream));
-    a.out = (TeamOut *) z;
-    a.sum = (long long *) (a.out + 1);
-    a.cnt = (u32 *) (a.sum + 2 * TS_N);
-    a.bar = a.cnt + 2 * TC_N;
-    a.bw = (s32 *) (a.bar + 2);
-    a.hist = (u32 *) (a.bw + k);
     TeamCtl ctl{};
     ctl.n_ratios = (u32) ratios.size();
     for (size_t i = 0; i < ratios.size() && i < 17; ++i) ctl.ratios[i] = ratios[i];
     ctl.obj = obj;
     ctl.maxw = maxw;
-    const u32 threads = cluster ? TEAM_CLUSTER_THREADS : TEAM_GRID_THREADS;
-    const size_t smem = team_smem(k, threads / 32, promap);
-    const void *kern = cluster ? team_kernel<true>(k, promap) : team_kernel<false>(k, promap);
     std::optional<CoopGuard> coop;  // cooperative budget (grid blocks), until the kernel has completed
-    if (!cluster) coop.emplace(ctx.device, ctx.stream, blocks, (u32) ctx.sm_count);
-    {
-        KernTimer kt(ctx, cluster ? "k_jet_fused" : "k_jet_coop");
-        cudaLaunchAttribute attr;
-        const cudaLaunchConfig_t cfg = team_config(blocks, threads, smem, ctx.stream, attr, cluster);
+    const void *kern = team_kernel(team, k, promap);
+    cudaLaunchAttribute attr;
+    if (team == TEAM_BLOCK) {
+        a.out = ctx.balloc<TeamOut>(1);
+        HP_CUDA(cudaMemsetAsync(a.out, 0, sizeof(TeamOut), ctx.stream));
+        u32 m = (u32) g.m, level = (u32) team_level_offset(k, promap);
+        const size_t smem = level + team_level_smem(n, m, k, a.width);
+        KernTimer kt(ctx, "k_jet_fused");
+        const cudaLaunchConfig_t cfg = team_config(1, TEAM_BLOCK_THREADS, smem, ctx.stream, attr, team);
+        void *args[] = {&a, &ctl, &m, &level};
+        HP_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
+        note_launch();
+    } else {
+        a.saved = saved;
+        a.tw = ctx.balloc<unsigned long long>(n);
+        a.abrec = ctx.balloc<unsigned long long>(n);
+        a.dest_cache = ctx.balloc<u32>(n);
+        a.gain_cache = ctx.balloc<s32>(n);
+        a.lock = ctx.balloc<u32>(n);
+        a.dest = ctx.balloc<u32>(n);
+        a.keys = ctx.balloc<u32>(n);
+        a.clist = ctx.balloc<u32>(n);
+        a.mlist = ctx.balloc<u32>(n);
+        a.hubs = ctx.balloc<u32>(n);
+        a.fails = a.clist;  // candidates belong to label propagation, fallbacks to strong rebalancing
+        a.mcomp = ctx.balloc<unsigned long long>(n);
+        a.mow = ctx.balloc<unsigned long long>(n);
+        a.tsum = ctx.balloc<s32>((u64) k * blocks);
+        a.ea = ctx.balloc<s32>(k);
+        // zeroed words in one allocation: outcome, sums, counters, barrier,
+        // block weights, bins
+        const size_t bins = (size_t) k * a.width + 2;
+        const size_t zero_bytes =
+            sizeof(TeamOut) + 2 * TS_N * sizeof(long long) + (2 * TC_N + 2 + k + bins) * sizeof(u32);
+        char *z = ctx.balloc<char>(zero_bytes);
+        HP_CUDA(cudaMemsetAsync(z, 0, zero_bytes, ctx.stream));
+        a.out = (TeamOut *) z;
+        a.sum = (long long *) (a.out + 1);
+        a.cnt = (u32 *) (a.sum + 2 * TS_N);
+        a.bar = a.cnt + 2 * TC_N;
+        a.bw = (s32 *) (a.bar + 2);
+        a.hist = (u32 *) (a.bw + k);
+        const u32 threads = team == TEAM_CLUSTER ? TEAM_CLUSTER_THREADS : TEAM_GRID_THREADS;
+        const size_t smem = team_smem(k, threads / 32, promap);
+        if (team == TEAM_GRID) coop.emplace(ctx.device, ctx.stream, blocks, (u32) ctx.sm_count);
+        KernTimer kt(ctx, team == TEAM_CLUSTER ? "k_jet_fused" : "k_jet_coop");
+        const cudaLaunchConfig_t cfg = team_config(blocks, threads, smem, ctx.stream, attr, team);
         void *args[] = {&a, &ctl};
         HP_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
         note_launch();
     }
     static_assert(sizeof(TeamOut) <= sizeof(DevStatus), "the outcome is read through the pinned status mirror");
+    static_assert(sizeof(TeamOut) % 8 == 0, "64-bit sums follow the outcome");
     HP_CUDA(cudaMemcpyAsync(ctx.h_status, a.out, sizeof(TeamOut), cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();
     const TeamOut o = *(const TeamOut *) ctx.h_status;
@@ -2853,7 +2889,7 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
 // uncapped, 342 / 359 ms with at least 32 / 64 blocks each.
 static u32 coop_blocks(Ctx &ctx, u32 n, u64 m, u32 k, bool promap) {
     int per_sm = 0;
-    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, team_kernel<false>(k, promap), TEAM_GRID_THREADS,
+    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, team_kernel(TEAM_GRID, k, promap), TEAM_GRID_THREADS,
                                                           team_smem(k, TEAM_GRID_THREADS / 32, promap)));
     if (per_sm <= 0) return 0;
     const u64 rows = std::max<u32>(1, ctx.tune.jet_coop_rows);
@@ -2876,24 +2912,34 @@ void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultr
     else ratios = {level == 0 ? 25u : 75u};
     // small and mid-size levels: the whole loop in one launch
     if (direct_tables(k, promap) && !ctx.prof.enabled) {
-        u32 blocks = 0;
-        const bool cluster = g.n <= std::min<u32>(ctx.tune.jet_fused_max_n, TEAM_CLUSTER_MAX_N) && g.m <= ctx.tune.jet_fused_max_m;
+        u32 blocks = 0, sections, width;
+        int team = TEAM_GRID;
         const u32 max_cluster = team_limits(ctx.device);
-        if (cluster)
+        sections_of(g.n, k, sections, width);
+        const bool fused = g.n <= std::min<u32>(ctx.tune.jet_fused_max_n, TEAM_CLUSTER_MAX_N) &&
+                           g.m <= ctx.tune.jet_fused_max_m;
+        if (fused && g.n <= TEAM_BLOCK_MAX_N &&
+            team_level_offset(k, promap) + team_level_smem(g.n, g.m, k, width) <= TEAM_BLOCK_SMEM) {
+            team = TEAM_BLOCK;
+            blocks = 1;
+        } else if (fused) {
+            team = TEAM_CLUSTER;
             blocks = std::max<u32>(1, std::min<u32>(max_cluster, (g.n + TEAM_CLUSTER_ROWS - 1) / TEAM_CLUSTER_ROWS));
-        else if (g.n <= ctx.tune.jet_coop_max_n && g.m <= ctx.tune.jet_coop_max_m &&
-                 (g.m <= (u64) ctx.tune.jet_coop_max_deg * g.n || g.m <= TEAM_ANY_DEG_M ||
-                  (g.m <= TEAM_MID_DEG_M && g.m <= TEAM_MID_DEG * g.n)))
+        } else if (g.n <= ctx.tune.jet_coop_max_n && g.m <= ctx.tune.jet_coop_max_m &&
+                   (g.m <= (u64) ctx.tune.jet_coop_max_deg * g.n || g.m <= TEAM_ANY_DEG_M ||
+                    (g.m <= TEAM_MID_DEG_M && g.m <= TEAM_MID_DEG * g.n))) {
             blocks = coop_blocks(ctx, g.n, g.m, k, promap);
+        }
         if (blocks) {
             ScratchScope ss2(ctx.arena);
             u32 *saved = ctx.balloc<u32>(g.n);
             const unsigned long long inval = cache_pure ? (g.m * ctx.tune.jet_inval_all_pct + 99) / 100 : ~0ull;
             try {
-                jet_refine_team(ctx, g, k, lmax, ratios, D, inval, part, saved, obj, maxw, cluster, blocks);
+                jet_refine_team(ctx, g, k, lmax, ratios, D, inval, part, saved, obj, maxw, team, blocks);
                 return;
             } catch (const CoopSpin &) {
-                // the per-kernel loop redoes the level from its input labels
+                // (a block team ranks all it has) the per-kernel loop redoes
+                // the level from its input labels
                 HP_CUDA(cudaMemcpyAsync(part, saved, sizeof(u32) * g.n, cudaMemcpyDeviceToDevice, ctx.stream));
                 ctx.sync();  // saved is released here
             }

@@ -2,37 +2,40 @@
 //
 // A team of blocks runs every iteration of jet_refine: the iteration control
 // (ratios, weak / strong switching, best-labelling tracking) and the steps of
-// the per-kernel path, with the same result. The team is a thread-block
-// cluster on small levels (hardware barrier, co-scheduled by the hardware) or
-// a cooperative grid on larger ones (bounded grid barrier).
+// the per-kernel path, with the same result. The team is one block whose
+// shared memory holds the level (graph and state) on the smallest levels, a
+// thread-block cluster on small levels (hardware barrier, co-scheduled by the
+// hardware), or a cooperative grid on larger ones (bounded grid barrier).
 //
-// What bounds it: the latency of one iteration (levels of a few thousand to a
-// few million vertices, tens to hundreds of iterations, everything in L2), so
-// the design minimises barriers and dependent loads per iteration:
+// What bounds it: the latency of one iteration (levels of a few dozen to a few
+// million vertices, tens to hundreds of iterations, everything in L2). A phase
+// with little work is a chain of dependent L2 accesses of 0.3 us each, so the
+// design minimises barriers and dependent accesses per iteration:
 //  * a label-propagation iteration has three barriers: gains and filter, then
 //    afterburner and moves, then the objective change. A vertex word holds
 //    label, previous label and the iteration that changed it, so moves are
 //    applied while other blocks still read the previous labels, and nothing
 //    has to be unmarked afterwards;
+//  * every warp owns a contiguous vertex range and keeps its candidates and
+//    moves in a list of its own: no shared counters, no list lengths to read;
 //  * a rebalance iteration sorts nothing. Candidates add their weight to a
 //    histogram over the mini-bucket keys; per overloaded block the histogram
 //    gives the mini-bucket in which the limit falls, and only the candidates
 //    of that one need their order (ascending vertex id): per-warp weight sums
-//    over contiguous vertex ranges, prefix sums over them and a prefix within
-//    32 vertices. Strong rebalancing needs the exact prefix of every evicted
+//    over the vertex ranges, prefix sums over them and a prefix within 32
+//    vertices. Strong rebalancing needs the exact prefix of every evicted
 //    vertex: the few evicted ones are ranked among each other;
 //  * rows are evaluated by 8 lanes (32 lanes for k > 256) with a
 //    direct-indexed block table in shared memory: an entry costs one add and
 //    one exchange, which collects each distinct block once and clears the
 //    table; no pass over all k blocks.
-// Measured (one B200, mean time of one iteration): against one 1024-thread
-// block that ran the same steps, levels of up to 4096 vertices of an RGG with
-// 3001 vertices 27 -> 14 us; against a cooperative grid whose block 0 sorted
-// the candidates, levels of up to 65536 vertices of a 256x256 grid 62 -> 21 us,
-// of an R-MAT graph with 65536 vertices 280 -> 71 us. Between two barriers
-// about 3 us remain when there is little work: the barrier, the list length,
-// the list entry, the row bounds, the row and the neighbours' words are read
-// one after the other.
+// Measured (one B200, mean time of one iteration): the levels of an RGG with
+// 3001 vertices, 27 us with one 1024-thread block per level in global memory,
+// 14 us as cluster teams with shared lists, now 10.5 us on the levels that fit
+// a block team and 12.5 us as cluster; levels of up to 65536 vertices of a
+// 256x256 grid, 62 us as a cooperative grid whose block 0 sorted the
+// candidates, now 18 us; the levels of an R-MAT graph with 65536 vertices,
+// 280 us (largest two) before, now 67 us (all).
 #pragma once
 
 constexpr u32 TEAM_HUB = 1024;         // rows above this length are evaluated by a whole block
@@ -41,8 +44,12 @@ constexpr u32 TEAM_LIST = 128;         // distinct-block list slots per warp (ma
 constexpr u32 TEAM_RANK_MAX = 32768;   // evicted vertices ranked by counting; more are left to the per-kernel path
 constexpr u32 TEAM_CLUSTER_MAX = 16;   // blocks of a cluster team
 
-enum TeamCnt { TC_HUB = 0, TC_CAND = 1, TC_MOVES = 2, TC_FAIL = 3, TC_N = 4 };
-enum TeamSum { TS_ENTRIES = 0, TS_DELTA = 1, TS_N = 2 };
+constexpr u32 TEAM_OWN = 64;           // candidates / moves of a warp kept in shared memory up to this range
+
+enum TeamKind { TEAM_BLOCK = 0, TEAM_CLUSTER = 1, TEAM_GRID = 2 };
+enum TeamCnt { TC_HUB = 0, TC_MOVES = 1, TC_FAIL = 2, TC_N = 4 };
+enum TeamSum { TS_MOVES = 0, TS_DELTA = 1, TS_N = 2 };  // (moves << 32) + their row entries; objective change
+constexpr u32 TW_STILL = 0x80000000u;  // stamp flag: in the move list with an unchanged label
 
 // Vertex word: label (16 bits), previous label (16 bits), iteration that
 // changed the label (32 bits).
@@ -64,10 +71,14 @@ struct TeamOut {
     u32 iterations;
     u32 gave_up;     // 1: more than TEAM_RANK_MAX evicted vertices in one step, nothing was decided
     u32 err;         // DevErr bits
+    u32 hubs;        // some row is longer than TEAM_HUB
 };
 
 struct TeamArgs {
-    DGraph g;
+    u32 n;
+    const u32 *rowptr, *rowlen;  // block team: rowlen unused, rows are contiguous
+    const u32 *adj;
+    const s32 *ew, *vw;          // null: unit weights (never null in a block team)
     u32 k;
     s32 lmax;
     s32 opt;
@@ -78,7 +89,7 @@ struct TeamArgs {
     const s32 *bitdist;
     unsigned long long inval_all_min;
     u32 *part;                  // in: labels; out: best labelling
-    u32 *saved;                 // receives a copy of the input labels
+    u32 *saved;                 // receives a copy of the input labels (or null)
     unsigned long long *tw;     // vertex words
     unsigned long long *abrec;  // afterburner records: gain, target (16 bits), label (16 bits)
     u32 *dest_cache;
@@ -86,7 +97,8 @@ struct TeamArgs {
     u32 *lock;
     u32 *dest;                  // rebalance targets
     u32 *keys;                  // mini-bucket keys
-    u32 *cand, *moves, *hubs;
+    u32 *clist, *mlist;         // candidates and moves of each warp, from the start of its vertex range
+    u32 *hubs, *fails;          // long rows of a pass; evicted vertices that need a fallback slot
     unsigned long long *mcomp;  // strong: (key, vertex) of every evicted vertex
     unsigned long long *mow;    // strong: (block, vertex weight)
     s32 *bw;                    // zero on entry
@@ -106,6 +118,7 @@ struct TeamSm {
     s32 *tab0;     // the block's first table
     u32 stride;    // words between the tables of two warps
     unsigned long long *list;  // this warp's distinct-block list (mapping objective)
+    u32 *own;      // this warp's candidate and move lists (2 * TEAM_OWN)
     s32 *bw, *bd, *cutbase, *tot, *spill, *toff;
     u32 *under, *olist, *cutkey;
     long long *es, *pre;
@@ -113,14 +126,24 @@ struct TeamSm {
     s32 *dist;
 };
 
+// vertex words 8, records (or targets and keys) 8, evicted 16, row offset,
+// weight, cached target, cached gain, lock, two lists 4 each
+constexpr size_t TEAM_VERTEX_BYTES = 8 + 8 + 16 + 7 * 4;
+
 // Bytes of dynamic shared memory of a team block of `warps` warps.
 inline size_t team_smem(u32 k, u32 warps, bool promap) {
     const size_t groups = k <= 256 ? 4 : 1;
     size_t b = (size_t) warps * groups * k * 4;
     b = (b + 15) & ~(size_t) 15;
     if (promap) b += (size_t) warps * std::max<u32>(TEAM_LIST, k) * 8;
-    b += ((size_t) k + 2) * 8 * 2 + (size_t) k * 4 * 10 + 32 * 4;
+    b += ((size_t) k + 2) * 8 * 2 + (size_t) k * 4 * 10 + 32 * 4 + (size_t) warps * 2 * TEAM_OWN * 4;
     return (b + 15) & ~(size_t) 15;
+}
+
+// Bytes of a level (graph, state, bins) in the shared memory of a block team.
+inline size_t team_level_smem(u32 n, u64 m, u32 k, u32 width) {
+    return (size_t) n * TEAM_VERTEX_BYTES + m * 8 + ((size_t) k * width + 2) * 4 + 64 +
+           (2 * TS_N) * 8 + (2 * TC_N + k + k) * 4 + 64;
 }
 
 template<int GL>
@@ -150,6 +173,7 @@ __device__ __forceinline__ TeamSm team_carve(unsigned char *base, u32 k, u32 war
     S.cutkey = (u32 *) (p + 8 * k);
     S.code = (u32 *) (p + 9 * k);
     S.dist = p + 10 * k;
+    S.own = (u32 *) (S.dist + 32) + warp * 2 * TEAM_OWN;
     return S;
 }
 
@@ -163,9 +187,13 @@ __device__ __forceinline__ TeamSm team_carve(unsigned char *base, u32 k, u32 war
 constexpr u32 TEAM_POISON = 0x80000000u;
 constexpr u32 TEAM_SPINS = 1u << 21;
 
-template<bool CLUSTER>
+template<int TEAM>
 __device__ __forceinline__ bool team_barrier(u32 *bar, u32 &target, u32 *err) {
-    if (CLUSTER) {
+    if (TEAM == TEAM_BLOCK) {
+        __syncthreads();
+        return true;
+    }
+    if (TEAM == TEAM_CLUSTER) {
         asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
         return true;
     }
@@ -189,6 +217,32 @@ __device__ __forceinline__ bool team_barrier(u32 *bar, u32 &target, u32 *err) {
     }
     __syncthreads();
     return s_ok != 0u;
+}
+
+// Graph reads: the level is in shared memory (block team) or constant in
+// global memory.
+template<int TEAM, typename T>
+__device__ __forceinline__ T ld_graph(const T *p) {
+    return TEAM == TEAM_BLOCK ? *p : __ldg(p);
+}
+template<int TEAM>
+__device__ __forceinline__ s32 ld_ew(const TeamArgs &a, u64 e) {
+    return TEAM == TEAM_BLOCK ? a.ew[e] : (a.ew ? __ldg(&a.ew[e]) : 1);
+}
+template<int TEAM>
+__device__ __forceinline__ s32 ld_vw(const TeamArgs &a, u32 u) {
+    return TEAM == TEAM_BLOCK ? a.vw[u] : (a.vw ? __ldg(&a.vw[u]) : 1);
+}
+template<int TEAM>
+__device__ __forceinline__ void ld_row(const TeamArgs &a, u32 u, u32 &beg, u32 &len) {
+    beg = ld_graph<TEAM>(&a.rowptr[u]);
+    len = TEAM == TEAM_BLOCK ? a.rowptr[u + 1] - beg : __ldg(&a.rowlen[u]);
+}
+// A word that other blocks wrote before the last barrier and that steers the
+// control flow: from L2, or shared memory.
+template<int TEAM, typename T>
+__device__ __forceinline__ T ld_fresh(const T *p) {
+    return TEAM == TEAM_BLOCK ? *(const volatile T *) p : __ldcg(p);
 }
 
 // ---- row evaluation --------------------------------------------------------------------
@@ -265,7 +319,7 @@ __device__ __forceinline__ u32 label_of(const TeamArgs &a, u32 v) { return ((con
 // Evaluates the rows of the lanes in `need` (beg, len <= 4 * GL, own block o
 // of each lane's row), 32 / GL rows at a time, GL lanes per row; every lane
 // receives its row's result. All lanes of the warp call this.
-template<int OP, int GL>
+template<int TEAM, int OP, int GL>
 __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u32 need, u32 beg, u32 len, u32 o,
                                            s32 max_b_w, RowOut &out) {
     constexpr int NG = 32 / GL;
@@ -288,8 +342,8 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const u32 t = gl + j * GL;
-            b[j] = t < rl ? __ldg(&a.g.adj[(u64) rb + t]) : EMPTY;
-            w[j] = t < rl ? g_ew(a.g, (u64) rb + t) : 0;
+            b[j] = t < rl ? ld_graph<TEAM>(&a.adj[(u64) rb + t]) : EMPTY;
+            w[j] = t < rl ? ld_ew<TEAM>(a, (u64) rb + t) : 0;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -336,6 +390,7 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
 }
 
 // Adds entries first, first + step, ... of a row to the direct table tv.
+template<int TEAM>
 __device__ __forceinline__ void row_add(const TeamArgs &a, u32 beg, u32 len, u32 first, u32 step, s32 *tv) {
     for (u32 t0 = first; t0 < len; t0 += 4 * step) {
         u32 b[4];
@@ -343,8 +398,8 @@ __device__ __forceinline__ void row_add(const TeamArgs &a, u32 beg, u32 len, u32
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const u32 t = t0 + j * step;
-            b[j] = t < len ? __ldg(&a.g.adj[(u64) beg + t]) : EMPTY;
-            w[j] = t < len ? g_ew(a.g, (u64) beg + t) : 0;
+            b[j] = t < len ? ld_graph<TEAM>(&a.adj[(u64) beg + t]) : EMPTY;
+            w[j] = t < len ? ld_ew<TEAM>(a, (u64) beg + t) : 0;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -389,14 +444,14 @@ __device__ __forceinline__ RowOut row_finish(const TeamArgs &a, const TeamSm &S,
 }
 
 // Evaluates the rows of the lanes in `need`, one at a time by the whole warp.
-template<int OP>
+template<int TEAM, int OP>
 __device__ __forceinline__ void rows_long(const TeamArgs &a, const TeamSm &S, u32 need, u32 beg, u32 len, u32 o,
                                           s32 max_b_w, RowOut &out) {
     while (need) {
         const int src = __ffs(need) - 1;
         need &= need - 1;
         const u32 rb = __shfl_sync(FULL, beg, src), rl = __shfl_sync(FULL, len, src), ro = __shfl_sync(FULL, o, src);
-        row_add(a, rb, rl, lane_id(), 32, S.tab);
+        row_add<TEAM>(a, rb, rl, lane_id(), 32, S.tab);
         __syncwarp();
         const RowOut r = row_finish<OP>(a, S, S.tab, ro, max_b_w);
         if (lane_id() == src) out = r;
@@ -441,12 +496,12 @@ __device__ __forceinline__ void team_move(const TeamArgs &a, const TeamSm &S, u3
         atomicAdd(&S.bd[nu], vw);
     }
     a.tw[u] = (unsigned long long) nu | ((unsigned long long) ou << 16) |
-              ((unsigned long long) (ou != nu ? stamp : 0u) << 32);
+              ((unsigned long long) (ou != nu ? stamp : stamp | TW_STILL) << 32);
     a.dest_cache[u] = NULL_PART;
 }
 
 // Afterburner terms of up to four loaded entries (ab_batch over abrec).
-template<bool MAP>
+template<int TEAM, bool MAP>
 __device__ __forceinline__ s32 team_ab(const TeamArgs &a, const TeamSm &S, u32 u, s32 ug, u32 ou, u32 nu, u32 beg,
                                        u32 len, u32 first, u32 step) {
     s32 change = 0;
@@ -457,8 +512,8 @@ __device__ __forceinline__ s32 team_ab(const TeamArgs &a, const TeamSm &S, u32 u
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const u32 t = t0 + j * step;
-            v[j] = t < len ? __ldg(&a.g.adj[(u64) beg + t]) : SENTINEL;
-            w[j] = t < len ? g_ew(a.g, (u64) beg + t) : 0;
+            v[j] = t < len ? ld_graph<TEAM>(&a.adj[(u64) beg + t]) : SENTINEL;
+            w[j] = t < len ? ld_ew<TEAM>(a, (u64) beg + t) : 0;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) x[j] = v[j] != SENTINEL ? a.abrec[v[j]] : 0ull;
@@ -482,7 +537,7 @@ __device__ __forceinline__ s32 team_ab(const TeamArgs &a, const TeamSm &S, u32 u
 }
 
 // Objective change and cache resets over a moved row (delta_batch).
-template<bool MAP>
+template<int TEAM, bool MAP>
 __device__ __forceinline__ long long team_delta(const TeamArgs &a, const TeamSm &S, u32 ou, u32 nu, bool moved,
                                                 u32 stamp, u32 beg, u32 len, u32 first, u32 step, bool inval) {
     long long acc = 0;
@@ -493,8 +548,8 @@ __device__ __forceinline__ long long team_delta(const TeamArgs &a, const TeamSm 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const u32 t = t0 + j * step;
-            v[j] = t < len ? __ldg(&a.g.adj[(u64) beg + t]) : SENTINEL;
-            w[j] = t < len ? g_ew(a.g, (u64) beg + t) : 0;
+            v[j] = t < len ? ld_graph<TEAM>(&a.adj[(u64) beg + t]) : SENTINEL;
+            w[j] = t < len ? ld_ew<TEAM>(a, (u64) beg + t) : 0;
         }
         if (moved) {
 #pragma unroll
@@ -560,10 +615,11 @@ __device__ __forceinline__ void team_flush_bw(const TeamArgs &a, const TeamSm &S
 
 // Copies the block weights to shared memory and returns their maximum (at
 // least 0). All threads call this.
+template<int TEAM>
 __device__ __forceinline__ s32 team_load_bw(const TeamArgs &a, const TeamSm &S, s32 *smx) {
     s32 m = 0;
     for (u32 b = threadIdx.x; b < a.k; b += blockDim.x) {
-        const s32 x = __ldcg(&a.bw[b]);
+        const s32 x = ld_fresh<TEAM>(&a.bw[b]);
         S.bw[b] = x;
         m = x > m ? x : m;
     }
@@ -576,47 +632,48 @@ __device__ __forceinline__ s32 team_load_bw(const TeamArgs &a, const TeamSm &S, 
     return r;
 }
 
-#define TEAM_SYNC()                                                         \
-    do {                                                                    \
-        if (!team_barrier<CLUSTER>(a.bar, bar_target, &a.out->err)) return;  \
+#define TEAM_SYNC()                                                          \
+    do {                                                                     \
+        if (!team_barrier<TEAM>(a.bar, bar_target, &a.out->err)) return;     \
     } while (0)
 
-// CLUSTER: the team is one cluster (gridDim.x blocks), else a cooperative
-// grid. GL: lanes per short row. MAP: process-mapping objective.
-template<bool CLUSTER, int GL, bool MAP>
-__global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ TeamArgs a,
-                                                        const __grid_constant__ TeamCtl ctl) {
-    extern __shared__ __align__(16) unsigned char team_dsm[];
+// The level loop of one team of gridDim.x blocks. GL: lanes per short row.
+// MAP: process-mapping objective.
+template<int TEAM, int GL, bool MAP>
+__device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl, const TeamSm &S) {
     __shared__ long long sl[33];
-    __shared__ u32 su[33];
+    __shared__ u32 su[33], su2[33];
     __shared__ s32 smx[32];
     const u32 tid = threadIdx.x, lane = lane_id(), warp = warp_in_block(), nw = blockDim.x >> 5;
-    const u32 n = a.g.n, k = a.k, G = gridDim.x;
-    TeamSm S = team_carve<GL>(team_dsm, k, nw, warp, MAP);
+    const u32 n = a.n, k = a.k, G = gridDim.x;
+    const u32 g = lane >> 3, gl = lane & 7;  // 8-lane groups of the list passes
+    const u32 lt = (1u << lane) - 1u;
     u32 bar_target = 0;
-    for (u32 i = tid; i < nw * S.stride; i += blockDim.x) S.tab0[i] = 0;
-    for (u32 b = tid; b < k; b += blockDim.x) {
-        S.bd[b] = 0;
-        if (MAP) S.code[b] = a.code[b];
-    }
-    if (MAP && tid < 32) S.dist[tid] = a.bitdist[tid];
-    __syncthreads();
     // contiguous vertex range of every warp (ascending with block and warp)
     const u32 gwarps = G * nw, gw = blockIdx.x * nw + warp;
     const u32 per = (n + gwarps - 1) / gwarps;
     const u32 r0 = (u32) min((u64) n, (u64) gw * per), r1 = (u32) min((u64) n, (u64) r0 + per);
+    const bool small = per <= TEAM_OWN;
+    u32 *const cl = small ? S.own : a.clist + r0;
+    u32 *const ml = small ? S.own + TEAM_OWN : a.mlist + r0;
+    bool hub = false;
     for (u32 u = r0 + lane; u < r1; u += 32) {
         const u32 o = a.part[u];
-        a.saved[u] = o;
+        if (a.saved) a.saved[u] = o;
         a.tw[u] = o;
         a.dest_cache[u] = NULL_PART;
         a.lock[u] = 0;
-        atomicAdd(&S.bd[o], g_vw(a.g, u));
+        atomicAdd(&S.bd[o], ld_vw<TEAM>(a, u));
+        u32 beg, len;
+        ld_row<TEAM>(a, u, beg, len);
+        hub |= len > TEAM_HUB;
     }
+    if (__any_sync(FULL, hub) && lane == 0) atomicOr(&a.out->hubs, 1u);
     __syncthreads();
     team_flush_bw(a, S);
     TEAM_SYNC();
-    team_load_bw(a, S, smx);
+    const bool hubs = ld_fresh<TEAM>(&a.out->hubs) != 0;
+    team_load_bw<TEAM>(a, S, smx);
     long long obj = ctl.obj, best_obj = obj;
     s32 maxw = ctl.maxw, best_max = maxw;
     u32 iterations = 0;
@@ -645,10 +702,14 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                 balance_iteration++;
                 step = balance_iteration < JET_MAX_WEAK_ITERATIONS ? 1 : 2;
             }
-            long long entries = 0;
+            long long moved = 0;  // (moves << 32) + their row entries, of this thread
+            u32 n_own = 0;        // moves in this warp's list
+            u32 n_over = 0;       // overloaded blocks (rebalance steps)
+            long long evicted = 0;  // evicted weight of all blocks (strong)
             if (step == 0) {
                 // gains (cached targets, else recomputed) and filter
                 constexpr int OP = MAP ? OP_MAP : OP_CUT;
+                u32 nc = 0;  // candidates in this warp's list
                 for (u32 base = r0; base < r1; base += 32) {
                     const u32 u = base + lane;
                     const bool act = u < r1;
@@ -659,35 +720,39 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                         lock = a.lock[u];
                         gain = a.gain_cache[u];
                         o = label_of(a, u);
+                        if (small) ld_row<TEAM>(a, u, beg, len);  // one dependent access less
                     }
                     const bool need = act && dest == NULL_PART;
-                    if (need) {
-                        len = __ldg(&a.g.rowlen[u]);
-                        beg = __ldg(&a.g.rowptr[u]);
-                    }
-                    const bool hub = need && len > TEAM_HUB;
+                    if (need && !small) ld_row<TEAM>(a, u, beg, len);
+                    const bool hb = need && len > TEAM_HUB;
                     RowOut r{0, 0, 0, 0};
-                    rows_short<OP, GL>(a, S, __ballot_sync(FULL, need && len <= 4 * GL), beg, len, o, 0, r);
-                    rows_long<OP>(a, S, __ballot_sync(FULL, need && len > 4 * GL && !hub), beg, len, o, 0, r);
-                    if (need && !hub) {
+                    rows_short<TEAM, OP, GL>(a, S, __ballot_sync(FULL, need && len <= 4 * GL), beg, len, o, 0, r);
+                    rows_long<TEAM, OP>(a, S, __ballot_sync(FULL, need && len > 4 * GL && !hb), beg, len, o, 0, r);
+                    if (need && !hb) {
                         lp_decide<MAP>(r, ratio, dest, gain);
                         a.dest_cache[u] = dest;
                         a.gain_cache[u] = gain;
                     }
-                    const u32 sh = warp_append(&cnt[TC_HUB], hub);
-                    if (hub) a.hubs[sh] = u;
-                    const bool c = act && !hub && lp_filter_one(a, u, o, dest, gain, lock);
-                    const u32 sc = warp_append(&cnt[TC_CAND], c);
-                    if (c) a.cand[sc] = u;
+                    if (hubs) {
+                        const u32 sh = warp_append(&cnt[TC_HUB], hb);
+                        if (hb) a.hubs[sh] = u;
+                    }
+                    // a hub row's record says later whether it is a candidate
+                    const bool c = hb || (act && lp_filter_one(a, u, o, dest, gain, lock));
+                    const u32 mask = __ballot_sync(FULL, c);
+                    if (c) cl[nc + __popc(mask & lt)] = u;
+                    nc += __popc(mask);
                 }
                 TEAM_SYNC();
                 if (blockIdx.x == 0 && tid < TC_N) cnt_o[tid] = 0;
                 if (blockIdx.x == 0 && tid < TS_N) sum_o[tid] = 0;
-                const u32 nhub = __ldcg(&cnt[TC_HUB]);
+                const u32 nhub = hubs ? ld_fresh<TEAM>(&cnt[TC_HUB]) : 0;
                 if (nhub) {
                     for (u32 i = blockIdx.x; i < nhub; i += G) {
                         const u32 u = a.hubs[i], o = label_of(a, u);
-                        row_add(a, __ldg(&a.g.rowptr[u]), __ldg(&a.g.rowlen[u]), tid, blockDim.x, S.tab0);
+                        u32 beg, len;
+                        ld_row<TEAM>(a, u, beg, len);
+                        row_add<TEAM>(a, beg, len, tid, blockDim.x, S.tab0);
                         __syncthreads();
                         if (warp == 0) {
                             const RowOut r = row_finish<OP>(a, S, S.tab0, o, 0);
@@ -697,7 +762,7 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                                 lp_decide<MAP>(r, ratio, dest, gain);
                                 a.dest_cache[u] = dest;
                                 a.gain_cache[u] = gain;
-                                if (lp_filter_one(a, u, o, dest, gain, a.lock[u])) a.cand[atomicAdd(&cnt[TC_CAND], 1u)] = u;
+                                lp_filter_one(a, u, o, dest, gain, a.lock[u]);
                             }
                         }
                         __syncthreads();
@@ -705,23 +770,24 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                     TEAM_SYNC();
                 }
                 // afterburner and moves: 8 lanes per candidate, long rows by the warp
-                const u32 nc = __ldcg(&cnt[TC_CAND]);
-                const u32 g = lane >> 3, gl = lane & 7;
-                for (u32 base = gw * 4; base < nc; base += gwarps * 4) {
+                for (u32 base = 0; base < nc; base += 4) {
                     const u32 i = base + g;
-                    const bool act = i < nc;
+                    bool act = i < nc;
                     u32 u = 0, len = 0, beg = 0;
                     unsigned long long rec = 0;
                     if (act) {
-                        u = a.cand[i];
-                        len = __ldg(&a.g.rowlen[u]);
-                        beg = __ldg(&a.g.rowptr[u]);
+                        u = cl[i];
+                        ld_row<TEAM>(a, u, beg, len);
                         rec = a.abrec[u];
                     }
                     const s32 ug = (s32) (u32) rec;
+                    if (ug == GAIN_MIN) {  // a hub row that is none
+                        act = false;
+                        len = 0;
+                    }
                     const u32 nu = (u32) (rec >> 32) & 0xFFFFu, ou = (u32) (rec >> 48);
                     s32 ch = 0;
-                    if (act && len <= TEAM_LONG) ch = team_ab<MAP>(a, S, u, ug, ou, nu, beg, len, gl, 8);
+                    if (act && len <= TEAM_LONG) ch = team_ab<TEAM, MAP>(a, S, u, ug, ou, nu, beg, len, gl, 8);
                     __syncwarp();
 #pragma unroll
                     for (int d = 4; d > 0; d >>= 1) ch = wadd(ch, __shfl_xor_sync(FULL, ch, d));
@@ -733,45 +799,56 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                                   xb = __shfl_sync(FULL, beg, src), xo = __shfl_sync(FULL, ou, src),
                                   xn = __shfl_sync(FULL, nu, src);
                         const s32 xg = __shfl_sync(FULL, ug, src);
-                        const s32 c = (s32) warp_sum<u32>((u32) team_ab<MAP>(a, S, xu, xg, xo, xn, xb, xl, lane, 32));
+                        const s32 c =
+                            (s32) warp_sum<u32>((u32) team_ab<TEAM, MAP>(a, S, xu, xg, xo, xn, xb, xl, lane, 32));
                         if ((int) lane == src) ch = c;
                     }
                     const bool mv = act && gl == 0 && wadd(ug, ch) >= 0;
                     if (mv) {
                         a.lock[u] = 1;
-                        team_move(a, S, u, ou, nu, g_vw(a.g, u), stamp);
-                        entries += len;
+                        team_move(a, S, u, ou, nu, ld_vw<TEAM>(a, u), stamp);
+                        moved += (1ll << 32) + len;
                     }
-                    const u32 sm_ = warp_append(&cnt[TC_MOVES], mv);
-                    if (mv) a.moves[sm_] = u;
+                    const u32 mask = __ballot_sync(FULL, mv);
+                    if (mv) ml[n_own + __popc(mask & lt)] = u;
+                    n_own += __popc(mask);
                 }
-                team_add(entries, &sum[TS_ENTRIES], sl);
-                team_flush_bw(a, S);
-                TEAM_SYNC();
             } else {
                 const bool strong = step == 2;
                 const s32 max_b_w = strong ? a.strong_max : a.weak_max;
                 const u32 sft = strong ? 1u : 0u;  // own keys of block o: [o * width + sft, (o + 1) * width + sft)
                 // blocks with room (weak) or the largest room (strong), and
                 // the overloaded blocks, from the block weights in shared memory
-                u32 n_under = 0, n_over = 0;
+                u32 n_under = 0;
                 s32 maxv = INT32_MIN;
                 for (u32 b0 = 0; b0 < k; b0 += blockDim.x) {
                     const u32 b = b0 + tid;
                     const s32 x = b < k ? S.bw[b] : INT32_MAX;
                     const bool un = b < k && x < max_b_w, ov = b < k && x > a.lmax;
                     if (un && max_b_w - x > maxv) maxv = max_b_w - x;
-                    u32 tot;
-                    const u32 p = block_exclusive_scan<u32>((un ? 1u : 0u) | (ov ? 0x10000u : 0u), tot, su);
-                    if (un) S.under[n_under + (p & 0xFFFFu)] = b;
-                    if (ov) S.olist[n_over + (p >> 16)] = b;
-                    n_under += tot & 0xFFFFu;
-                    n_over += tot >> 16;
+                    const u32 mu = __ballot_sync(FULL, un), mo = __ballot_sync(FULL, ov);
+                    const s32 mv = __reduce_max_sync(FULL, maxv);
+                    if (lane == 0) {
+                        su[warp] = __popc(mu);
+                        su2[warp] = __popc(mo);
+                        smx[warp] = mv;
+                    }
+                    __syncthreads();
+                    const u32 used = (min(k - b0, blockDim.x) + 31) >> 5;
+                    u32 pu = n_under, po = n_over;
+                    for (u32 w = 0; w < used; ++w) {
+                        if (w == warp) {
+                            pu = n_under;
+                            po = n_over;
+                        }
+                        n_under += su[w];
+                        n_over += su2[w];
+                        maxv = smx[w] > maxv ? smx[w] : maxv;
+                    }
+                    if (un) S.under[pu + __popc(mu & lt)] = b;
+                    if (ov) S.olist[po + __popc(mo & lt)] = b;
+                    __syncthreads();
                 }
-                maxv = __reduce_max_sync(FULL, maxv);
-                if (lane == 0) smx[warp] = maxv;
-                __syncthreads();
-                for (u32 w = 0; w < nw; ++w) maxv = smx[w] > maxv ? smx[w] : maxv;
                 if (strong && blockIdx.x == 0)
                     for (u32 b = tid; b < k; b += blockDim.x) a.ea[b] = 0;
                 // picks: target and mini-bucket key of every candidate, whose
@@ -803,7 +880,8 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                     s32 vw = 0;
                     if (act) {
                         o = label_of(a, u);
-                        vw = g_vw(a.g, u);
+                        vw = ld_vw<TEAM>(a, u);
+                        if (small) ld_row<TEAM>(a, u, beg, len);
                     }
                     bool need = false;
                     if (act) {
@@ -812,48 +890,49 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                             need = strong ? ((s64) vw <= 2 * (s64) maxv && (s64) vw < 2 * (ow - a.opt))
                                           : 2 * (s64) vw < 3 * (ow - a.opt);
                     }
-                    if (need) {
-                        len = __ldg(&a.g.rowlen[u]);
-                        beg = __ldg(&a.g.rowptr[u]);
-                    }
-                    const bool hub = need && len > TEAM_HUB;
+                    if (need && !small) ld_row<TEAM>(a, u, beg, len);
+                    const bool hb = need && len > TEAM_HUB;
                     RowOut r{0, 0, 0, 0};
                     const u32 ms = __ballot_sync(FULL, need && len <= 4 * GL);
-                    const u32 ml = __ballot_sync(FULL, need && len > 4 * GL && !hub);
+                    const u32 mg = __ballot_sync(FULL, need && len > 4 * GL && !hb);
                     if (strong) {
-                        rows_short<OP_STRONG, GL>(a, S, ms, beg, len, o, max_b_w, r);
-                        rows_long<OP_STRONG>(a, S, ml, beg, len, o, max_b_w, r);
+                        rows_short<TEAM, OP_STRONG, GL>(a, S, ms, beg, len, o, max_b_w, r);
+                        rows_long<TEAM, OP_STRONG>(a, S, mg, beg, len, o, max_b_w, r);
                     } else {
-                        rows_short<OP_WEAK, GL>(a, S, ms, beg, len, o, max_b_w, r);
-                        rows_long<OP_WEAK>(a, S, ml, beg, len, o, max_b_w, r);
+                        rows_short<TEAM, OP_WEAK, GL>(a, S, ms, beg, len, o, max_b_w, r);
+                        rows_long<TEAM, OP_WEAK>(a, S, mg, beg, len, o, max_b_w, r);
                     }
                     u32 key = NOKEY;
-                    if (need && !hub) key = finish(u, o, vw, r);
-                    if (act && !hub) a.keys[u] = key;
+                    if (need && !hb) key = finish(u, o, vw, r);
+                    if (act && !hb) a.keys[u] = key;
                     // one add per distinct key of the warp
-                    const u32 peers = __match_any_sync(FULL, key);
                     if (__any_sync(FULL, key != NOKEY)) {
+                        const u32 peers = __match_any_sync(FULL, key);
                         s32 p, t;
                         peer_prefix(peers, vw, p, t);
-                        if (key != NOKEY && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(&a.hist[key], (u32) t);
+                        if (key != NOKEY && (peers & lt) == 0) atomicAdd(&a.hist[key], (u32) t);
                     }
-                    const u32 sh = warp_append(&cnt[TC_HUB], hub);
-                    if (hub) a.hubs[sh] = u;
+                    if (hubs) {
+                        const u32 sh = warp_append(&cnt[TC_HUB], hb);
+                        if (hb) a.hubs[sh] = u;
+                    }
                 }
                 TEAM_SYNC();
                 if (blockIdx.x == 0 && tid < TC_N) cnt_o[tid] = 0;
                 if (blockIdx.x == 0 && tid < TS_N) sum_o[tid] = 0;
-                const u32 nhub = __ldcg(&cnt[TC_HUB]);
+                const u32 nhub = hubs ? ld_fresh<TEAM>(&cnt[TC_HUB]) : 0;
                 if (nhub) {
                     for (u32 i = blockIdx.x; i < nhub; i += G) {
                         const u32 u = a.hubs[i], o = label_of(a, u);
-                        row_add(a, __ldg(&a.g.rowptr[u]), __ldg(&a.g.rowlen[u]), tid, blockDim.x, S.tab0);
+                        u32 beg, len;
+                        ld_row<TEAM>(a, u, beg, len);
+                        row_add<TEAM>(a, beg, len, tid, blockDim.x, S.tab0);
                         __syncthreads();
                         if (warp == 0) {
                             const RowOut r = strong ? row_finish<OP_STRONG>(a, S, S.tab0, o, max_b_w)
                                                     : row_finish<OP_WEAK>(a, S, S.tab0, o, max_b_w);
                             if (lane == 0) {
-                                const s32 vw = g_vw(a.g, u);
+                                const s32 vw = ld_vw<TEAM>(a, u);
                                 const u32 key = finish(u, o, vw, r);
                                 a.keys[u] = key;
                                 if (key != NOKEY) atomicAdd(&a.hist[key], (u32) vw);
@@ -865,26 +944,34 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                 }
                 // per overloaded block: the bin in which the limit falls, by 8
                 // lanes over contiguous shares of the block's bins
-                for (u32 b = tid; b < k; b += blockDim.x) {
-                    S.tot[b] = 0;
-                    S.spill[b] = 0;
+                if (strong) {
+                    for (u32 b = tid; b < k; b += blockDim.x) S.tot[b] = 0;
+                    __syncthreads();
                 }
-                __syncthreads();
-                const u32 g = lane >> 3, gl = lane & 7;
+                const u32 share = (a.width + 7) / 8;
                 for (u32 i0 = warp * 4; i0 < n_over; i0 += nw * 4) {
                     const u32 i = i0 + g;
                     const bool act = i < n_over;
                     const u32 o = act ? S.olist[i] : 0;
-                    const u32 share = (a.width + 7) / 8;
                     const u32 b0 = min(gl * share, a.width), b1 = min(b0 + share, a.width);
                     const u32 *h = a.hist + (u64) o * a.width + sft;
-                    s32 mine = 0, last = 0;
+                    s32 mine = 0, last = 0, spill = 0;
+                    s32 hv[8];
                     if (act) {
+                        if (share <= 8) {
+#pragma unroll
+                            for (u32 x = 0; x < 8; ++x) hv[x] = b0 + x < b1 ? (s32) ld_fresh<TEAM>(&h[b0 + x]) : 0;
+#pragma unroll
+                            for (u32 x = 0; x < 8; ++x) mine += hv[x];
+                        } else {
 #pragma unroll 8
-                        for (u32 x = b0; x < b1; ++x) mine += (s32) __ldcg(&h[x]);
-                        last = (s32) __ldcg(&h[a.width - 1]);
+                            for (u32 x = b0; x < b1; ++x) mine += (s32) ld_fresh<TEAM>(&h[x]);
+                        }
+                        if (strong) {
+                            last = (s32) ld_fresh<TEAM>(&h[a.width - 1]);
+                            spill = (s32) ld_fresh<TEAM>(h - 1);
+                        }
                     }
-                    const s32 spill = act && strong ? (s32) __ldcg(&h[-1]) : 0;
                     s32 inc = mine;
 #pragma unroll
                     for (int d = 1; d < 8; d <<= 1) {
@@ -895,6 +982,7 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                     s32 run = spill + inc - mine;
                     const s32 limit = act ? S.bw[o] - a.lmax : 0;
                     if (act && gl == 0) {
+                        S.toff[o] = 0;
                         // all bins but the last one of strong keys, which the
                         // next block's range starts with (key = (o + 1) * width)
                         S.tot[o] = strong ? total - last : total;
@@ -908,10 +996,22 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                     }
                     if (act && run < limit && limit <= run + mine) {
                         u32 x = b0;
-                        for (; x < b1; ++x) {
-                            const s32 c = (s32) __ldcg(&h[x]);
-                            if (limit <= run + c) break;
-                            run += c;
+                        if (share <= 8) {
+                            bool done = false;
+#pragma unroll
+                            for (u32 y = 0; y < 8; ++y) {
+                                done = done || limit <= run + hv[y];
+                                if (!done) {
+                                    run += hv[y];
+                                    ++x;
+                                }
+                            }
+                        } else {
+                            for (; x < b1; ++x) {
+                                const s32 c = (s32) ld_fresh<TEAM>(&h[x]);
+                                if (limit <= run + c) break;
+                                run += c;
+                            }
                         }
                         S.cutkey[o] = o * a.width + sft + x;
                         S.cutbase[o] = run;
@@ -923,7 +1023,8 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                     // within the limit holds only that block's last bin
                     for (u32 i = tid; i < n_over; i += blockDim.x) {
                         const u32 o = S.olist[i];
-                        if (o + 1 < k && S.bw[o + 1] <= a.lmax) S.tot[o + 1] = (s32) __ldcg(&a.hist[(u64) (o + 1) * a.width]);
+                        if (o + 1 < k && S.bw[o + 1] <= a.lmax)
+                            S.tot[o + 1] = (s32) ld_fresh<TEAM>(&a.hist[(u64) (o + 1) * a.width]);
                     }
                 // weight of each warp's candidates in the cut bins
                 for (u32 base = r0; base < r1; base += 32) {
@@ -932,7 +1033,20 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                         const u32 key = a.keys[u];
                         if (key != NOKEY) {
                             const u32 o = (key - sft) / a.width;
-                            if (key == S.cutkey[o]) atomicAdd(&S.tab[o], g_vw(a.g, u));
+                            if (key == S.cutkey[o]) atomicAdd(&S.tab[o], ld_vw<TEAM>(a, u));
+                        }
+                    }
+                }
+                if (TEAM == TEAM_CLUSTER) {
+                    // weight in the cut bins before this block's vertices: a
+                    // cluster's levels are small enough for every block to
+                    // look at all keys before its own (one barrier less)
+                    const u32 first = (u32) min((u64) n, (u64) blockIdx.x * nw * per);
+                    for (u32 u = tid; u < first; u += blockDim.x) {
+                        const u32 key = __ldcg(&a.keys[u]);
+                        if (key != NOKEY) {
+                            const u32 o = (key - sft) / a.width;
+                            if (key == S.cutkey[o]) atomicAdd(&S.toff[o], ld_vw<TEAM>(a, u));
                         }
                     }
                 }
@@ -946,25 +1060,23 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                         *p = run;
                         run += x;
                     }
-                    a.tsum[(u64) o * G + blockIdx.x] = run;
+                    if (TEAM == TEAM_GRID) a.tsum[(u64) o * G + blockIdx.x] = run;
                 }
-                TEAM_SYNC();
-                // weight before this block's share of the cut bins
-                for (u32 i0 = warp * 4; i0 < n_over; i0 += nw * 4) {
-                    const u32 i = i0 + g;
-                    const bool act = i < n_over;
-                    const u32 o = act ? S.olist[i] : 0;
-                    s32 x = 0;
-                    if (act)
-                        for (u32 b = gl; b < blockIdx.x; b += 8) x += __ldcg(&a.tsum[(u64) o * G + b]);
+                if (TEAM == TEAM_GRID) {
+                    TEAM_SYNC();
+                    // weight before this block's share of the cut bins
+                    for (u32 i0 = warp * 4; i0 < n_over; i0 += nw * 4) {
+                        const u32 i = i0 + g;
+                        const bool act = i < n_over;
+                        const u32 o = act ? S.olist[i] : 0;
+                        s32 x = 0;
+                        if (act)
+#pragma unroll 4
+                            for (u32 b = gl; b < blockIdx.x; b += 8) x += __ldcg(&a.tsum[(u64) o * G + b]);
 #pragma unroll
-                    for (int d = 4; d > 0; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
-                    if (act && gl == 0) S.toff[o] = x;
-                }
-                // the bins are not read any more in this step: clear them
-                for (u32 i = blockIdx.x; i < n_over; i += G) {
-                    u32 *h = a.hist + (u64) S.olist[i] * a.width;
-                    for (u32 x = tid; x <= a.width; x += blockDim.x) h[x] = 0;
+                        for (int d = 4; d > 0; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
+                        if (act && gl == 0) S.toff[o] = x;
+                    }
                 }
                 __syncthreads();
                 // selection in ascending vertex id
@@ -977,7 +1089,7 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                     bool take = false, cut = false;
                     if (key != NOKEY) {
                         o = (key - sft) / a.width;
-                        vw = g_vw(a.g, u);
+                        vw = ld_vw<TEAM>(a, u);
                         cut = key == S.cutkey[o];
                         take = key < S.cutkey[o];
                     }
@@ -989,7 +1101,7 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                         if (cut) before = S.tab[o];
                         __syncwarp();
                         if (cut) {
-                            if ((peers & ((1u << lane) - 1u)) == 0) S.tab[o] = before + t;
+                            if ((peers & lt) == 0) S.tab[o] = before + t;
                             const s32 score = S.cutbase[o] + S.toff[o] + before + p;
                             const s32 limit = S.bw[o] - a.lmax;
                             take = score < limit;
@@ -997,25 +1109,30 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                         }
                         __syncwarp();
                     }
-                    if (take && !strong) {
-                        const u32 nu = a.dest[u];
-                        team_move(a, S, u, o, nu, vw, stamp);
-                        entries += __ldg(&a.g.rowlen[u]);
-                    }
-                    const u32 s = warp_append(&cnt[TC_MOVES], take);
-                    if (take) {
-                        a.moves[s] = u;
-                        if (strong) {
+                    if (strong) {
+                        if (!__any_sync(FULL, take)) continue;
+                        const u32 s = warp_append(&cnt[TC_MOVES], take);
+                        if (take) {
                             a.mcomp[s] = ((unsigned long long) key << 32) | u;
                             a.mow[s] = ((unsigned long long) o << 32) | (u32) vw;
                         }
+                    } else {
+                        if (take) {
+                            u32 beg, len;
+                            ld_row<TEAM>(a, u, beg, len);
+                            team_move(a, S, u, o, a.dest[u], vw, stamp);
+                            moved += (1ll << 32) + len;
+                        }
+                        const u32 mask = __ballot_sync(FULL, take);
+                        if (take) ml[n_own + __popc(mask & lt)] = u;
+                        n_own += __popc(mask);
                     }
                 }
                 __syncwarp();
                 for (u32 i = lane; i < n_over; i += 32) S.tab[S.olist[i]] = 0;
                 if (strong) {
                     TEAM_SYNC();
-                    const u32 ns = __ldcg(&cnt[TC_MOVES]);
+                    const u32 ns = ld_fresh<TEAM>(&cnt[TC_MOVES]);
                     if (ns > TEAM_RANK_MAX) {
                         if (blockIdx.x == 0 && tid == 0) a.out->gave_up = 1;
                         return;
@@ -1027,7 +1144,7 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                         const u32 b = b0 + tid;
                         long long add = 0, cap = 0;
                         if (b < k) {
-                            add = __ldcg(&a.ea[b]);
+                            add = ld_fresh<TEAM>(&a.ea[b]);
                             if (add == 0) add = S.tot[b];
                             cap = max_b_w > S.bw[b] ? (long long) max_b_w - S.bw[b] : 0;
                         }
@@ -1041,6 +1158,7 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                         c1 += t1;
                         c2 += t2;
                     }
+                    evicted = c1;
                     if (tid == 0) S.es[0] = 0;
                     __syncthreads();
                     // exact prefix of each evicted vertex among its block's
@@ -1072,79 +1190,88 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                             const s32 id = chunk_of(S.es, k, tg);
                             const bool fits = id < (s32) k && (long long) (vw / 2) <= S.es[id + 1] - tg;
                             if (!fits && id < (s32) k) {
-                                a.cand[atomicAdd(&cnt[TC_FAIL], 1u)] = u;
+                                a.fails[atomicAdd(&cnt[TC_FAIL], 1u)] = u;
                             } else {
                                 team_move(a, S, u, o, fits ? (u32) id : o, vw, stamp);
                             }
-                            entries += __ldg(&a.g.rowlen[u]);
+                            u32 beg, len;
+                            ld_row<TEAM>(a, u, beg, len);
+                            moved += (1ll << 32) + len;
                         }
                         __syncwarp();
                     }
-                    team_add(entries, &sum[TS_ENTRIES], sl);
-                    team_flush_bw(a, S);
-                    TEAM_SYNC();
-                    const u32 nf = __ldcg(&cnt[TC_FAIL]);
-                    if (nf) {
-                        // fallback slots in ascending vertex id (block 0)
-                        if (blockIdx.x == 0) {
-                            for (u32 j = tid; j < nf; j += blockDim.x) {
-                                const u32 u = a.cand[j];
-                                u32 p = 0;
-                                for (u32 i = 0; i < nf; ++i) p += a.cand[i] < u;
-                                a.hubs[p] = u;
-                            }
-                            __syncthreads();
-                            if (tid == 0) {
-                                long long mv = c1;
-                                for (u32 j = 0; j < nf; ++j) {
-                                    const u32 u = a.hubs[j];
-                                    const u32 o = label_of(a, u);
-                                    const s32 vw = g_vw(a.g, u);
-                                    u32 dest = o;
-                                    for (u32 guard = 0; guard < 2 * k + 4; ++guard) {
-                                        const long long tg = mv;
-                                        mv += vw;
-                                        const s32 id = chunk_of(S.es, k, tg);
-                                        if (id >= (s32) k) break;
-                                        if ((long long) (vw / 2) <= S.es[id + 1] - tg) {
-                                            dest = (u32) id;
-                                            break;
-                                        }
-                                    }
-                                    team_move(a, S, u, o, dest, vw, stamp);
-                                }
-                            }
-                            __syncthreads();
-                            team_flush_bw(a, S);
+                }
+            }
+            team_add(moved, &sum[TS_MOVES], sl);
+            team_flush_bw(a, S);
+            TEAM_SYNC();
+            if (step == 2) {
+                const u32 nf = ld_fresh<TEAM>(&cnt[TC_FAIL]);
+                if (nf) {
+                    // fallback slots in ascending vertex id (block 0)
+                    if (blockIdx.x == 0) {
+                        for (u32 j = tid; j < nf; j += blockDim.x) {
+                            const u32 u = a.fails[j];
+                            u32 p = 0;
+                            for (u32 i = 0; i < nf; ++i) p += a.fails[i] < u;
+                            a.hubs[p] = u;
                         }
-                        TEAM_SYNC();
+                        __syncthreads();
+                        if (tid == 0) {
+                            long long mv = evicted;
+                            for (u32 j = 0; j < nf; ++j) {
+                                const u32 u = a.hubs[j];
+                                const u32 o = label_of(a, u);
+                                const s32 vw = ld_vw<TEAM>(a, u);
+                                u32 dest = o;
+                                for (u32 guard = 0; guard < 2 * k + 4; ++guard) {
+                                    const long long tg = mv;
+                                    mv += vw;
+                                    const s32 id = chunk_of(S.es, k, tg);
+                                    if (id >= (s32) k) break;
+                                    if ((long long) (vw / 2) <= S.es[id + 1] - tg) {
+                                        dest = (u32) id;
+                                        break;
+                                    }
+                                }
+                                team_move(a, S, u, o, dest, vw, stamp);
+                            }
+                        }
+                        __syncthreads();
+                        team_flush_bw(a, S);
                     }
-                } else {
-                    team_add(entries, &sum[TS_ENTRIES], sl);
-                    team_flush_bw(a, S);
                     TEAM_SYNC();
                 }
             }
             // exact objective change and the neighbours' cache resets
-            const u32 nm = __ldcg(&cnt[TC_MOVES]);
-            const bool inval = (unsigned long long) __ldcg(&sum[TS_ENTRIES]) < a.inval_all_min;
-            const s32 new_maxw = team_load_bw(a, S, smx);
+            const unsigned long long ent = (unsigned long long) ld_fresh<TEAM>(&sum[TS_MOVES]);
+            const u32 nm = (u32) (ent >> 32);
+            const bool inval = (ent & 0xFFFFFFFFull) < a.inval_all_min;
+            const s32 new_maxw = team_load_bw<TEAM>(a, S, smx);
+            // the bins are not read any more: clear them
+            if (step != 0)
+                for (u32 i = blockIdx.x; i < n_over; i += G) {
+                    u32 *h = a.hist + (u64) S.olist[i] * a.width;
+                    for (u32 x = tid; x <= a.width; x += blockDim.x) h[x] = 0;
+                }
             long long acc = 0;
             {
-                const u32 g = lane >> 3, gl = lane & 7;
-                for (u32 base = gw * 4; base < nm; base += gwarps * 4) {
+                // this warp's own moves, or its share of the evicted vertices
+                const bool shared_list = step == 2;
+                const u32 first = shared_list ? gw * 4 : 0, stride = shared_list ? gwarps * 4 : 4;
+                const u32 total = shared_list ? nm : n_own;
+                for (u32 base = first; base < total; base += stride) {
                     const u32 i = base + g;
                     u32 u = 0, len = 0, beg = 0;
                     unsigned long long x = 0;
-                    if (i < nm) {
-                        u = a.moves[i];
-                        len = __ldg(&a.g.rowlen[u]);
-                        beg = __ldg(&a.g.rowptr[u]);
+                    if (i < total) {
+                        u = shared_list ? (u32) a.mcomp[i] : ml[i];
+                        ld_row<TEAM>(a, u, beg, len);
                         x = a.tw[u];
                     }
                     if (len <= TEAM_LONG)
-                        acc += team_delta<MAP>(a, S, tw_old(x), tw_label(x), tw_stamp(x) == stamp, stamp, beg, len, gl, 8,
-                                               inval);
+                        acc += team_delta<TEAM, MAP>(a, S, tw_old(x), tw_label(x), tw_stamp(x) == stamp, stamp, beg, len,
+                                                     gl, 8, inval);
                     __syncwarp();
                     u32 lng = __ballot_sync(FULL, gl == 0 && len > TEAM_LONG);
                     while (lng) {
@@ -1152,8 +1279,8 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                         lng &= lng - 1;
                         const u32 xl = __shfl_sync(FULL, len, src), xb = __shfl_sync(FULL, beg, src);
                         const unsigned long long xx = __shfl_sync(FULL, x, src);
-                        acc += team_delta<MAP>(a, S, tw_old(xx), tw_label(xx), tw_stamp(xx) == stamp, stamp, xb, xl, lane,
-                                               32, inval);
+                        acc += team_delta<TEAM, MAP>(a, S, tw_old(xx), tw_label(xx), tw_stamp(xx) == stamp, stamp, xb, xl,
+                                                     lane, 32, inval);
                     }
                 }
             }
@@ -1161,7 +1288,7 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
                 for (u32 u = r0 + lane; u < r1; u += 32) a.dest_cache[u] = NULL_PART;
             team_add(acc, &sum[TS_DELTA], sl);
             TEAM_SYNC();
-            const long long d = __ldcg(&sum[TS_DELTA]);
+            const long long d = ld_fresh<TEAM>(&sum[TS_DELTA]);
             // control (jet_label_propagation.h:966-1030, promap :1250-1305)
             if (!MAP) {
                 if (nm == 0) {
@@ -1200,3 +1327,110 @@ __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ Te
 }
 
 #undef TEAM_SYNC
+
+// Zeroes the tables and loads the distance oracle.
+template<int GL, bool MAP>
+__device__ __forceinline__ TeamSm team_setup(const TeamArgs &a, unsigned char *dsm) {
+    const u32 tid = threadIdx.x, nw = blockDim.x >> 5;
+    const TeamSm S = team_carve<GL>(dsm, a.k, nw, warp_in_block(), MAP);
+    for (u32 i = tid; i < nw * S.stride; i += blockDim.x) S.tab0[i] = 0;
+    for (u32 b = tid; b < a.k; b += blockDim.x) {
+        S.bd[b] = 0;
+        if (MAP) S.code[b] = a.code[b];
+    }
+    if (MAP && tid < 32) S.dist[tid] = a.bitdist[tid];
+    __syncthreads();
+    return S;
+}
+
+// A cluster or a cooperative grid on a level in global memory.
+template<int TEAM, int GL, bool MAP>
+__global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ TeamArgs a,
+                                                        const __grid_constant__ TeamCtl ctl) {
+    extern __shared__ __align__(16) unsigned char team_dsm[];
+    const TeamSm S = team_setup<GL, MAP>(a, team_dsm);
+    team_loop<TEAM, GL, MAP>(a, ctl, S);
+}
+
+// One block that copies the level to shared memory first (rows made
+// contiguous). `level` is the offset of the level's arrays.
+template<int GL, bool MAP>
+__global__ void __launch_bounds__(512, 1) k_jet_block(const __grid_constant__ TeamArgs ga,
+                                                        const __grid_constant__ TeamCtl ctl, u32 m, u32 level) {
+    extern __shared__ __align__(16) unsigned char team_dsm[];
+    __shared__ u32 scan_sm[32];
+    const TeamSm S = team_setup<GL, MAP>(ga, team_dsm);
+    const u32 n = ga.n, k = ga.k, tid = threadIdx.x, lane = lane_id();
+    TeamArgs a = ga;
+    unsigned long long *q = (unsigned long long *) (team_dsm + level);
+    a.tw = q;
+    a.abrec = q + n;
+    a.dest = (u32 *) a.abrec;  // records belong to label propagation, targets and keys to rebalancing
+    a.keys = a.dest + n;
+    a.mcomp = q + 2 * (u64) n;
+    a.mow = q + 3 * (u64) n;
+    q += 4 * (u64) n;
+    TeamOut *out = (TeamOut *) q;
+    a.out = out;
+    a.sum = (long long *) (out + 1);
+    u32 *p = (u32 *) (a.sum + 2 * TS_N);
+    u32 *rowptr = p;
+    p += n + 1;
+    a.dest_cache = p;
+    a.gain_cache = (s32 *) (p + n);
+    a.lock = p + 2 * n;
+    s32 *vw = (s32 *) (p + 3 * n);
+    a.clist = a.fails = p + 4 * n;
+    a.mlist = a.hubs = p + 5 * n;
+    p += 6 * n;
+    u32 *adj = p;
+    s32 *ew = (s32 *) (p + m);
+    p += 2 * m;
+    a.cnt = p;
+    a.bw = (s32 *) (p + 2 * TC_N);
+    a.ea = a.bw + k;
+    a.hist = (u32 *) (a.ea + k);
+    const u32 bins = k * a.width + 2;
+    if (tid == 0) {
+        out->hubs = 0;
+        out->gave_up = 0;
+    }
+    if (tid < 2 * TS_N) a.sum[tid] = 0;
+    if (tid < 2 * TC_N) a.cnt[tid] = 0;
+    for (u32 b = tid; b < k; b += blockDim.x) a.bw[b] = 0;
+    for (u32 b = tid; b < bins; b += blockDim.x) a.hist[b] = 0;
+    // row offsets, then the rows, 8 lanes each
+    u32 run = 0;
+    for (u32 u0 = 0; u0 < n; u0 += blockDim.x) {
+        const u32 u = u0 + tid;
+        const u32 len = u < n ? __ldg(&ga.rowlen[u]) : 0;
+        u32 tot;
+        const u32 pos = run + block_exclusive_scan<u32>(len, tot, scan_sm);
+        if (u < n) {
+            rowptr[u] = pos;
+            vw[u] = ga.vw ? __ldg(&ga.vw[u]) : 1;
+        }
+        run += tot;
+    }
+    if (tid == 0) rowptr[n] = run;
+    __syncthreads();
+    for (u32 u = tid >> 3; u < n; u += blockDim.x >> 3) {
+        const u32 src = __ldg(&ga.rowptr[u]), dst = rowptr[u], len = rowptr[u + 1] - dst;
+        for (u32 t = lane & 7; t < len; t += 8) {
+            adj[dst + t] = __ldg(&ga.adj[src + t]);
+            ew[dst + t] = ga.ew ? __ldg(&ga.ew[src + t]) : 1;
+        }
+    }
+    __syncthreads();
+    a.rowptr = rowptr;
+    a.adj = adj;
+    a.ew = ew;
+    a.vw = vw;
+    team_loop<TEAM_BLOCK, GL, MAP>(a, ctl, S);
+    if (tid == 0) {
+        ga.out->obj = out->obj;
+        ga.out->maxw = out->maxw;
+        ga.out->iterations = out->iterations;
+        ga.out->gave_up = out->gave_up;
+    }
+}
