@@ -22,8 +22,8 @@ import numpy as np
 CANDIDATES = {
     "jet_graph_max_m": [0, 1 << 20, 1 << 22, 1 << 24, 1 << 26],
     "order_small_n": [0, 4096, 16384, 65536],
-    "match_coop_max_n": [0, 1 << 15, 1 << 17, 1 << 19],
-    "match_coop_max_m": [0, 1 << 19, 1 << 21, 1 << 23],
+    "match_coop_max_n": [0, 1 << 16, 1 << 18, 1 << 20],
+    "match_coop_max_m": [0, 1 << 20, 1 << 22, 1 << 24],
     "jet_fused_max_n": [0, 2048, 4096, 8192],
     "jet_fused_max_m": [1 << 16, 1 << 18, 1 << 20],
     "jet_coop_max_n": [0, 65536, 1 << 20, 1 << 24],
@@ -37,8 +37,8 @@ CANDIDATES = {
     "jet_vec_loads": [0, 1],
     "jet_chunk_mode": [0, 1],
 }
-DEFAULTS = {"jet_graph_max_m": 1 << 24, "order_small_n": 16384, "match_coop_max_n": 1 << 17,
-            "match_coop_max_m": 1 << 21, "jet_fused_max_n": 8192, "jet_fused_max_m": 1 << 18,
+DEFAULTS = {"jet_graph_max_m": 1 << 24, "order_small_n": 16384, "match_coop_max_n": 1 << 20,
+            "match_coop_max_m": 1 << 24, "jet_fused_max_n": 8192, "jet_fused_max_m": 1 << 18,
             "jet_coop_max_n": 1 << 24, "jet_coop_max_m": 1 << 27, "jet_coop_max_deg": 24, "jet_coop_rows": 512,
             "jet_hub_deg": 1024, "jet_hub_conn": 1, "jet_hub_track_pct": 50, "jet_inval_all_pct": 5,
             "jet_vec_loads": 1, "jet_chunk_mode": 0}

@@ -17,4 +17,24 @@ u32 match_graph(Ctx &ctx, const DGraph &g, u32 *mapping);
 // hash-slot order; the row contents are exact.
 DGraph contract_graph(Ctx &ctx, const DGraph &g, const u32 *mapping, u32 n_c);
 
+// One coarsening level in one launch (coarsen_team.cu). `mapping` receives
+// the fine->coarse map. With `rows` (adj and ew allocated with room for g.m
+// entries), the coarse rows are written there and rowptr (n + 1), rowlen and vw
+// point to scratch with the coarse graph's row bounds and vertex weights; they
+// are valid until the caller releases the scratch. contracted is false when a
+// coarse row is too long for the kernel's tables (contract_graph then builds
+// the graph). Throws CoopSpin when the launch cannot be made or gave up.
+struct CoarsenResult {
+    u32 n = 0;
+    u64 m = 0;
+    bool contracted = false;
+    double contract_ms = 0;
+    u32 *rowptr = nullptr, *rowlen = nullptr;
+    s32 *vw = nullptr;
+};
+constexpr u32 COARSEN_TEAM_MAX_N = 1u << 20;  // upper bound of Tunables::match_coop_max_n
+
+bool coarsen_team_applies(const Ctx &ctx, const DGraph &g);
+CoarsenResult coarsen_team(Ctx &ctx, const DGraph &g, u32 *mapping, DGraph *rows);
+
 } // namespace hp

@@ -128,8 +128,8 @@ struct PhaseProf {
 struct Tunables {
     u64 jet_graph_max_m = 1ull << 24;  // Jet iterations replayed as CUDA graphs up to this many entries
     u32 order_small_n = 16384;         // single-block rebalance ordering up to this many vertices
-    u32 match_coop_max_n = 1u << 17;   // cooperative matching loop up to this many vertices ...
-    u64 match_coop_max_m = 1ull << 21; // ... and entries
+    u32 match_coop_max_n = 1u << 20;   // matching and contraction of a level in one launch up to this many vertices ...
+    u64 match_coop_max_m = 1ull << 24; // ... and entries
     u32 jet_fused_max_n = 8192;        // whole Jet level loop in one thread-block cluster up to this many vertices ...
     u64 jet_fused_max_m = 1ull << 18;  // ... and entries
     u32 jet_coop_max_n = 1u << 24;     // ... else as a cooperative grid up to this many vertices ...

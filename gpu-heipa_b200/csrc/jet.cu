@@ -4,6 +4,7 @@
 // mini-bucket order by vertex id, fallback slots in ascending vertex id).
 #include "jet.cuh"
 #include "stage.cuh"
+#include "team.cuh"
 
 #include <mutex>
 #include <optional>
@@ -2692,14 +2693,9 @@ void JetLevel::run_step(int kind, u32 ratio_pct) {
 
 // ---- host side of the single-launch level loop ------------------------------------------
 
-constexpr u32 TEAM_BLOCK_THREADS = 512;
-constexpr u32 TEAM_CLUSTER_THREADS = 512;
-constexpr u32 TEAM_GRID_THREADS = 1024;
-constexpr size_t TEAM_BLOCK_SMEM = 226 * 1024;  // dynamic shared memory of a block team
 // vertices per block of a cluster team (up to its largest size): 4 rows per warp
 constexpr u32 TEAM_CLUSTER_ROWS = 64;
 constexpr u32 TEAM_CLUSTER_MAX_N = 1u << 16;  // upper bound of Tunables::jet_fused_max_n
-constexpr u32 TEAM_PEER_BLOCKS = 40;
 // Block teams: what fits in shared memory. The cluster took 14.7 us per
 // iteration on the levels of up to 1700 vertices of an RGG with 3001 vertices,
 // one block with the level in shared memory 10.5 us.
@@ -2728,27 +2724,6 @@ static const void *team_kernel(int team, u32 k, bool promap) {
     return k <= 256 ? (const void *) k_jet_team<TEAM_GRID, 8, false> : (const void *) k_jet_team<TEAM_GRID, 32, false>;
 }
 
-static cudaLaunchConfig_t team_config(u32 blocks, u32 threads, size_t smem, cudaStream_t stream,
-                                      cudaLaunchAttribute &attr, int team) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    if (team == TEAM_CLUSTER) {
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = blocks;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-    } else {
-        attr.id = cudaLaunchAttributeCooperative;
-        attr.val.cooperative = 1;
-    }
-    cfg.attrs = &attr;
-    cfg.numAttrs = team == TEAM_BLOCK ? 0 : 1;
-    return cfg;
-}
-
 // Per device, once: shared-memory and cluster-size limits of the team
 // kernels; returns the largest cluster that the device can run with the
 // largest tables.
@@ -2765,18 +2740,10 @@ static u32 team_limits(int device) {
         const void *kc = team_kernel(TEAM_CLUSTER, k, promap), *kg = team_kernel(TEAM_GRID, k, promap);
         const size_t sc = team_smem(k, TEAM_CLUSTER_THREADS / 32, promap);
         const size_t sg = team_smem(k, TEAM_GRID_THREADS / 32, promap);
-        HP_CUDA(cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sc));
         HP_CUDA(cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sg));
         HP_CUDA(cudaFuncSetAttribute(team_kernel(TEAM_BLOCK, k, promap), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int) TEAM_BLOCK_SMEM));
-        HP_CUDA(cudaFuncSetAttribute(kc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        for (; best > 1; best /= 2) {
-            cudaLaunchAttribute attr;
-            const cudaLaunchConfig_t cfg = team_config(best, TEAM_CLUSTER_THREADS, sc, nullptr, attr, TEAM_CLUSTER);
-            int fits = 0;
-            if (cudaOccupancyMaxActiveClusters(&fits, kc, &cfg) == cudaSuccess && fits > 0) break;
-            cudaGetLastError();
-        }
+                                     (int) TEAM_SMEM_MAX));
+        best = team_cluster_limit(kc, sc, best);
     }
     done.emplace_back(device, best);
     return best;
@@ -2859,7 +2826,7 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
         a.bar = a.cnt + 2 * TC_N;
         a.bw = (s32 *) (a.bar + 2);
         a.hist = (u32 *) (a.bw + k);
-        const u32 threads = team == TEAM_CLUSTER ? TEAM_CLUSTER_THREADS : TEAM_GRID_THREADS;
+        const u32 threads = team_threads(team);
         const size_t smem = team_smem(k, threads / 32, promap);
         if (team == TEAM_GRID) coop.emplace(ctx.device, ctx.stream, blocks, (u32) ctx.sm_count);
         KernTimer kt(ctx, team == TEAM_CLUSTER ? "k_jet_fused" : "k_jet_coop");
@@ -2881,22 +2848,12 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
 
 // Blocks of the cooperative level loop for a level of n vertices and m
 // entries (0 when it does not apply): one per Tunables::jet_coop_rows vertices
-// or 16 times as many entries, at least two, at most as many as fit on the GPU
-// at once. 512 rows against 1024 / 2048 (one B200): ultra R-MAT 65k 222 / 229
-// / 253 ms, RGG 200k 20.5 / 20.7 / 21.8 ms. Beside other solves (HM sub-solves,
-// batch and server workers) a grid takes a share of the SMs, so that grids run
-// side by side instead of one after another at full width: HM RGG 8M 403 ms
-// uncapped, 342 / 359 ms with at least 32 / 64 blocks each.
-static u32 coop_blocks(Ctx &ctx, u32 n, u64 m, u32 k, bool promap) {
-    int per_sm = 0;
-    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, team_kernel(TEAM_GRID, k, promap), TEAM_GRID_THREADS,
-                                                          team_smem(k, TEAM_GRID_THREADS / 32, promap)));
-    if (per_sm <= 0) return 0;
+// or 16 times as many entries. 512 rows against 1024 / 2048 (one B200): ultra
+// R-MAT 65k 222 / 229 / 253 ms, RGG 200k 20.5 / 20.7 / 21.8 ms.
+static u32 coop_blocks(const Ctx &ctx, u32 n, u64 m, u32 k, bool promap) {
     const u64 rows = std::max<u32>(1, ctx.tune.jet_coop_rows);
-    const u64 want = (std::max<u64>(n, m / 16) + rows - 1) / rows;
-    u64 cap = (u64) per_sm * ctx.sm_count;
-    if (ctx.peers > 1) cap = std::min<u64>(cap, std::max<u64>(TEAM_PEER_BLOCKS, 2 * (u64) ctx.sm_count / ctx.peers));
-    return (u32) std::max<u64>(2, std::min<u64>(want, cap));
+    return team_grid_blocks(ctx, team_kernel(TEAM_GRID, k, promap), team_smem(k, TEAM_GRID_THREADS / 32, promap),
+                            (std::max<u64>(n, m / 16) + rows - 1) / rows);
 }
 
 void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultra, u32 level, s64 &obj, s32 &maxw,
@@ -2919,7 +2876,7 @@ void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultr
         const bool fused = g.n <= std::min<u32>(ctx.tune.jet_fused_max_n, TEAM_CLUSTER_MAX_N) &&
                            g.m <= ctx.tune.jet_fused_max_m;
         if (fused && g.n <= TEAM_BLOCK_MAX_N &&
-            team_level_offset(k, promap) + team_level_smem(g.n, g.m, k, width) <= TEAM_BLOCK_SMEM) {
+            team_level_offset(k, promap) + team_level_smem(g.n, g.m, k, width) <= TEAM_SMEM_MAX) {
             team = TEAM_BLOCK;
             blocks = 1;
         } else if (fused) {

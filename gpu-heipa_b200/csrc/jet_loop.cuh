@@ -42,11 +42,9 @@ constexpr u32 TEAM_HUB = 1024;         // rows above this length are evaluated b
 constexpr u32 TEAM_LONG = 64;          // afterburner / delta rows above this length take a whole warp
 constexpr u32 TEAM_LIST = 128;         // distinct-block list slots per warp (mapping objective; at least k)
 constexpr u32 TEAM_RANK_MAX = 32768;   // evicted vertices ranked by counting; more are left to the per-kernel path
-constexpr u32 TEAM_CLUSTER_MAX = 16;   // blocks of a cluster team
 
 constexpr u32 TEAM_OWN = 64;           // candidates / moves of a warp kept in shared memory up to this range
 
-enum TeamKind { TEAM_BLOCK = 0, TEAM_CLUSTER = 1, TEAM_GRID = 2 };
 enum TeamCnt { TC_HUB = 0, TC_MOVES = 1, TC_FAIL = 2, TC_N = 4 };
 enum TeamSum { TS_MOVES = 0, TS_DELTA = 1, TS_N = 2 };  // (moves << 32) + their row entries; objective change
 constexpr u32 TW_STILL = 0x80000000u;  // stamp flag: in the move list with an unchanged label
@@ -177,48 +175,6 @@ __device__ __forceinline__ TeamSm team_carve(unsigned char *base, u32 k, u32 war
     return S;
 }
 
-// ---- team barrier ----------------------------------------------------------------------
-
-// Cluster: the hardware barrier (release / acquire at cluster scope). Grid:
-// one counter that only grows; thread 0 of every block adds one and waits for
-// it to reach a multiple of the grid size. The wait is bounded: after
-// TEAM_SPINS polls a block adds TEAM_POISON, which ends every wait, and all
-// blocks leave (the host redoes the level).
-constexpr u32 TEAM_POISON = 0x80000000u;
-constexpr u32 TEAM_SPINS = 1u << 21;
-
-template<int TEAM>
-__device__ __forceinline__ bool team_barrier(u32 *bar, u32 &target, u32 *err) {
-    if (TEAM == TEAM_BLOCK) {
-        __syncthreads();
-        return true;
-    }
-    if (TEAM == TEAM_CLUSTER) {
-        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-        return true;
-    }
-    __shared__ u32 s_ok;
-    target += gridDim.x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        u32 v;
-        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(bar) : "memory");
-        v += 1;
-        u32 spins = 0;
-        while (v < target) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-            if (++spins > TEAM_SPINS) {
-                set_error(err, DEV_ERR_SPIN);
-                atomicOr(bar, TEAM_POISON);
-                v = TEAM_POISON;
-            }
-        }
-        s_ok = v < TEAM_POISON ? 1u : 0u;
-    }
-    __syncthreads();
-    return s_ok != 0u;
-}
-
 // Graph reads: the level is in shared memory (block team) or constant in
 // global memory.
 template<int TEAM, typename T>
@@ -238,13 +194,6 @@ __device__ __forceinline__ void ld_row(const TeamArgs &a, u32 u, u32 &beg, u32 &
     beg = ld_graph<TEAM>(&a.rowptr[u]);
     len = TEAM == TEAM_BLOCK ? a.rowptr[u + 1] - beg : __ldg(&a.rowlen[u]);
 }
-// A word that other blocks wrote before the last barrier and that steers the
-// control flow: from L2, or shared memory.
-template<int TEAM, typename T>
-__device__ __forceinline__ T ld_fresh(const T *p) {
-    return TEAM == TEAM_BLOCK ? *(const volatile T *) p : __ldcg(p);
-}
-
 // ---- row evaluation --------------------------------------------------------------------
 
 enum TeamOp { OP_CUT = 0, OP_MAP = 1, OP_WEAK = 2, OP_STRONG = 3 };

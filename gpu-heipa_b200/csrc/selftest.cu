@@ -1,6 +1,6 @@
 // Diagnostics of the bounded waits (hp_selftest_barrier_timeout, declared in
 // include/gpuheipa.h). The cooperative level loops wait for one another at
-// grid barriers whose wait is bounded (grid_barrier, common.cuh): when a
+// grid barriers whose wait is bounded (team_barrier, team.cuh): when a
 // block does not arrive, the others give up after about a second, set an
 // error bit and end, and the host reports an error instead of hanging. This
 // entry point exercises exactly that path with a block that never arrives, so
@@ -10,6 +10,7 @@
 #include "../../include/gpuheipa.h"
 #include "common.cuh"
 #include "context.h"
+#include "team.cuh"
 
 #include <cuda_runtime.h>
 
@@ -20,7 +21,8 @@ namespace {
 
 __global__ void k_barrier_selftest(u32 *bar, u32 *err, u32 absent) {
     if (blockIdx.x == absent) return;  // this block never reaches the barrier
-    grid_barrier(bar, err);
+    u32 target = 0;
+    team_barrier<TEAM_GRID>(bar, target, err);
 }
 
 } // namespace

@@ -48,6 +48,58 @@ struct Hierarchy {
     std::vector<u32 *> maps;
 };
 
+enum class CoarsenStep { None, Matched, Contracted };
+
+// One level by the single-launch kernel, where it applies: the mapping and
+// coarse size (Matched), and the coarse graph in the front of the arena
+// (Contracted) unless the level shrinks by less than 1%. None: nothing was
+// done (level too large, no room for its scratch, or the launch gave up).
+CoarsenStep coarsen_level(Ctx &ctx, const DGraph &g, u32 *mp, DGraph &c, u32 &nc, SolveStats *stats) {
+    if (!coarsen_team_applies(ctx, g)) return CoarsenStep::None;
+    ProfScope prof(ctx, "coarsen_level");
+    auto t0 = Clock::now();
+    const size_t mark = ctx.arena.front_mark();
+    CoarsenResult r;
+    try {
+        ScratchScope ss(ctx.arena);
+        c = DGraph{};
+        c.cap = g.m;
+        c.total_vw = g.total_vw;
+        c.adj = ctx.falloc<u32>(c.cap);
+        c.ew = ctx.falloc<s32>(c.cap);
+        r = coarsen_team(ctx, g, mp, &c);
+        nc = r.n;
+        if (r.contracted && (u64) nc * 100 <= (u64) g.n * 99) {
+            c.n = nc;
+            c.m = r.m;
+            c.rowptr = ctx.falloc<u32>((u64) nc + 1);
+            c.rowlen = ctx.falloc<u32>(nc);
+            c.vw = ctx.falloc<s32>(nc);
+            auto keep = [&](void *dst, const void *src, size_t bytes) {
+                HP_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, ctx.stream));
+            };
+            keep(c.rowptr, r.rowptr, sizeof(u32) * ((size_t) nc + 1));
+            keep(c.rowlen, r.rowlen, sizeof(u32) * nc);
+            keep(c.vw, r.vw, sizeof(s32) * nc);
+        } else {
+            r.contracted = false;
+            ctx.arena.front_release(mark);
+        }
+    } catch (const CoopSpin &) {
+        ctx.arena.front_release(mark);
+        return CoarsenStep::None;
+    } catch (const HpError &e) {
+        if (e.code != HP_ERR_OOM) throw;
+        ctx.arena.front_release(mark);
+        return CoarsenStep::None;
+    }
+    if (stats) {
+        stats->contraction_ms += r.contract_ms;
+        stats->coarsening_ms += ms_since(t0) - r.contract_ms;
+    }
+    return r.contracted ? CoarsenStep::Contracted : CoarsenStep::Matched;
+}
+
 // Coarsen while n > 8k (solver.h:343-347); stops early when a matching
 // shrinks its level by less than 1% (the reference has no such check and
 // loops on graphs that stop coarsening; every level here costs arena space).
@@ -57,12 +109,19 @@ void coarsen(Ctx &ctx, const DGraph &g, u32 k, Hierarchy &H, SolveStats *stats) 
         const DGraph cur = H.graphs.back();
         auto t0 = Clock::now();
         u32 *mp = ctx.falloc<u32>(cur.n);
-        const u32 nc = match_graph(ctx, cur, mp);
-        if (stats) stats->coarsening_ms += ms_since(t0);
+        DGraph c;
+        u32 nc = 0;
+        const CoarsenStep step = coarsen_level(ctx, cur, mp, c, nc, stats);
+        if (step == CoarsenStep::None) {
+            nc = match_graph(ctx, cur, mp);
+            if (stats) stats->coarsening_ms += ms_since(t0);
+        }
         if ((u64) nc * 100 > (u64) cur.n * 99) break;
-        auto t1 = Clock::now();
-        DGraph c = contract_graph(ctx, cur, mp, nc);
-        if (stats) stats->contraction_ms += ms_since(t1);
+        if (step != CoarsenStep::Contracted) {
+            auto t1 = Clock::now();
+            c = contract_graph(ctx, cur, mp, nc);
+            if (stats) stats->contraction_ms += ms_since(t1);
+        }
         H.graphs.push_back(c);
         H.maps.push_back(mp);
     }

@@ -211,8 +211,8 @@ int hp_coop_slot_release(int device);
  * (levels up to this many CSR entries replay Jet iterations as CUDA graphs;
  * 0 = never), "order_small_n" (single-block rebalance ordering up to this many
  * vertices, at most 65536; 0 = never), "match_coop_max_n" / "match_coop_max_m"
- * (one cooperative launch for the matching loop of levels up to these sizes;
- * 0 = never), "jet_fused_max_n" / "jet_fused_max_m" (the whole refinement loop
+ * (one launch for the matching and contraction of levels up to these sizes,
+ * vertices capped at 1048576; 0 = never), "jet_fused_max_n" / "jet_fused_max_m" (the whole refinement loop
  * of a level in one launch of a thread-block cluster up to these sizes,
  * vertices capped at 65536, when k <= 1024, or k <= 256 for the mapping
  * objective; 0 = never), "jet_coop_max_n" / "jet_coop_max_m" /
