@@ -2710,18 +2710,16 @@ constexpr u32 TEAM_BLOCK_MAX_N = 4096;
 constexpr u64 TEAM_ANY_DEG_M = 1ull << 21;
 constexpr u64 TEAM_MID_DEG_M = 1ull << 26, TEAM_MID_DEG = 128;
 
+template<bool HASH, bool MAP>
+static const void *team_kernel_of(int team) {
+    return team == TEAM_BLOCK ? (const void *) k_jet_block<HASH, MAP>
+                              : (team == TEAM_CLUSTER ? (const void *) k_jet_team<TEAM_CLUSTER, HASH, MAP>
+                                                      : (const void *) k_jet_team<TEAM_GRID, HASH, MAP>);
+}
+
 static const void *team_kernel(int team, u32 k, bool promap) {
-    if (team == TEAM_BLOCK) {
-        if (promap) return (const void *) k_jet_block<8, true>;
-        return k <= 256 ? (const void *) k_jet_block<8, false> : (const void *) k_jet_block<32, false>;
-    }
-    if (team == TEAM_CLUSTER) {
-        if (promap) return (const void *) k_jet_team<TEAM_CLUSTER, 8, true>;
-        return k <= 256 ? (const void *) k_jet_team<TEAM_CLUSTER, 8, false>
-                        : (const void *) k_jet_team<TEAM_CLUSTER, 32, false>;
-    }
-    if (promap) return (const void *) k_jet_team<TEAM_GRID, 8, true>;
-    return k <= 256 ? (const void *) k_jet_team<TEAM_GRID, 8, false> : (const void *) k_jet_team<TEAM_GRID, 32, false>;
+    if (promap) return team_kernel_of<false, true>(team);
+    return k <= TEAM_DIRECT_K ? team_kernel_of<false, false>(team) : team_kernel_of<true, false>(team);
 }
 
 // Per device, once: shared-memory and cluster-size limits of the team

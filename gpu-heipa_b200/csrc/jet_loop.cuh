@@ -25,10 +25,12 @@
 //    over the vertex ranges, prefix sums over them and a prefix within 32
 //    vertices. Strong rebalancing needs the exact prefix of every evicted
 //    vertex: the few evicted ones are ranked among each other;
-//  * rows are evaluated by 8 lanes (32 lanes for k > 256) with a
-//    direct-indexed block table in shared memory: an entry costs one add and
-//    one exchange, which collects each distinct block once and clears the
-//    table; no pass over all k blocks.
+//  * rows of up to 32 entries are evaluated by 8 lanes with a block table in
+//    shared memory (direct-indexed, or 64 hashed slots for k > 256): an entry
+//    costs one add and one exchange, which collects each distinct block once
+//    and clears the table; no pass over all k blocks;
+//  * long rows are shared by the warps of their block (afterburner, objective
+//    change), so that no warp scans a hub row alone.
 // Measured (one B200, mean time of one iteration): the levels of an RGG with
 // 3001 vertices, 27 us with one 1024-thread block per level in global memory,
 // 14 us as cluster teams with shared lists, now 10.5 us on the levels that fit
@@ -39,11 +41,14 @@
 #pragma once
 
 constexpr u32 TEAM_HUB = 1024;         // rows above this length are evaluated by a whole block
-constexpr u32 TEAM_LONG = 64;          // afterburner / delta rows above this length take a whole warp
+constexpr u32 TEAM_LONG = 64;          // afterburner / delta rows above this length take a whole warp ...
+constexpr u32 TEAM_SHARE = 256;        // ... and above this one the warps of the block, 128 entries at a time
+constexpr u32 TEAM_SHARE_MAX = 128;    // rows a block shares in one phase (others stay with their warp)
+constexpr u32 TEAM_DIRECT_K = 256;     // direct-indexed tables per 8 lanes up to this k, hashed ones above
 constexpr u32 TEAM_LIST = 128;         // distinct-block list slots per warp (mapping objective; at least k)
 constexpr u32 TEAM_RANK_MAX = 32768;   // evicted vertices ranked by counting; more are left to the per-kernel path
 
-constexpr u32 TEAM_OWN = 64;           // candidates / moves of a warp kept in shared memory up to this range
+constexpr u32 TEAM_OWN = 48;           // candidates / moves of a warp kept in shared memory up to this range
 
 enum TeamCnt { TC_HUB = 0, TC_MOVES = 1, TC_FAIL = 2, TC_N = 4 };
 enum TeamSum { TS_MOVES = 0, TS_DELTA = 1, TS_N = 2 };  // (moves << 32) + their row entries; objective change
@@ -129,9 +134,10 @@ struct TeamSm {
 constexpr size_t TEAM_VERTEX_BYTES = 8 + 8 + 16 + 7 * 4;
 
 // Bytes of dynamic shared memory of a team block of `warps` warps.
+__host__ __device__ inline u32 team_stride(u32 k) { return k <= TEAM_DIRECT_K ? 4 * k : (k < 512 ? 512 : k); }
+
 inline size_t team_smem(u32 k, u32 warps, bool promap) {
-    const size_t groups = k <= 256 ? 4 : 1;
-    size_t b = (size_t) warps * groups * k * 4;
+    size_t b = (size_t) warps * team_stride(k) * 4;
     b = (b + 15) & ~(size_t) 15;
     if (promap) b += (size_t) warps * std::max<u32>(TEAM_LIST, k) * 8;
     b += ((size_t) k + 2) * 8 * 2 + (size_t) k * 4 * 10 + 32 * 4 + (size_t) warps * 2 * TEAM_OWN * 4;
@@ -144,10 +150,9 @@ inline size_t team_level_smem(u32 n, u64 m, u32 k, u32 width) {
            (2 * TS_N) * 8 + (2 * TC_N + k + k) * 4 + 64;
 }
 
-template<int GL>
 __device__ __forceinline__ TeamSm team_carve(unsigned char *base, u32 k, u32 warps, u32 warp, bool promap) {
     TeamSm S;
-    S.stride = (32 / GL) * k;
+    S.stride = team_stride(k);
     S.tab0 = (s32 *) base;
     S.tab = S.tab0 + warp * S.stride;
     size_t off = ((size_t) warps * S.stride * 4 + 15) & ~(size_t) 15;
@@ -265,15 +270,17 @@ __device__ __forceinline__ void row_reduce(RowOut &r) {
 
 __device__ __forceinline__ u32 label_of(const TeamArgs &a, u32 v) { return ((const u32 *) a.tw)[2 * (u64) v] & 0xFFFFu; }
 
-// Evaluates the rows of the lanes in `need` (beg, len <= 4 * GL, own block o
-// of each lane's row), 32 / GL rows at a time, GL lanes per row; every lane
-// receives its row's result. All lanes of the warp call this.
-template<int TEAM, int OP, int GL>
+// Evaluates the rows of the lanes in `need` (beg, len <= 32, own block o of
+// each lane's row), four rows at a time, 8 lanes per row; every lane receives
+// its row's result. HASH: 64 slots of (block + 1, connection) per row instead
+// of a direct-indexed table; both are all zero between rows. All lanes of the
+// warp call this.
+template<int TEAM, int OP, bool HASH>
 __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u32 need, u32 beg, u32 len, u32 o,
                                            s32 max_b_w, RowOut &out) {
-    constexpr int NG = 32 / GL;
+    constexpr int NG = 4, GL = 8;
     const u32 lane = lane_id(), g = lane / GL, gl = lane % GL;
-    s32 *tv = S.tab + g * a.k;
+    s32 *tv = S.tab + g * (HASH ? 128 : a.k);
     while (need) {
         u32 m = need, rest = need;
 #pragma unroll
@@ -297,14 +304,31 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
 #pragma unroll
         for (int j = 0; j < 4; ++j)
             if (b[j] != EMPTY) b[j] = label_of(a, b[j]);
+        u32 at[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            at[j] = b[j];
+            if (HASH && b[j] != EMPTY) {  // at most 32 keys in 64 slots
+                u32 h = (b[j] * 2654435761u) >> 26;
+                for (;;) {
+                    const u32 prev = atomicCAS((u32 *) &tv[h], 0u, b[j] + 1);
+                    if (prev == 0 || prev == b[j] + 1) break;
+                    h = (h + 1) & 63u;
+                }
+                at[j] = 64 + h;
+            }
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (b[j] != EMPTY) atomicAdd(&tv[b[j]], w[j]);
+            if (b[j] != EMPTY) atomicAdd(&tv[at[j]], w[j]);
         __syncwarp();
         // the exchange returns a block's connection to one of its entries and
         // clears the table
 #pragma unroll
-        for (int j = 0; j < 4; ++j) w[j] = b[j] != EMPTY ? atomicExch(&tv[b[j]], 0) : 0;
+        for (int j = 0; j < 4; ++j) {
+            w[j] = b[j] != EMPTY ? atomicExch(&tv[at[j]], 0) : 0;
+            if (HASH && w[j] != 0) tv[at[j] - 64] = 0;
+        }
         __syncwarp();
         RowOut r{0, 0, 0, 0};
         if (OP == OP_MAP) {
@@ -312,7 +336,7 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
             u32 cnt = 0;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const u32 mask = (__ballot_sync(FULL, w[j] != 0) >> (g * GL)) & (GL == 32 ? FULL : (1u << GL) - 1u);
+                const u32 mask = (__ballot_sync(FULL, w[j] != 0) >> (g * GL)) & 0xFFu;
                 if (w[j] != 0) list[cnt + __popc(mask & ((1u << gl) - 1u))] = ((unsigned long long) b[j] << 32) | (u32) w[j];
                 cnt += __popc(mask);
             }
@@ -586,13 +610,20 @@ __device__ __forceinline__ s32 team_load_bw(const TeamArgs &a, const TeamSm &S, 
         if (!team_barrier<TEAM>(a.bar, bar_target, &a.out->err)) return;     \
     } while (0)
 
-// The level loop of one team of gridDim.x blocks. GL: lanes per short row.
+// The level loop of one team of gridDim.x blocks. HASH: hashed tables for
+// short rows (k > TEAM_DIRECT_K).
 // MAP: process-mapping objective.
-template<int TEAM, int GL, bool MAP>
+template<int TEAM, bool HASH, bool MAP>
 __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl, const TeamSm &S) {
     __shared__ long long sl[33];
     __shared__ u32 su[33], su2[33];
     __shared__ s32 smx[32];
+    // rows shared by the block: candidates (vertex, row, record, sum of the
+    // afterburner terms) and moved vertices (row, vertex word)
+    __shared__ u32 c_cnt, m_cnt, c_u[TEAM_SHARE_MAX], c_beg[TEAM_SHARE_MAX], c_len[TEAM_SHARE_MAX],
+        m_beg[TEAM_SHARE_MAX], m_len[TEAM_SHARE_MAX];
+    __shared__ unsigned long long c_rec[TEAM_SHARE_MAX], m_tw[TEAM_SHARE_MAX];
+    __shared__ s32 c_sum[TEAM_SHARE_MAX];
     const u32 tid = threadIdx.x, lane = lane_id(), warp = warp_in_block(), nw = blockDim.x >> 5;
     const u32 n = a.n, k = a.k, G = gridDim.x;
     const u32 g = lane >> 3, gl = lane & 7;  // 8-lane groups of the list passes
@@ -620,6 +651,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
     if (__any_sync(FULL, hub) && lane == 0) atomicOr(&a.out->hubs, 1u);
     __syncthreads();
     team_flush_bw(a, S);
+    if (tid == 0) c_cnt = m_cnt = 0;
     TEAM_SYNC();
     const bool hubs = ld_fresh<TEAM>(&a.out->hubs) != 0;
     team_load_bw<TEAM>(a, S, smx);
@@ -675,8 +707,8 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                     if (need && !small) ld_row<TEAM>(a, u, beg, len);
                     const bool hb = need && len > TEAM_HUB;
                     RowOut r{0, 0, 0, 0};
-                    rows_short<TEAM, OP, GL>(a, S, __ballot_sync(FULL, need && len <= 4 * GL), beg, len, o, 0, r);
-                    rows_long<TEAM, OP>(a, S, __ballot_sync(FULL, need && len > 4 * GL && !hb), beg, len, o, 0, r);
+                    rows_short<TEAM, OP, HASH>(a, S, __ballot_sync(FULL, need && len <= 32), beg, len, o, 0, r);
+                    rows_long<TEAM, OP>(a, S, __ballot_sync(FULL, need && len > 32 && !hb), beg, len, o, 0, r);
                     if (need && !hb) {
                         lp_decide<MAP>(r, ratio, dest, gain);
                         a.dest_cache[u] = dest;
@@ -740,7 +772,19 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                     __syncwarp();
 #pragma unroll
                     for (int d = 4; d > 0; d >>= 1) ch = wadd(ch, __shfl_xor_sync(FULL, ch, d));
-                    u32 lng = __ballot_sync(FULL, gl == 0 && len > TEAM_LONG);
+                    bool mine = act && gl == 0;  // decided here
+                    if (mine && len > TEAM_SHARE) {
+                        const u32 p = atomicAdd(&c_cnt, 1u);
+                        if (p < TEAM_SHARE_MAX) {
+                            c_u[p] = u;
+                            c_beg[p] = beg;
+                            c_len[p] = len;
+                            c_rec[p] = rec;
+                            c_sum[p] = 0;
+                            mine = false;
+                        }
+                    }
+                    u32 lng = __ballot_sync(FULL, mine && len > TEAM_LONG);
                     while (lng) {
                         const int src = __ffs(lng) - 1;
                         lng &= lng - 1;
@@ -752,7 +796,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                             (s32) warp_sum<u32>((u32) team_ab<TEAM, MAP>(a, S, xu, xg, xo, xn, xb, xl, lane, 32));
                         if ((int) lane == src) ch = c;
                     }
-                    const bool mv = act && gl == 0 && wadd(ug, ch) >= 0;
+                    const bool mv = mine && wadd(ug, ch) >= 0;
                     if (mv) {
                         a.lock[u] = 1;
                         team_move(a, S, u, ou, nu, ld_vw<TEAM>(a, u), stamp);
@@ -761,6 +805,42 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                     const u32 mask = __ballot_sync(FULL, mv);
                     if (mv) ml[n_own + __popc(mask & lt)] = u;
                     n_own += __popc(mask);
+                }
+                // the block's long candidates, 128 entries per warp and turn
+                __syncthreads();
+                const u32 n_long = min(c_cnt, TEAM_SHARE_MAX);
+                if (n_long) {
+                    for (u32 i = 0; i < n_long; ++i) {
+                        const u32 len = c_len[i], beg = c_beg[i], u = c_u[i];
+                        const unsigned long long rec = c_rec[i];
+                        const s32 ug = (s32) (u32) rec;
+                        const u32 nu = (u32) (rec >> 32) & 0xFFFFu, ou = (u32) (rec >> 48);
+                        s32 part = 0;
+                        bool any = false;
+                        for (u32 t = ((warp + 5 * i) % nw) * 128; t < len; t += nw * 128) {
+                            part = wadd(part, team_ab<TEAM, MAP>(a, S, u, ug, ou, nu, beg + t, min(len - t, 128u), lane, 32));
+                            any = true;
+                        }
+                        if (any) {
+                            part = (s32) warp_sum<u32>((u32) part);
+                            if (lane == 0) atomicAdd(&c_sum[i], part);
+                        }
+                    }
+                    __syncthreads();
+                    if (tid < n_long) {
+                        const u32 u = c_u[tid], len = c_len[tid];
+                        const unsigned long long rec = c_rec[tid];
+                        if (wadd((s32) (u32) rec, c_sum[tid]) >= 0) {
+                            const u32 nu = (u32) (rec >> 32) & 0xFFFFu, ou = (u32) (rec >> 48);
+                            a.lock[u] = 1;
+                            team_move(a, S, u, ou, nu, ld_vw<TEAM>(a, u), stamp);
+                            moved += (1ll << 32) + len;
+                            const u32 p = atomicAdd(&m_cnt, 1u);  // at most n_long
+                            m_beg[p] = c_beg[tid];
+                            m_len[p] = len;
+                            m_tw[p] = a.tw[u];
+                        }
+                    }
                 }
             } else {
                 const bool strong = step == 2;
@@ -842,13 +922,13 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                     if (need && !small) ld_row<TEAM>(a, u, beg, len);
                     const bool hb = need && len > TEAM_HUB;
                     RowOut r{0, 0, 0, 0};
-                    const u32 ms = __ballot_sync(FULL, need && len <= 4 * GL);
-                    const u32 mg = __ballot_sync(FULL, need && len > 4 * GL && !hb);
+                    const u32 ms = __ballot_sync(FULL, need && len <= 32);
+                    const u32 mg = __ballot_sync(FULL, need && len > 32 && !hb);
                     if (strong) {
-                        rows_short<TEAM, OP_STRONG, GL>(a, S, ms, beg, len, o, max_b_w, r);
+                        rows_short<TEAM, OP_STRONG, HASH>(a, S, ms, beg, len, o, max_b_w, r);
                         rows_long<TEAM, OP_STRONG>(a, S, mg, beg, len, o, max_b_w, r);
                     } else {
-                        rows_short<TEAM, OP_WEAK, GL>(a, S, ms, beg, len, o, max_b_w, r);
+                        rows_short<TEAM, OP_WEAK, HASH>(a, S, ms, beg, len, o, max_b_w, r);
                         rows_long<TEAM, OP_WEAK>(a, S, mg, beg, len, o, max_b_w, r);
                     }
                     u32 key = NOKEY;
@@ -1112,8 +1192,11 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                     __syncthreads();
                     // exact prefix of each evicted vertex among its block's
                     // and the first slot attempt (adjust_scores :560-584)
-                    for (u32 j0 = gw * 4; j0 < ns; j0 += gwarps * 4) {
-                        const u32 j = j0 + g;
+                    // (8 lanes per vertex, or a warp when there are enough)
+                    const u32 lanes = ns <= gwarps ? 32 : 8, li = lane & (lanes - 1);
+                    const u32 each = 32 / lanes;
+                    for (u32 j0 = gw * each; j0 < ns; j0 += gwarps * each) {
+                        const u32 j = j0 + lane / lanes;
                         const bool act = j < ns;
                         unsigned long long comp = 0, ow = 0;
                         if (act) {
@@ -1124,15 +1207,14 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                         s32 x = 0;
                         if (act) {
 #pragma unroll 4
-                            for (u32 i = gl; i < ns; i += 8) {
+                            for (u32 i = li; i < ns; i += lanes) {
                                 const unsigned long long ci = a.mcomp[i], wi = a.mow[i];
                                 if ((u32) (wi >> 32) == o && ci < comp) x += (s32) (u32) wi;
                             }
                         }
                         __syncwarp();
-#pragma unroll
-                        for (int d = 4; d > 0; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
-                        if (act && gl == 0) {
+                        for (u32 d = lanes / 2; d > 0; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
+                        if (act && li == 0) {
                             const u32 u = (u32) comp;
                             const s32 vw = (s32) (u32) ow;
                             const long long tg = (long long) S.spill[o] + x + S.pre[o];
@@ -1222,7 +1304,17 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                         acc += team_delta<TEAM, MAP>(a, S, tw_old(x), tw_label(x), tw_stamp(x) == stamp, stamp, beg, len,
                                                      gl, 8, inval);
                     __syncwarp();
-                    u32 lng = __ballot_sync(FULL, gl == 0 && len > TEAM_LONG);
+                    bool mine = gl == 0 && len > TEAM_LONG;
+                    if (mine && len > TEAM_SHARE) {
+                        const u32 p = atomicAdd(&m_cnt, 1u);
+                        if (p < TEAM_SHARE_MAX) {
+                            m_beg[p] = beg;
+                            m_len[p] = len;
+                            m_tw[p] = x;
+                            mine = false;
+                        }
+                    }
+                    u32 lng = __ballot_sync(FULL, mine);
                     while (lng) {
                         const int src = __ffs(lng) - 1;
                         lng &= lng - 1;
@@ -1235,7 +1327,18 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
             }
             if (!inval)
                 for (u32 u = r0 + lane; u < r1; u += 32) a.dest_cache[u] = NULL_PART;
-            team_add(acc, &sum[TS_DELTA], sl);
+            // the block's long moved rows, 128 entries per warp and turn
+            __syncthreads();
+            const u32 m_long = min(m_cnt, TEAM_SHARE_MAX);
+            for (u32 i = 0; i < m_long; ++i) {
+                const u32 len = m_len[i], beg = m_beg[i];
+                const unsigned long long x = m_tw[i];
+                for (u32 t = ((warp + 5 * i) % nw) * 128; t < len; t += nw * 128)
+                    acc += team_delta<TEAM, MAP>(a, S, tw_old(x), tw_label(x), tw_stamp(x) == stamp, stamp, beg + t,
+                                                 min(len - t, 128u), lane, 32, inval);
+            }
+            team_add(acc, &sum[TS_DELTA], sl);  // (every thread has read m_cnt after its barrier)
+            if (tid == 0) c_cnt = m_cnt = 0;
             TEAM_SYNC();
             const long long d = ld_fresh<TEAM>(&sum[TS_DELTA]);
             // control (jet_label_propagation.h:966-1030, promap :1250-1305)
@@ -1278,10 +1381,10 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
 #undef TEAM_SYNC
 
 // Zeroes the tables and loads the distance oracle.
-template<int GL, bool MAP>
+template<bool MAP>
 __device__ __forceinline__ TeamSm team_setup(const TeamArgs &a, unsigned char *dsm) {
     const u32 tid = threadIdx.x, nw = blockDim.x >> 5;
-    const TeamSm S = team_carve<GL>(dsm, a.k, nw, warp_in_block(), MAP);
+    const TeamSm S = team_carve(dsm, a.k, nw, warp_in_block(), MAP);
     for (u32 i = tid; i < nw * S.stride; i += blockDim.x) S.tab0[i] = 0;
     for (u32 b = tid; b < a.k; b += blockDim.x) {
         S.bd[b] = 0;
@@ -1293,22 +1396,22 @@ __device__ __forceinline__ TeamSm team_setup(const TeamArgs &a, unsigned char *d
 }
 
 // A cluster or a cooperative grid on a level in global memory.
-template<int TEAM, int GL, bool MAP>
+template<int TEAM, bool HASH, bool MAP>
 __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ TeamArgs a,
                                                         const __grid_constant__ TeamCtl ctl) {
     extern __shared__ __align__(16) unsigned char team_dsm[];
-    const TeamSm S = team_setup<GL, MAP>(a, team_dsm);
-    team_loop<TEAM, GL, MAP>(a, ctl, S);
+    const TeamSm S = team_setup<MAP>(a, team_dsm);
+    team_loop<TEAM, HASH, MAP>(a, ctl, S);
 }
 
 // One block that copies the level to shared memory first (rows made
 // contiguous). `level` is the offset of the level's arrays.
-template<int GL, bool MAP>
+template<bool HASH, bool MAP>
 __global__ void __launch_bounds__(512, 1) k_jet_block(const __grid_constant__ TeamArgs ga,
                                                         const __grid_constant__ TeamCtl ctl, u32 m, u32 level) {
     extern __shared__ __align__(16) unsigned char team_dsm[];
     __shared__ u32 scan_sm[32];
-    const TeamSm S = team_setup<GL, MAP>(ga, team_dsm);
+    const TeamSm S = team_setup<MAP>(ga, team_dsm);
     const u32 n = ga.n, k = ga.k, tid = threadIdx.x, lane = lane_id();
     TeamArgs a = ga;
     unsigned long long *q = (unsigned long long *) (team_dsm + level);
@@ -1375,7 +1478,7 @@ __global__ void __launch_bounds__(512, 1) k_jet_block(const __grid_constant__ Te
     a.adj = adj;
     a.ew = ew;
     a.vw = vw;
-    team_loop<TEAM_BLOCK, GL, MAP>(a, ctl, S);
+    team_loop<TEAM_BLOCK, HASH, MAP>(a, ctl, S);
     if (tid == 0) {
         ga.out->obj = out->obj;
         ga.out->maxw = out->maxw;

@@ -12,7 +12,7 @@ constexpr u32 TEAM_CLUSTER_MAX = 16;        // blocks of a cluster team
 constexpr u32 TEAM_BLOCK_THREADS = 512;     // threads of a block team ...
 constexpr u32 TEAM_CLUSTER_THREADS = 512;   // ... of a block of a cluster team ...
 constexpr u32 TEAM_GRID_THREADS = 1024;     // ... and of a grid team
-constexpr size_t TEAM_SMEM_MAX = 226 * 1024;  // dynamic shared memory of a block (1 KB is left for static arrays)
+constexpr size_t TEAM_SMEM_MAX = 220 * 1024;  // dynamic shared memory of a block (7 KB are left for static arrays)
 
 inline u32 team_threads(int team) {
     return team == TEAM_GRID ? TEAM_GRID_THREADS : (team == TEAM_CLUSTER ? TEAM_CLUSTER_THREADS : TEAM_BLOCK_THREADS);
