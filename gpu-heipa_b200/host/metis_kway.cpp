@@ -54,11 +54,55 @@ constexpr int OPT_REFINE = 1;   // kway_utility.h:39
 constexpr int OPT_BALANCE = 2;  // kway_utility.h:40
 constexpr int FREE = -1;        // unmatched (kway_utility.h:42)
 
+// Arrays whose elements are all written before they are read: not cleared on
+// allocation. A k-way partition makes hundreds of bisections of a few dozen
+// vertices, and clearing, copying and allocating took as long as the work.
+template<typename T>
+struct Uncleared : std::allocator<T> {
+    template<typename U>
+    struct rebind {
+        using other = Uncleared<U>;
+    };
+    template<typename U>
+    void construct(U *p) {
+        ::new ((void *) p) U;
+    }
+    template<typename U, typename... A>
+    void construct(U *p, A &&...a) {
+        ::new ((void *) p) U(std::forward<A>(a)...);
+    }
+};
+using IVec = std::vector<int, Uncleared<int> >;
+
+// Storage of a heap (MaxHeap): items, and positions that are -1 between uses.
+template<typename K>
+struct HeapStore {
+    struct Item {
+        K key;
+        int v;
+    };
+    std::vector<Item> h;
+    std::vector<int> at;
+};
+
+// The random sequence and the buffers of one partitioning call; between uses
+// every element of `slot`, `dense`, `moved` and the heaps' positions is -1.
+struct Rand : LibcRand {
+    using LibcRand::LibcRand;
+    std::vector<int> slot, dense, moved;
+    IVec swaps, perm;
+    HeapStore<int> q0, q1;
+    static std::vector<int> &room(std::vector<int> &v, int n) {
+        if ((int) v.size() < n) v.resize(n, -1);
+        return v;
+    }
+};
+
 // Graph of the partitioner (kway_graph.h): int arrays, the vertex weight
 // total `w` and the running cut of the current bisection or partition.
 struct KGraph {
     int n = -1, m = -1, w = -1;
-    std::vector<int> vw, xadj, adj, ew;
+    IVec vw, xadj, adj, ew;
     int cut = -1;
     KGraph() = default;
     KGraph(int n_, int m_, int w_ = 0) : n(n_), m(m_), w(w_), vw(n_), xadj(n_ + 1), adj(m_), ew(m_), cut(0) {}
@@ -77,8 +121,13 @@ struct KGraph {
 // order of `val` is observable (it is permuted and scanned).
 struct BndSet {
     int cnt = 0;
-    std::vector<int> pos, val;
+    IVec pos, val;
     explicit BndSet(int n = 0) : cnt(0), pos(n, -1), val(n) {}
+    // empties the set for a graph of n vertices (larger ids are not touched)
+    void clear(int n) {
+        cnt = 0;
+        std::fill_n(pos.begin(), n, -1);
+    }
     void add(int v) {
         val[cnt] = v;
         pos[v] = cnt++;
@@ -90,30 +139,32 @@ struct BndSet {
         pos[v] = -1;
     }
     bool has(int v) const { return pos[v] != -1; }
-    void clear() {
-        cnt = 0;
-        std::fill(pos.begin(), pos.end(), -1);
-    }
 };
 
 // Internal / external edge weight per vertex for a bisection (BisectInfo).
 struct Side2 {
-    std::vector<int> in, ex;
+    IVec in, ex;
     explicit Side2(int n = 0) : in(n), ex(n) {}
 };
 
 // Per-vertex block connectivity for the k-way refinement (kway_block_conn.h):
 // dense weights per (vertex, block), the list of connected blocks in
 // insertion order with swap-remove, internal and external weight, and a second
-// copy of the per-vertex counters for projection.
+// copy of the per-vertex counters for projection. A vertex's row of k weights
+// is cleared when it is first used after clear(): interior vertices have none
+// (n * k words were cleared three times per level before).
 class KConn {
 public:
     KConn(int n, int k)
         : n_(n), k_(k), cnt_(n, 0), cnt2_(n, 0), in_(n, 0), in2_(n, 0), ex_(n, 0), ex2_(n, 0),
-          w_((size_t) n * k, 0), at_((size_t) n * k, -1), ids_((size_t) n * k, -1) {}
+          row_(n, 0), w_((size_t) n * k), at_((size_t) n * k), ids_((size_t) n * k) {}
     void update(int v, int id, int delta) {
         if (delta == 0) return;
         const size_t o = (size_t) v * k_ + id;
+        if (row_[v] != epoch_) {
+            row_[v] = epoch_;
+            std::fill_n(w_.begin() + (size_t) v * k_, k_, 0);
+        }
         const int before = w_[o];
         const int after = before + delta;
         w_[o] = after;
@@ -131,18 +182,14 @@ public:
                 ids_[(size_t) v * k_ + p] = last_id;
                 at_[(size_t) v * k_ + last_id] = p;
             }
-            ids_[(size_t) v * k_ + last] = -1;
-            at_[o] = -1;
             --cnt_[v];
         }
     }
-    int get(int v, int id) const { return w_[(size_t) v * k_ + id]; }
+    int get(int v, int id) const { return row_[v] == epoch_ ? w_[(size_t) v * k_ + id] : 0; }
     void clear() {
         std::fill(cnt_.begin(), cnt_.end(), 0);
         std::fill(cnt2_.begin(), cnt2_.end(), 0);
-        std::fill(w_.begin(), w_.end(), 0);
-        std::fill(at_.begin(), at_.end(), -1);
-        std::fill(ids_.begin(), ids_.end(), -1);
+        ++epoch_;
         std::fill(in_.begin(), in_.end(), 0);
         std::fill(in2_.begin(), in2_.end(), 0);
         std::fill(ex_.begin(), ex_.end(), 0);
@@ -166,7 +213,8 @@ public:
 
 private:
     int n_, k_;
-    std::vector<int> cnt_, cnt2_, in_, in2_, ex_, ex2_, w_, at_, ids_;
+    int epoch_ = 1;  // rows of an older epoch are empty
+    IVec cnt_, cnt2_, in_, in2_, ex_, ex2_, row_, w_, at_, ids_;
 };
 
 // Binary max-heap of (key, vertex) with a position index (kway_prio_queue.h,
@@ -176,7 +224,13 @@ private:
 template<typename K>
 class MaxHeap {
 public:
-    explicit MaxHeap(size_t cap) : size_(0), h_(cap), at_(cap, -1) {}
+    MaxHeap(HeapStore<K> &store, size_t cap) : size_(0), h_(store.h), at_(store.at) {
+        if (h_.size() < cap) h_.resize(cap);
+        if (at_.size() < cap) at_.resize(cap, -1);
+    }
+    ~MaxHeap() { clear(); }
+    MaxHeap(const MaxHeap &) = delete;
+    MaxHeap &operator=(const MaxHeap &) = delete;
     bool empty() const { return size_ == 0; }
     bool contains(int v) const { return v >= 0 && (size_t) v < at_.size() && at_[v] != -1; }
     void clear() {
@@ -219,19 +273,15 @@ public:
     }
 
 private:
-    struct Item {
-        K key;
-        int v;
-    };
     size_t size_;
-    std::vector<Item> h_;
-    std::vector<long> at_;
+    std::vector<typename HeapStore<K>::Item> &h_;
+    std::vector<int> &at_;
     void up(long &i, const K &key) {
         while (i > 0) {
             const long p = (i - 1) >> 1;
             if (!(key > h_[p].key)) break;
             h_[i] = h_[p];
-            at_[h_[i].v] = i;
+            at_[h_[i].v] = (int) i;
             i = p;
         }
     }
@@ -248,20 +298,20 @@ private:
                 break;
             }
             h_[i] = h_[c];
-            at_[h_[i].v] = i;
+            at_[h_[i].v] = (int) i;
             i = c;
         }
     }
     void put(long i, int v, const K &key) {
         h_[i].key = key;
         h_[i].v = v;
-        at_[v] = i;
+        at_[v] = (int) i;
     }
 };
 
 // permute (kway_utility.h:58-75): nshuffles random 4-element block swaps, or
 // n random pair swaps for n < 10.
-void shuffle(int n, std::vector<int> &p, int nshuffles, LibcRand &R) {
+void shuffle(int n, IVec &p, int nshuffles, Rand &R) {
     if (n < 10) {
         for (int i = 0; i < n; ++i) {
             const int a = R.next() % n;
@@ -281,9 +331,9 @@ void shuffle(int n, std::vector<int> &p, int nshuffles, LibcRand &R) {
 }
 
 // counting_sort (kway_utility.h:77-92): stable by key in the order of tperm.
-void bucket_order(int n, int maxkey, const std::vector<int> &keys, const std::vector<int> &tperm,
-                  std::vector<int> &perm) {
-    std::vector<int> start(maxkey + 2, 0);
+void bucket_order(int n, int maxkey, const IVec &keys, const IVec &tperm,
+                  IVec &perm) {
+    IVec start(maxkey + 2, 0);
     for (int i = 0; i < n; ++i) ++start[keys[i]];
     for (int i = 1; i < maxkey + 1; ++i) start[i] += start[i - 1];
     for (int i = maxkey + 1; i > 0; --i) start[i] = start[i - 1];
@@ -296,16 +346,16 @@ void bucket_order(int n, int maxkey, const std::vector<int> &keys, const std::ve
 
 // Match_2HopAny (kway_core.h:285-327): unmatched vertices of degree < max_deg
 // that share a neighbour are paired, from the ends of each neighbour's list.
-int pair_two_hop_any(const KGraph &g, std::vector<int> &match, std::vector<int> &cmap, int cn, int &unmatched,
-                     int max_deg, const std::vector<int> &perm) {
-    std::vector<int> off(g.n + 1, 0);
+int pair_two_hop_any(const KGraph &g, IVec &match, IVec &cmap, int cn, int &unmatched,
+                     int max_deg, const IVec &perm) {
+    IVec off(g.n + 1, 0);
     for (int v = 0; v < g.n; ++v)
         if (match[v] == FREE && g.xadj[v + 1] - g.xadj[v] < max_deg)
             for (int j = g.xadj[v]; j < g.xadj[v + 1]; ++j) off[g.adj[j]]++;
     for (int i = 1; i < g.n; ++i) off[i] += off[i - 1];
     for (int i = g.n; i > 0; --i) off[i] = off[i - 1];
     off[0] = 0;
-    std::vector<int> lst(off[g.n]);
+    IVec lst(off[g.n]);
     for (int pi = 0; pi < g.n; ++pi) {
         const int i = perm[pi];
         if (match[i] == FREE && g.xadj[i + 1] - g.xadj[i] < max_deg)
@@ -345,8 +395,8 @@ int by_neighbourhood_key(const void *a, const void *b) {
 // Match_2HopAll (kway_core.h:329-387): unmatched vertices with identical
 // neighbourhoods are paired (candidates ordered by a neighbourhood checksum
 // with the C library's qsort, as the reference orders them).
-int pair_two_hop_all(const KGraph &g, std::vector<int> &match, std::vector<int> &cmap, int cn, int &unmatched,
-                     int max_deg, const std::vector<int> &perm) {
+int pair_two_hop_all(const KGraph &g, IVec &match, IVec &cmap, int cn, int &unmatched,
+                     int max_deg, const IVec &perm) {
     const int mask = INT32_MAX / max_deg;
     int nc = 0;
     std::vector<NeighbourhoodKey> keys(unmatched);
@@ -362,7 +412,7 @@ int pair_two_hop_all(const KGraph &g, std::vector<int> &match, std::vector<int> 
         }
     }
     std::qsort(keys.data(), nc, sizeof(NeighbourhoodKey), by_neighbourhood_key);
-    std::vector<int> mark(g.n, 0);
+    IVec mark(g.n, 0);
     for (int pi = 0; pi < nc; ++pi) {
         const int i = keys[pi].vertex;
         if (match[i] != FREE) continue;
@@ -389,8 +439,8 @@ int pair_two_hop_all(const KGraph &g, std::vector<int> &match, std::vector<int> 
 
 // Match_2Hop (kway_core.h:389-397). The unmatched count is passed by value,
 // as in the reference: the later passes see the count after the first two.
-int pair_two_hop(const KGraph &g, std::vector<int> &match, std::vector<int> &cmap, int cn, int unmatched,
-                 const std::vector<int> &perm) {
+int pair_two_hop(const KGraph &g, IVec &match, IVec &cmap, int cn, int unmatched,
+                 const IVec &perm) {
     cn = pair_two_hop_any(g, match, cmap, cn, unmatched, 2, perm);
     cn = pair_two_hop_all(g, match, cmap, cn, unmatched, 64, perm);
     if (unmatched > 1.5 * 0.10 * g.n) cn = pair_two_hop_any(g, match, cmap, cn, unmatched, 3, perm);
@@ -403,8 +453,8 @@ int pair_two_hop(const KGraph &g, std::vector<int> &match, std::vector<int> &cma
 // weight limit; isolated vertices pair with the next free vertex; two-hop
 // passes when more than 10% stay unmatched. Returns the coarse vertex count;
 // cmap holds coarse ids in vertex order.
-int heavy_edge_match(const KGraph &g, std::vector<int> &match, std::vector<int> &cmap, int max_vw, LibcRand &R) {
-    std::vector<int> perm(g.n), tperm(g.n), deg(g.n);
+int heavy_edge_match(const KGraph &g, IVec &match, IVec &cmap, int max_vw, Rand &R) {
+    IVec perm(g.n), tperm(g.n), deg(g.n);
     std::fill_n(match.data(), g.n, FREE);
     for (int i = 0; i < g.n; ++i) tperm[i] = i;
     shuffle(g.n, tperm, g.n / 8, R);
@@ -467,11 +517,11 @@ int heavy_edge_match(const KGraph &g, std::vector<int> &match, std::vector<int> 
 // first-occurrence order of the coarse neighbours; a small hash table for
 // short rows (the coarse vertex's own id is kept in slot 0 while aggregating
 // and replaced by the last entry at the end), a dense index otherwise.
-KGraph contract_pairs(const KGraph &g, const std::vector<int> &match, const std::vector<int> &cmap, int cn) {
+KGraph contract_pairs(const KGraph &g, const IVec &match, const IVec &cmap, int cn, Rand &R) {
     constexpr int mask = (1 << 13) - 1;
     KGraph c(cn, g.m + 1);
     c.cut = -1;
-    std::vector<int> slot(mask + 1, -1), dense(cn, -1);
+    std::vector<int> &slot = Rand::room(R.slot, mask + 1), &dense = Rand::room(R.dense, cn);
     int cv = 0, ce = 0;
     c.xadj[0] = 0;
     for (int v = 0; v < g.n; ++v) {
@@ -485,6 +535,7 @@ KGraph contract_pairs(const KGraph &g, const std::vector<int> &match, const std:
         if (dv + du < (mask >> 2)) {
             slot[cv & mask] = 0;
             c.adj[base] = cv;
+            c.ew[base] = 0;
             ne = 1;
             auto add_row = [&](int x) {
                 for (int j = g.xadj[x]; j < g.xadj[x + 1]; ++j) {
@@ -549,16 +600,17 @@ KGraph contract_pairs(const KGraph &g, const std::vector<int> &match, const std:
 }
 
 // balance_bisection_boundary (kway_core.h:136-219).
-void balance_from_boundary(KGraph &g, Side2 &s, BndSet &bnd, std::vector<int> &pw, const std::vector<float> &tw,
-                           std::vector<int> &side, LibcRand &R) {
-    std::vector<int> moved(g.n, -1), perm(g.n);
+void balance_from_boundary(KGraph &g, Side2 &s, BndSet &bnd, IVec &pw, const std::vector<float> &tw,
+                           IVec &side, Rand &R) {
+    IVec moved(g.n, -1), perm(g.n);
     int target[2];
     target[0] = (int) g.w * tw[0];
     target[1] = g.w - target[0];
     const int mindiff = std::abs(target[0] - pw[0]);
     const int from = pw[0] < target[0] ? 1 : 0;
     const int to = (from + 1) % 2;
-    MaxHeap<int> q(g.n);
+    HeapStore<int> qs;
+    MaxHeap<int> q(qs, g.n);
     for (int i = 0; i < bnd.cnt; ++i) perm[i] = i;
     shuffle(bnd.cnt, perm, bnd.cnt / 5, R);
     for (int i = 0; i < bnd.cnt; ++i) {
@@ -600,16 +652,17 @@ void balance_from_boundary(KGraph &g, Side2 &s, BndSet &bnd, std::vector<int> &p
 }
 
 // balance_bisection_general (kway_core.h:221-283).
-void balance_from_all(KGraph &g, Side2 &s, BndSet &bnd, std::vector<int> &pw, const std::vector<float> &tw,
-                      std::vector<int> &side, LibcRand &R) {
-    std::vector<int> moved(g.n, -1), perm(g.n);
+void balance_from_all(KGraph &g, Side2 &s, BndSet &bnd, IVec &pw, const std::vector<float> &tw,
+                      IVec &side, Rand &R) {
+    IVec moved(g.n, -1), perm(g.n);
     int target[2];
     target[0] = (int) g.w * tw[0];
     target[1] = g.w - target[0];
     const int mindiff = std::abs(target[0] - pw[0]);
     const int from = pw[0] < target[0] ? 1 : 0;
     const int to = (from + 1) % 2;
-    MaxHeap<int> q(g.n);
+    HeapStore<int> qs;
+    MaxHeap<int> q(qs, g.n);
     for (int i = 0; i < g.n; ++i) perm[i] = i;
     shuffle(g.n, perm, g.n / 5, R);
     for (int ii = 0; ii < g.n; ++ii) {
@@ -646,9 +699,14 @@ void balance_from_all(KGraph &g, Side2 &s, BndSet &bnd, std::vector<int> &pw, co
 // FM_2WayCutRefine (kway_core.h:597-741): max_iter passes of boundary FM with
 // one queue per side, moving from the heavier side, rolled back to the best
 // prefix of moves.
-void fm_two_way(KGraph &g, BndSet &bnd, Side2 &s, std::vector<int> &pw, const std::vector<float> &tw,
-                std::vector<int> &side, int max_iter, LibcRand &R) {
-    std::vector<int> moved(g.n, -1), swaps(g.n), perm(g.n);
+void fm_two_way(KGraph &g, BndSet &bnd, Side2 &s, IVec &pw, const std::vector<float> &tw,
+                IVec &side, int max_iter, Rand &R) {
+    std::vector<int> &moved = Rand::room(R.moved, g.n);
+    if ((int) R.swaps.size() < g.n) {
+        R.swaps.resize(g.n);
+        R.perm.resize(g.n);
+    }
+    IVec &swaps = R.swaps, &perm = R.perm;
     int target[2];
     target[0] = g.w * tw[0];
     target[1] = g.w - target[0];
@@ -656,7 +714,7 @@ void fm_two_way(KGraph &g, BndSet &bnd, Side2 &s, std::vector<int> &pw, const st
                                                                             : (100));
     const int avgvw = ((pw[0] + pw[1]) / 20) < (2 * (pw[0] + pw[1]) / g.n) ? ((pw[0] + pw[1]) / 20)
                                                                            : (2 * (pw[0] + pw[1]) / g.n);
-    MaxHeap<int> q0(g.n), q1(g.n);
+    MaxHeap<int> q0(R.q0, g.n), q1(R.q1, g.n);
     MaxHeap<int> *q[2] = {&q0, &q1};
     const int origdiff = std::abs(target[0] - pw[0]);
     for (int pass = 0; pass < max_iter; ++pass) {
@@ -740,8 +798,8 @@ void fm_two_way(KGraph &g, BndSet &bnd, Side2 &s, std::vector<int> &pw, const st
 
 // Project2WayPartition (kway_core.h:105-134): coarse sides to the fine
 // graph; vertices of non-boundary coarse vertices are interior.
-void project_two_way(const KGraph &g, Side2 &s, std::vector<int> &cmap, BndSet &bnd, const BndSet &cbnd,
-                     std::vector<int> &side, const std::vector<int> &cside) {
+void project_two_way(const KGraph &g, Side2 &s, IVec &cmap, BndSet &bnd, const BndSet &cbnd,
+                     IVec &side, const IVec &cside) {
     for (int i = 0; i < g.n; ++i) {
         const int j = cmap[i];
         side[i] = cside[j];
@@ -765,7 +823,7 @@ void project_two_way(const KGraph &g, Side2 &s, std::vector<int> &cmap, BndSet &
 }
 
 // ComputeLoadImbalanceDiff (kway_core.h:863-873).
-float imbalance_excess(const KGraph &g, int k, const std::vector<int> &pw, float ub) {
+float imbalance_excess(const KGraph &g, int k, const IVec &pw, float ub) {
     float mx = -1.0f;
     for (int j = 0; j < k; ++j) {
         const float cur = pw[j] * ((float) k / g.w) - ub;
@@ -775,7 +833,7 @@ float imbalance_excess(const KGraph &g, int k, const std::vector<int> &pw, float
 }
 
 // ComputeLoadImbalance (kway_core.h:852-861).
-float imbalance_of(const KGraph &g, int k, const std::vector<int> &pw) {
+float imbalance_of(const KGraph &g, int k, const IVec &pw) {
     float mx = 1.0;
     for (int j = 0; j < k; ++j) {
         const float cur = pw[j] * ((float) k / g.w);
@@ -785,7 +843,7 @@ float imbalance_of(const KGraph &g, int k, const std::vector<int> &pw) {
 }
 
 // ComputeLoadImbalanceDiffWeighted (kway_core.h:890-900).
-float imbalance_excess_2(const KGraph &g, const std::vector<int> &pw, const std::vector<float> &tw, float ub) {
+float imbalance_excess_2(const KGraph &g, const IVec &pw, const std::vector<float> &tw, float ub) {
     float mx = -1.0f;
     for (int i = 0; i < 2; ++i) {
         const float cur = pw[i] * (1.0f / (g.w * tw[i])) - ub;
@@ -795,8 +853,8 @@ float imbalance_excess_2(const KGraph &g, const std::vector<int> &pw, const std:
 }
 
 // balance_bisection (kway_core.h:875-884).
-void balance_two_way(KGraph &g, BndSet &bnd, Side2 &s, const std::vector<float> &tw, std::vector<int> &pw,
-                     std::vector<int> &side, float ub, LibcRand &R) {
+void balance_two_way(KGraph &g, BndSet &bnd, Side2 &s, const std::vector<float> &tw, IVec &pw,
+                     IVec &side, float ub, Rand &R) {
     if (imbalance_excess(g, 2, pw, ub) <= 0) return;
     if (fabsf(tw[0] * g.w - pw[0]) < 3 * g.w / g.n) return;
     if (bnd.cnt > 0) balance_from_boundary(g, s, bnd, pw, tw, side, R);
@@ -804,9 +862,9 @@ void balance_two_way(KGraph &g, BndSet &bnd, Side2 &s, const std::vector<float> 
 }
 
 // Compute2WayPartitionParams (kway_core.h:1064-1095).
-void two_way_params(KGraph &g, BndSet &bnd, std::vector<int> &pw, const std::vector<int> &side, Side2 &s) {
+void two_way_params(KGraph &g, BndSet &bnd, IVec &pw, const IVec &side, Side2 &s) {
     std::fill_n(pw.data(), 2, 0);
-    bnd.clear();
+    bnd.clear(g.n);
     int cut = 0;
     for (int i = 0; i < g.n; ++i) pw[side[i]] += g.vw[i];
     for (int i = 0; i < g.n; ++i) {
@@ -829,9 +887,9 @@ void two_way_params(KGraph &g, BndSet &bnd, std::vector<int> &pw, const std::vec
 // bisection (kway_core.h:1097-1185): max_tries graph-growing bisections from
 // random seeds (breadth-first until side 1 falls to its bound), each balanced
 // and refined by FM; the best cut is kept.
-void grow_bisection(KGraph &g, BndSet &bnd, float ub, const std::vector<float> &tw, std::vector<int> &pw,
-                    std::vector<int> &side, Side2 &s, int max_tries, int max_iter, LibcRand &R) {
-    std::vector<int> trial(g.n), fifo(g.n), seen(g.n);
+void grow_bisection(KGraph &g, BndSet &bnd, float ub, const std::vector<float> &tw, IVec &pw,
+                    IVec &side, Side2 &s, int max_tries, int max_iter, Rand &R) {
+    IVec trial(g.n), fifo(g.n), seen(g.n);
     const int maxw = ub * g.w * tw[1];
     const int minw = (1.0 / ub) * g.w * tw[1];
     int bestcut = 0;
@@ -897,10 +955,10 @@ void grow_bisection(KGraph &g, BndSet &bnd, float ub, const std::vector<float> &
 // split_graph (kway_core.h:1187-1265): the two sides as graphs of their own
 // (vertices in order; rows of interior vertices copied, boundary rows
 // filtered), with the original labels carried along.
-void split_two(const KGraph &g, const BndSet &bnd, const std::vector<int> &label, const std::vector<int> &side,
-               KGraph &lg, std::vector<int> &llab, KGraph &rg, std::vector<int> &rlab) {
+void split_two(const KGraph &g, const BndSet &bnd, const IVec &label, const IVec &side,
+               KGraph &lg, IVec &llab, KGraph &rg, IVec &rlab) {
     int ns[2] = {0, 0}, ms[2] = {0, 0}, ws[2] = {0, 0};
-    std::vector<int> rename(g.n);
+    IVec rename(g.n);
     for (int i = 0; i < g.n; ++i) {
         const int p = side[i];
         rename[i] = ns[p]++;
@@ -951,50 +1009,51 @@ void split_two(const KGraph &g, const BndSet &bnd, const std::vector<int> &label
 // multilevel_bisection (kway_core.h:1267-1361). `side` and `spare` (and
 // `bnd` and `bnd2`) are exchanged level by level as in the reference; the
 // result ends in `side`.
-void multilevel_two_way(KGraph &g, BndSet &bnd, std::vector<int> &side, const std::vector<float> &tw, int max_tries,
-                        int threshold, float ub, int max_iter, BndSet &bnd2, std::vector<int> &spare, LibcRand &R) {
+void multilevel_two_way(KGraph &g, BndSet &bnd, IVec &side, const std::vector<float> &tw, int max_tries,
+                        int threshold, float ub, int max_iter, BndSet &bnd2, IVec &spare, Rand &R) {
     int bestobj = 0, curobj = 0;
     float bestbal = 0.0, curbal = 0.0;
     if (g.n == 0) return;
-    std::vector<int> pw(2);
+    IVec pw(2);
     Side2 s(g.n);
-    std::vector<int> match(g.n);
+    IVec match(g.n);
     int *const side_orig = side.data();
-    std::vector<int> best;
+    IVec best;
     if (max_tries > 1) best.resize(g.n);
     for (int t = 0; t < max_tries; ++t) {
-        std::vector<KGraph> levels;
-        std::vector<std::vector<int> > cmaps;
-        levels.push_back(g);
-        const int maxvw = 1.5 * levels.back().w / threshold;
-        do {
-            KGraph &fine = levels.back();
+        std::vector<KGraph> coarser;  // level l > 0; level 0 is g itself
+        std::vector<IVec> cmaps;
+        auto level_of = [&](size_t l) -> KGraph & { return l == 0 ? g : coarser[l - 1]; };
+        const int maxvw = 1.5 * g.w / threshold;
+        for (;;) {
+            KGraph &fine = level_of(coarser.size());
             cmaps.emplace_back(fine.n);
-            std::vector<int> &cm = cmaps.back();
+            IVec &cm = cmaps.back();
             const int cn = heavy_edge_match(fine, match, cm, maxvw, R);
-            KGraph coarse = contract_pairs(fine, match, cm, cn);
-            levels.push_back(std::move(coarse));
-        } while (levels.back().n > threshold && levels.back().n < 0.85 * levels[levels.size() - 2].n &&
-                 levels.back().m > levels.back().n / 2);
-        const int nlevels = (int) levels.size() - 1;
+            const int fine_n = fine.n;
+            KGraph coarse = contract_pairs(fine, match, cm, cn, R);
+            coarser.push_back(std::move(coarse));
+            const KGraph &last = coarser.back();
+            if (!(last.n > threshold && last.n < 0.85 * fine_n && last.m > last.n / 2)) break;
+        }
+        const int nlevels = (int) coarser.size();
         bnd.cnt = 0;
-        grow_bisection(levels.back(), bnd, ub, tw, pw, side, s, 2, max_iter, R);
-        two_way_params(levels.back(), bnd, pw, side, s);
+        grow_bisection(coarser.back(), bnd, ub, tw, pw, side, s, 2, max_iter, R);
+        two_way_params(coarser.back(), bnd, pw, side, s);
         for (int level = nlevels; level > 0; --level) {
-            KGraph &coarse = levels[level];
-            std::vector<int> &cm = cmaps[level - 1];
+            KGraph &coarse = level_of(level);
+            IVec &cm = cmaps[level - 1];
             balance_two_way(coarse, bnd, s, tw, pw, side, ub, R);
             fm_two_way(coarse, bnd, s, pw, tw, side, max_iter, R);
-            KGraph &fine = levels[level - 1];
-            bnd2.clear();
+            KGraph &fine = level_of(level - 1);
+            bnd2.clear(fine.n);
             project_two_way(fine, s, cm, bnd2, bnd, spare, side);
             fine.cut = coarse.cut;
             std::swap(bnd, bnd2);
             std::swap(side, spare);
         }
-        balance_two_way(levels[0], bnd, s, tw, pw, side, ub, R);
-        fm_two_way(levels[0], bnd, s, pw, tw, side, max_iter, R);
-        g.cut = levels[0].cut;
+        balance_two_way(g, bnd, s, tw, pw, side, ub, R);
+        fm_two_way(g, bnd, s, pw, tw, side, max_iter, R);
         curobj = g.cut;
         curbal = imbalance_excess_2(g, pw, tw, ub);
         if (t == 0 || (curbal <= 0.0005 && bestobj > curobj) || (bestbal > 0.0005 && curbal < bestbal)) {
@@ -1014,16 +1073,16 @@ void multilevel_two_way(KGraph &g, BndSet &bnd, std::vector<int> &side, const st
 // recursive_bisection (kway_core.h:1363-1390): bisect with target weights
 // from tw, write the blocks of this level, split and recurse on both halves
 // with renormalised targets.
-void recursive_two_way(KGraph &g, BndSet &bnd, int k, const std::vector<int> &label, std::vector<int> &part,
+void recursive_two_way(KGraph &g, BndSet &bnd, int k, const IVec &label, IVec &part,
                        float *tw, int first, int max_tries, int threshold, float ub, int max_iter, BndSet &bnd2,
-                       std::vector<int> &side, std::vector<int> &spare, LibcRand &R) {
+                       IVec &side, IVec &spare, Rand &R) {
     std::vector<float> tw2(2);
     tw2[0] = std::accumulate(tw, tw + (k >> 1), 0.0f);
     tw2[1] = 1.0 - tw2[0];
     multilevel_two_way(g, bnd, side, tw2, max_tries, threshold, ub, max_iter, bnd2, spare, R);
     for (int i = 0; i < g.n; ++i) part[label[i]] = side[i] + first;
     KGraph lg, rg;
-    std::vector<int> llab, rlab;
+    IVec llab, rlab;
     if (k > 2) split_two(g, bnd, label, side, lg, llab, rg, rlab);
     const float wsum = std::accumulate(tw, tw + (k >> 1), 0.0f);
     std::transform(tw, tw + (k >> 1), tw, [wsum](float x) { return x / wsum; });
@@ -1041,23 +1100,23 @@ void recursive_two_way(KGraph &g, BndSet &bnd, int k, const std::vector<int> &la
 
 // recursive_bisection_head (kway_core.h:1392-1414): restarts the random
 // sequence at 4321, as the reference does.
-void recursive_kway(KGraph &g, int k, float ub, int max_tries, std::vector<int> &part, LibcRand &R) {
+void recursive_kway(KGraph &g, int k, float ub, int max_tries, IVec &part, Rand &R) {
     std::fill_n(part.data(), g.n, 0);
     if (k == 1) return;
     R.seed_with(4321);
     ub += 0.0000499f;
     std::vector<float> tw(k, 1.0f / k);
-    std::vector<int> label(g.n);
+    IVec label(g.n);
     for (int i = 0; i < g.n; ++i) label[i] = i;
     BndSet bnd(g.n), bnd2(g.n);
-    std::vector<int> side(g.n), spare(g.n);
+    IVec side(g.n), spare(g.n);
     recursive_two_way(g, bnd, k, label, part, tw.data(), 0, max_tries, 50, ub, 3, bnd2, side, spare, R);
 }
 
 // ComputeKWayPartitionParams (kway_core.h:743-784).
-void kway_params(KGraph &g, BndSet &bnd, int k, std::vector<int> &pw, const std::vector<int> &part, KConn &C) {
+void kway_params(KGraph &g, BndSet &bnd, int k, IVec &pw, const IVec &part, KConn &C) {
     std::fill_n(pw.data(), k, 0);
-    bnd.clear();
+    bnd.clear(g.n);
     C.clear();
     int cut = 0;
     for (int u = 0; u < g.n; ++u) pw[part[u]] += g.vw[u];
@@ -1082,8 +1141,8 @@ void kway_params(KGraph &g, BndSet &bnd, int k, std::vector<int> &pw, const std:
 // ProjectKWayPartition (kway_core.h:786-840): projects the coarse blocks and
 // rebuilds the connectivity of fine vertices whose coarse vertex had external
 // weight (the others are interior).
-void project_kway(KGraph &g, BndSet &bnd, std::vector<int> &cmap, std::vector<int> &part, KGraph &coarse,
-                  const std::vector<int> &cpart, KConn &C) {
+void project_kway(KGraph &g, BndSet &bnd, IVec &cmap, IVec &part, KGraph &coarse,
+                  const IVec &cpart, KConn &C) {
     for (int u = 0; u < g.n; ++u) {
         const int v = cmap[u];
         part[u] = cpart[v];
@@ -1092,7 +1151,7 @@ void project_kway(KGraph &g, BndSet &bnd, std::vector<int> &cmap, std::vector<in
     C.clear();
     const int coarse_cut = coarse.cut;
     coarse.reshape(0, 0);
-    bnd.clear();
+    bnd.clear(g.n);
     for (int i = 0; i < g.n; ++i) {
         const int a = g.xadj[i], b = g.xadj[i + 1];
         if (cmap[i] == 0) {
@@ -1121,13 +1180,13 @@ void project_kway(KGraph &g, BndSet &bnd, std::vector<int> &cmap, std::vector<in
 
 // compute_boundary (kway_core.h:842-850).
 void kway_boundary(const KGraph &g, BndSet &bnd, int type, const KConn &C) {
-    bnd.clear();
+    bnd.clear(g.n);
     for (int u = 0; u < g.n; ++u)
         if (C.ex(u) > 0 && (type != BND_REFINE || C.ex(u) >= C.in(u))) bnd.add(u);
 }
 
 // is_balanced (kway_core.h:886-888).
-bool balanced(const KGraph &g, int k, const std::vector<int> &pw, float ub, float slack) {
+bool balanced(const KGraph &g, int k, const IVec &pw, float ub, float slack) {
     return imbalance_excess(g, k, pw, ub) <= slack;
 }
 
@@ -1155,7 +1214,7 @@ void neighbour_moved(int v, int v_id, int from, int to, int w, KConn &C, BndSet 
 }
 
 // UpdateMovedVertexInfoAndBND (kway_core.h:81-103).
-void vertex_moved(int u, int from, int to, KConn &C, BndSet &bnd, std::vector<int> &part, int type) {
+void vertex_moved(int u, int from, int to, KConn &C, BndSet &bnd, IVec &part, int type) {
     part[u] = to;
     const int w_to = C.get(u, to);
     C.add_ex(u, C.in(u) - w_to);
@@ -1178,8 +1237,8 @@ inline float rgain_of(const KConn &C, int u) {
 
 // Greedy_KWayCutOptimize (kway_core.h:902-1062): greedy k-way refinement (or
 // balancing) over the boundary, vertices taken by a float priority.
-void greedy_kway(KGraph &g, BndSet &bnd, int k, float ub, std::vector<int> &pw, std::vector<int> &part, int max_iter,
-                 int mode, KConn &C, LibcRand &R) {
+void greedy_kway(KGraph &g, BndSet &bnd, int k, float ub, IVec &pw, IVec &part, int max_iter,
+                 int mode, KConn &C, Rand &R) {
     const int type = mode == OPT_REFINE ? BND_REFINE : BND_BALANCE;
     if (mode != OPT_BALANCE) {
         const float cur = imbalance_of(g, k, pw);
@@ -1187,8 +1246,9 @@ void greedy_kway(KGraph &g, BndSet &bnd, int k, float ub, std::vector<int> &pw, 
     }
     const int maxpw = (1.0f / k) * g.w * ub;
     const int minpw = (1.0f / k) * g.w * (1.0f / ub);
-    std::vector<int> perm(g.n), moved(g.n, -1);
-    MaxHeap<float> q(g.n);
+    IVec perm(g.n), moved(g.n, -1);
+    HeapStore<float> qs;
+    MaxHeap<float> q(qs, g.n);
     for (int pass = 0; pass < max_iter; ++pass) {
         if (mode == OPT_BALANCE) {
             bool stop = true;
@@ -1272,37 +1332,39 @@ void greedy_kway(KGraph &g, BndSet &bnd, int k, float ub, std::vector<int> &pw, 
 // multilevel_partition (kway_core.h:1416-1525): coarsen to `threshold`
 // vertices, recursive bisection of the coarsest graph, greedy k-way
 // balancing and refinement on every level while projecting back.
-int multilevel_kway(KGraph &g, int k, float ub, std::vector<int> &part, int threshold, int n_init, int max_tries,
-                    int max_iter, LibcRand &R) {
+int multilevel_kway(KGraph &g, int k, float ub, IVec &part, int threshold, int n_init, int max_tries,
+                    int max_iter, Rand &R) {
     int curobj = 0, bestobj = 0;
     float curbal = 0.0f, bestbal = 0.0f;
     BndSet bnd(g.n);
-    std::vector<int> pw(k), where1(g.n), where2(g.n), match(g.n);
-    std::vector<KGraph> levels;
-    std::vector<std::vector<int> > cmaps;
+    IVec pw(k), where1(g.n), where2(g.n), match(g.n);
+    std::vector<KGraph> coarser;  // level l > 0; level 0 is g itself
+    std::vector<IVec> cmaps;
     KConn C(g.n, k);
+    auto level_of = [&](size_t l) -> KGraph & { return l == 0 ? g : coarser[l - 1]; };
     for (int t = 0; t < max_tries; ++t) {
-        levels.clear();
+        coarser.clear();
         cmaps.clear();
-        levels.push_back(g);
-        const int maxvw = 1.5 * levels.back().w / threshold;
-        do {
-            KGraph &fine = levels.back();
+        const int maxvw = 1.5 * g.w / threshold;
+        for (;;) {
+            KGraph &fine = level_of(coarser.size());
             cmaps.emplace_back(fine.n);
-            std::vector<int> &cm = cmaps.back();
+            IVec &cm = cmaps.back();
             const int cn = heavy_edge_match(fine, match, cm, maxvw, R);
-            KGraph coarse = contract_pairs(fine, match, cm, cn);
-            levels.push_back(std::move(coarse));
-        } while (levels.back().n > threshold && levels.back().n < 0.85 * levels[levels.size() - 2].n &&
-                 levels.back().m > levels.back().n / 2);
+            const int fine_n = fine.n;
+            KGraph coarse = contract_pairs(fine, match, cm, cn, R);
+            coarser.push_back(std::move(coarse));
+            const KGraph &last = coarser.back();
+            if (!(last.n > threshold && last.n < 0.85 * fine_n && last.m > last.n / 2)) break;
+        }
         const float ub_level = (float) std::pow(ub, 1.0 / std::log(k));
-        recursive_kway(levels.back(), k, ub_level, n_init, where1, R);
+        recursive_kway(coarser.back(), k, ub_level, n_init, where1, R);
         const int nlevels = (int) cmaps.size();
         bnd.cnt = 0;
-        kway_params(levels.back(), bnd, k, pw, where1, C);
+        kway_params(coarser.back(), bnd, k, pw, where1, C);
         int cl = nlevels;
         for (int pass = 0; cl >= 0; ++pass) {
-            KGraph &cg = levels[cl];
+            KGraph &cg = level_of(cl);
             if (2 * pass >= nlevels && !balanced(cg, k, pw, ub, .02f)) {
                 kway_boundary(cg, bnd, BND_BALANCE, C);
                 greedy_kway(cg, bnd, k, ub, pw, where1, 1, OPT_BALANCE, C, R);
@@ -1310,21 +1372,19 @@ int multilevel_kway(KGraph &g, int k, float ub, std::vector<int> &part, int thre
             }
             greedy_kway(cg, bnd, k, ub, pw, where1, max_iter, OPT_REFINE, C, R);
             if (cl > 0) {
-                KGraph &fine = levels[cl - 1];
+                KGraph &fine = level_of(cl - 1);
                 C.swap_copies();
                 project_kway(fine, bnd, cmaps[cl - 1], where2, cg, where1, C);
                 std::swap(where1, where2);
             }
             --cl;
         }
-        g.cut = levels[0].cut;
-        if (!balanced(levels[0], k, pw, ub, 0.0f)) {
-            kway_boundary(levels[0], bnd, BND_BALANCE, C);
-            greedy_kway(levels[0], bnd, k, ub, pw, where1, 3, OPT_BALANCE, C, R);
-            kway_boundary(levels[0], bnd, BND_REFINE, C);
-            greedy_kway(levels[0], bnd, k, ub, pw, where1, max_iter, OPT_REFINE, C, R);
+        if (!balanced(g, k, pw, ub, 0.0f)) {
+            kway_boundary(g, bnd, BND_BALANCE, C);
+            greedy_kway(g, bnd, k, ub, pw, where1, 3, OPT_BALANCE, C, R);
+            kway_boundary(g, bnd, BND_REFINE, C);
+            greedy_kway(g, bnd, k, ub, pw, where1, max_iter, OPT_REFINE, C, R);
         }
-        g.cut = levels[0].cut;
         curobj = g.cut;
         curbal = imbalance_excess(g, k, pw, ub);
         if (t == 0 || (curbal <= 0.0005f && bestobj > curobj) || (bestbal > 0.0005f && curbal < bestbal)) {
@@ -1357,10 +1417,10 @@ void metis_kway(u32 n, const u32 *xadj, const u32 *adj, const s32 *vw, const s32
     const int uf = static_cast<int>(imbalance * 1000.0f);
     float ub = 1.0f + 0.001f * uf;
     ub += 0.0000499f;
-    LibcRand R((u32) seed);
+    Rand R((u32) seed);
     const int candidate = static_cast<int>((double) g.n / (40.0 * log2(k)));
     const int threshold = (candidate > 30 * k) ? candidate : 30 * k;
-    std::vector<int> out(n, 0);
+    IVec out(n, 0);
     multilevel_kway(g, k, ub, out, threshold, 1, 1, 3, R);
     for (u32 u = 0; u < n; ++u) part[u] = (u32) out[u];
 }
