@@ -37,8 +37,12 @@ DGraph graph_upload(Ctx &ctx, u32 n, u64 m, const u32 *xadj, const u32 *adj, con
 DGraph graph_from_device(Ctx &ctx, u32 n, u64 m, const u32 *d_xadj, const u32 *d_adj, const s32 *d_ew,
                          const s32 *d_vw, bool validate);
 
-// Writes a compact CSR copy of g to host arrays (xadj n+1, adj m, ew m, vw n).
-void graph_download(Ctx &ctx, const DGraph &g, u32 *xadj, u32 *adj, s32 *ew, s32 *vw);
+// Writes a compact CSR copy of g to host arrays (xadj n+1, adj m, ew m, vw n);
+// sorted: rows in ascending neighbour id, for graphs without parallel edges of
+// up to SORTED_ROWS_MAX_N vertices (graph_sorts_rows; 44 KB of shared memory).
+constexpr u32 SORTED_ROWS_MAX_N = 44 * 1024 / 8 * 32;
+bool graph_sorts_rows(const DGraph &g);
+void graph_download(Ctx &ctx, const DGraph &g, u32 *xadj, u32 *adj, s32 *ew, s32 *vw, bool sorted = false);
 
 // All subgraphs induced by parts 0..k-1 of `part`, in one pass over g
 // (hierarchical_multisection.h:104-206 induces them one part at a time):

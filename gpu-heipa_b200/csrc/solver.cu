@@ -29,8 +29,10 @@ __global__ void k_scatter_leaf(const u32 *tmp, const u32 *n_to_o, u32 n, u32 off
         global_part[n_to_o[u]] = offset + tmp[u];
 }
 
-// Downloads the coarsest graph with rows in canonical (sorted) order.
-HostCSR download_sorted(Ctx &ctx, const DGraph &g) {
+// Downloads the coarsest graph with rows in canonical (sorted) order, sorted on
+// the device when it is a contracted graph (an input graph may have parallel
+// edges).
+HostCSR download_sorted(Ctx &ctx, const DGraph &g, bool contracted) {
     HostCSR h;
     h.n = g.n;
     h.m = (u32) g.m;
@@ -38,8 +40,9 @@ HostCSR download_sorted(Ctx &ctx, const DGraph &g) {
     h.adj.resize(g.m);
     h.ew.resize(g.m);
     h.vw.resize(g.n);
-    graph_download(ctx, g, h.xadj.data(), h.adj.data(), h.ew.data(), h.vw.data());
-    sort_rows(h);
+    const bool on_device = contracted && graph_sorts_rows(g);
+    graph_download(ctx, g, h.xadj.data(), h.adj.data(), h.ew.data(), h.vw.data(), on_device);
+    if (!on_device) sort_rows(h);
     return h;
 }
 
@@ -202,7 +205,7 @@ s64 solve_partition(Ctx &ctx, const DGraph &g, u32 k, double eps, bool ultra, u6
     // initial partitioning on the host (kway_core.h:1573-1588)
     auto t0 = Clock::now();
     ProfScope prof_ip(ctx, "initial_partitioning");
-    HostCSR hc = download_sorted(ctx, coarsest);
+    HostCSR hc = download_sorted(ctx, coarsest, !H.maps.empty());
     std::vector<u32> hpart;
     initial_kway(hc, k, eps, seed, hpart);
     u32 *cpart = ctx.falloc<u32>(coarsest.n);
@@ -381,7 +384,7 @@ s64 solve_mapping(Ctx &ctx, const DGraph &g, const std::vector<u32> &hier, const
         coarsen(ctx, g, k, H, stats);
         const DGraph &coarsest = H.graphs.back();
         auto t0 = Clock::now();
-        HostCSR hc = download_sorted(ctx, coarsest);
+        HostCSR hc = download_sorted(ctx, coarsest, !H.maps.empty());
         std::vector<u32> hpart;
         global_multisection(hc, hier, eps, seed, hpart);
         u32 *cpart = ctx.falloc<u32>(coarsest.n);
