@@ -19,9 +19,10 @@ DGraph contract_graph(Ctx &ctx, const DGraph &g, const u32 *mapping, u32 n_c);
 
 // One coarsening level in one launch (coarsen_team.cu). `mapping` receives
 // the fine->coarse map. With `rows` (adj and ew allocated with room for g.m
-// entries), the coarse rows are written there and rowptr (n + 1), rowlen and vw
-// point to scratch with the coarse graph's row bounds and vertex weights; they
-// are valid until the caller releases the scratch. contracted is false when a
+// entries), the coarse rows are written there, and the coarse graph's row
+// bounds and vertex weights to its rowptr (room for n + 1), rowlen and vw, or,
+// where those are null, to scratch that is valid until the caller releases it
+// (the result's rowptr, rowlen and vw). contracted is false when a
 // coarse row is too long for the kernel's tables (contract_graph then builds
 // the graph). Throws CoopSpin when the launch cannot be made or gave up.
 struct CoarsenResult {

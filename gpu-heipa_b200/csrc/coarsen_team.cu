@@ -57,12 +57,6 @@ struct CoarsenOut {
     unsigned long long contract_ns;  // time from the coarse ids on
 };
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
 struct CoarsenArgs {
     u32 n;
     const u32 *rowptr, *rowlen, *adj;
@@ -941,9 +935,9 @@ CoarsenResult coarsen_team(Ctx &ctx, const DGraph &g, u32 *mapping, DGraph *rows
     CoarsenResult r;
     if (rows) {
         // sized for n until the coarse size is known
-        a.c_rowptr = r.rowptr = ctx.balloc<u32>((size_t) n + 1);
-        a.c_rowlen = r.rowlen = ctx.balloc<u32>(n);
-        a.c_vw = r.vw = ctx.balloc<s32>(n);
+        a.c_rowptr = r.rowptr = rows->rowptr ? rows->rowptr : ctx.balloc<u32>((size_t) n + 1);
+        a.c_rowlen = r.rowlen = rows->rowlen ? rows->rowlen : ctx.balloc<u32>(n);
+        a.c_vw = r.vw = rows->vw ? rows->vw : ctx.balloc<s32>(n);
         a.c_adj = rows->adj;
         a.c_ew = rows->ew;
     }

@@ -6,6 +6,7 @@
 #include "stage.cuh"
 #include "team.cuh"
 
+#include <chrono>
 #include <mutex>
 #include <optional>
 #include <vector>
@@ -2778,7 +2779,7 @@ static size_t team_level_offset(u32 k, bool promap) { return team_smem(k, TEAM_B
 // evictions to rank); part is then to be restored from saved.
 static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const std::vector<u32> &ratios,
                             const DistOracle *D, unsigned long long inval_all_min, u32 *part, u32 *saved, s64 &obj,
-                            s32 &maxw, int team, u32 blocks) {
+                            s32 &maxw, int team, u32 blocks, const Projection &proj) {
     const u32 n = g.n;
     const bool promap = D != nullptr;
     TeamArgs a{};
@@ -2798,6 +2799,8 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
     a.bitdist = promap ? D->bitdist : nullptr;
     a.inval_all_min = inval_all_min;
     a.part = part;
+    a.cpart = proj.coarse;
+    a.cmap = proj.map;
     TeamCtl ctl{};
     ctl.n_ratios = (u32) ratios.size();
     for (size_t i = 0; i < ratios.size() && i < 17; ++i) ctl.ratios[i] = ratios[i];
@@ -2864,6 +2867,7 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
     if (o.err) throw HpError{HP_ERR_DEVICE, "Jet kernel reported error bits " + std::to_string(o.err)};
     obj = o.obj;
     maxw = o.maxw;
+    if (proj.ms) *proj.ms += (double) o.setup_ns * 1e-6;
 }
 
 // Blocks of the cooperative level loop for a level of n vertices and m
@@ -2876,9 +2880,31 @@ static u32 coop_blocks(const Ctx &ctx, u32 n, u64 m, u32 k, bool promap) {
                             (std::max<u64>(n, m / 16) + rows - 1) / rows);
 }
 
+__global__ void k_project(const u32 *coarse_part, const u32 *map, u32 *fine_part, u32 n) {
+    for (u32 u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x)
+        fine_part[u] = coarse_part[map[u]];
+}
+
+// The single-launch level loops project while they set up; the other paths
+// start from projected labels.
+static void project(Ctx &ctx, const Projection &proj, u32 *part, u32 n) {
+    if (!proj.map) return;
+    const auto t0 = std::chrono::steady_clock::now();
+    k_project<<<ctx.grid(n, BLOCK), BLOCK, 0, ctx.stream>>>(proj.coarse, proj.map, part, n); note_launch();
+    HP_LAUNCH_CHECK();
+    if (proj.ms) {
+        ctx.sync();
+        *proj.ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    }
+}
+
 void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultra, u32 level, s64 &obj, s32 &maxw,
-                const DistOracle *D) {
-    if (g.n == 0 || k <= 1) return;
+                const DistOracle *D, const Projection &proj) {
+    if (g.n == 0) return;
+    if (k <= 1) {
+        project(ctx, proj, part, g.n);
+        return;
+    }
     ScratchScope ss(ctx.arena);
     const bool promap = D != nullptr;
     // one filter ratio per level (or none for the mapping objective): a
@@ -2912,16 +2938,18 @@ void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultr
             u32 *saved = ctx.balloc<u32>(g.n);
             const unsigned long long inval = cache_pure ? (g.m * ctx.tune.jet_inval_all_pct + 99) / 100 : ~0ull;
             try {
-                jet_refine_team(ctx, g, k, lmax, ratios, D, inval, part, saved, obj, maxw, team, blocks);
+                jet_refine_team(ctx, g, k, lmax, ratios, D, inval, part, saved, obj, maxw, team, blocks, proj);
                 return;
             } catch (const CoopSpin &) {
                 // (a block team ranks all it has) the per-kernel loop redoes
                 // the level from its input labels
-                HP_CUDA(cudaMemcpyAsync(part, saved, sizeof(u32) * g.n, cudaMemcpyDeviceToDevice, ctx.stream));
+                if (!proj.map)
+                    HP_CUDA(cudaMemcpyAsync(part, saved, sizeof(u32) * g.n, cudaMemcpyDeviceToDevice, ctx.stream));
                 ctx.sync();  // saved is released here
             }
         }
     }
+    project(ctx, proj, part, g.n);
     JetLevel L;
     L.setup(ctx, g, k, lmax, D, part);
     L.cache_pure = cache_pure;

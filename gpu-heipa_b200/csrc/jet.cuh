@@ -150,7 +150,14 @@ constexpr int MAX_BW = 0;
 // (promap_jet_label_propagation.h:1218-1311). `part` (device, g.n) holds the
 // input labelling and receives the best labelling found; obj / maxw are the
 // running objective (edge cut or J) and maximum block weight.
+// With a projection, the input labels are coarse[map[u]] and part is output
+// only.
+struct Projection {
+    const u32 *coarse = nullptr;  // labels of the coarse graph
+    const u32 *map = nullptr;     // fine -> coarse
+    double *ms = nullptr;         // its time is added here (part of the whole call's)
+};
 void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultra, u32 level, s64 &obj, s32 &maxw,
-                const DistOracle *D);
+                const DistOracle *D, const Projection &proj = {});
 
 } // namespace hp

@@ -75,6 +75,7 @@ struct TeamOut {
     u32 gave_up;     // 1: more than TEAM_RANK_MAX evicted vertices in one step, nothing was decided
     u32 err;         // DevErr bits
     u32 hubs;        // some row is longer than TEAM_HUB
+    unsigned long long setup_ns;  // time of the set-up (projection, block weights) on block 0
 };
 
 struct TeamArgs {
@@ -91,7 +92,8 @@ struct TeamArgs {
     const u32 *code;
     const s32 *bitdist;
     unsigned long long inval_all_min;
-    u32 *part;                  // in: labels; out: best labelling
+    u32 *part;                  // in: labels (unless projected); out: best labelling
+    const u32 *cpart, *cmap;    // projection: labels of the coarse vertices, fine -> coarse map (or null)
     u32 *saved;                 // receives a copy of the input labels (or null)
     unsigned long long *tw;     // vertex words
     unsigned long long *abrec;  // afterburner records: gain, target (16 bits), label (16 bits)
@@ -539,9 +541,14 @@ __device__ __forceinline__ long long team_delta(const TeamArgs &a, const TeamSm 
             }
         }
         if (inval) {
+            // only where a target is cached: most neighbours have been reset
+            // already, and a cached read is cheaper than a scattered store
+            u32 x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = v[j] != SENTINEL ? a.dest_cache[v[j]] : NULL_PART;
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (v[j] != SENTINEL) a.dest_cache[v[j]] = NULL_PART;
+                if (x[j] != NULL_PART) a.dest_cache[v[j]] = NULL_PART;
         }
     }
     return acc;
@@ -637,8 +644,11 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
     u32 *const cl = small ? S.own : a.clist + r0;
     u32 *const ml = small ? S.own + TEAM_OWN : a.mlist + r0;
     bool hub = false;
+    const unsigned long long t0 = global_ns();
     for (u32 u = r0 + lane; u < r1; u += 32) {
-        const u32 o = a.part[u];
+        u32 o;
+        if (a.cmap) a.part[u] = o = __ldg(&a.cpart[__ldg(&a.cmap[u])]);
+        else o = a.part[u];
         if (a.saved) a.saved[u] = o;
         a.tw[u] = o;
         a.dest_cache[u] = NULL_PART;
@@ -653,6 +663,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
     team_flush_bw(a, S);
     if (tid == 0) c_cnt = m_cnt = 0;
     TEAM_SYNC();
+    if (blockIdx.x == 0 && tid == 0) a.out->setup_ns = global_ns() - t0;
     const bool hubs = ld_fresh<TEAM>(&a.out->hubs) != 0;
     team_load_bw<TEAM>(a, S, smx);
     long long obj = ctl.obj, best_obj = obj;
@@ -1484,5 +1495,6 @@ __global__ void __launch_bounds__(512, 1) k_jet_block(const __grid_constant__ Te
         ga.out->maxw = out->maxw;
         ga.out->iterations = out->iterations;
         ga.out->gave_up = out->gave_up;
+        ga.out->setup_ns = out->setup_ns;
     }
 }

@@ -19,11 +19,6 @@ double ms_since(Clock::time_point t) {
     return std::chrono::duration<double, std::milli>(Clock::now() - t).count();
 }
 
-__global__ void k_project(const u32 *coarse_part, const u32 *map, u32 *fine_part, u32 n) {
-    for (u32 u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x)
-        fine_part[u] = coarse_part[map[u]];
-}
-
 __global__ void k_scatter_leaf(const u32 *tmp, const u32 *n_to_o, u32 n, u32 offset, u32 *global_part) {
     for (u32 u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x)
         global_part[n_to_o[u]] = offset + tmp[u];
@@ -51,6 +46,8 @@ struct Hierarchy {
     std::vector<u32 *> maps;
 };
 
+constexpr u32 COARSEN_DIRECT_MAX_N = 1u << 16;
+
 enum class CoarsenStep { None, Matched, Contracted };
 
 // One level by the single-launch kernel, where it applies: the mapping and
@@ -68,13 +65,25 @@ CoarsenStep coarsen_level(Ctx &ctx, const DGraph &g, u32 *mp, DGraph &c, u32 &nc
         c = DGraph{};
         c.cap = g.m;
         c.total_vw = g.total_vw;
+        // Small levels keep the row bounds where the kernel writes them, sized
+        // for n (12 n bytes more, instead of three copies of a few
+        // microseconds each); larger ones copy them to arrays of the coarse size.
+        const bool direct = g.n <= COARSEN_DIRECT_MAX_N;
+        if (direct) {
+            c.rowptr = ctx.falloc<u32>((u64) g.n + 1);
+            c.rowlen = ctx.falloc<u32>(g.n);
+            c.vw = ctx.falloc<s32>(g.n);
+        }
         c.adj = ctx.falloc<u32>(c.cap);
         c.ew = ctx.falloc<s32>(c.cap);
         r = coarsen_team(ctx, g, mp, &c);
         nc = r.n;
-        if (r.contracted && (u64) nc * 100 <= (u64) g.n * 99) {
+        const bool keep_level = r.contracted && (u64) nc * 100 <= (u64) g.n * 99;
+        if (keep_level) {
             c.n = nc;
             c.m = r.m;
+        }
+        if (keep_level && !direct) {
             c.rowptr = ctx.falloc<u32>((u64) nc + 1);
             c.rowlen = ctx.falloc<u32>(nc);
             c.vw = ctx.falloc<s32>(nc);
@@ -84,7 +93,8 @@ CoarsenStep coarsen_level(Ctx &ctx, const DGraph &g, u32 *mp, DGraph &c, u32 &nc
             keep(c.rowptr, r.rowptr, sizeof(u32) * ((size_t) nc + 1));
             keep(c.rowlen, r.rowlen, sizeof(u32) * nc);
             keep(c.vw, r.vw, sizeof(s32) * nc);
-        } else {
+        }
+        if (!keep_level) {
             r.contracted = false;
             ctx.arena.front_release(mark);
         }
@@ -143,17 +153,13 @@ void uncoarsen(Ctx &ctx, Hierarchy &H, u32 *coarse_part, u32 *part_out, u32 k, s
     u32 *cpart = coarse_part;
     for (size_t l = H.maps.size(); l > 0; --l) {
         const DGraph &fine = H.graphs[l - 1];
-        auto t0 = Clock::now();
         u32 *fpart = (l == 1) ? part_out : ctx.falloc<u32>(fine.n);
-        k_project<<<ctx.grid(fine.n, BLOCK), BLOCK, 0, ctx.stream>>>(cpart, H.maps[l - 1], fpart, fine.n); note_launch();
-        HP_LAUNCH_CHECK();
-        if (stats) {
-            ctx.sync();
-            stats->uncontraction_ms += ms_since(t0);
-        }
         auto t1 = Clock::now();
-        jet_refine(ctx, fine, fpart, k, lmax, ultra, (u32) (l - 1), obj, maxw, D);
-        if (stats) stats->refinement_ms += ms_since(t1);
+        // (the projection, solver.h:388-392, is part of the level's set-up)
+        const double before = stats ? stats->uncontraction_ms : 0;
+        jet_refine(ctx, fine, fpart, k, lmax, ultra, (u32) (l - 1), obj, maxw, D,
+                   Projection{cpart, H.maps[l - 1], stats ? &stats->uncontraction_ms : nullptr});
+        if (stats) stats->refinement_ms += ms_since(t1) - (stats->uncontraction_ms - before);
         cpart = fpart;
     }
     if (H.maps.empty())

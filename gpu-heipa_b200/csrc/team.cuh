@@ -64,6 +64,12 @@ __device__ __forceinline__ T ld_fresh(const T *p) {
     return TEAM == TEAM_BLOCK ? *(const volatile T *) p : __ldcg(p);
 }
 
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
 // Launch configuration of a team of `blocks` blocks (attr must outlive it).
 inline cudaLaunchConfig_t team_config(u32 blocks, u32 threads, size_t smem, cudaStream_t stream,
                                       cudaLaunchAttribute &attr, int team) {
