@@ -163,14 +163,6 @@ struct Grp {
     }
 };
 
-// Loads of Jet state (labels, targets, gains) that the calling kernel does not
-// write go through the non-coherent path (NC); the fused small-level kernel,
-// which writes them between its phases, uses plain loads.
-template<bool NC, typename T>
-__device__ __forceinline__ T ldj(const T *p) {
-    return NC ? __ldg(p) : *p;
-}
-
 // Loads B row entries (ids and weights) strided by nthreads from t0.
 template<int B>
 __device__ __forceinline__ void load_entries(const JArgs &a, u64 beg, u32 t0, u32 to, u32 nthreads, u32 (&v)[B],
@@ -236,7 +228,7 @@ __device__ __forceinline__ u32 table_mask_for(u32 len, u32 k, u32 cap) {
 
 // Aggregates conn(u, .) into the group's hashed table (cleared on entry).
 // Four entries per thread are loaded before they are inserted.
-template<bool BLK, bool NC = true>
+template<bool BLK>
 __device__ __forceinline__ void table_build(const JArgs &a, u32 u, u32 *tk, s32 *tv, u32 mask) {
     const u64 beg = __ldg(&a.g.rowptr[u]);
     const u32 len = __ldg(&a.g.rowlen[u]);
@@ -252,7 +244,7 @@ __device__ __forceinline__ void table_build(const JArgs &a, u32 u, u32 *tk, s32 
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (bb[j] != EMPTY) bb[j] = ldj<NC>(&a.map[bb[j]]);
+            if (bb[j] != EMPTY) bb[j] = __ldg(&a.map[bb[j]]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const u32 b = bb[j];
@@ -288,11 +280,11 @@ __device__ __forceinline__ void table_clear(u32 *tk, s32 *tv, u32 mask) {
 // connection; weights are positive), so an entry costs one shared-memory add
 // and no compare-and-swap. Four entries per thread are loaded (ids, then
 // labels) before any table update, which keeps four gathers in flight.
-template<bool BLK, bool NC = true>
+template<bool BLK>
 __device__ __forceinline__ void dtable_build_range(const JArgs &a, u32 u, s32 *tv, u32 from, u32 len) {
     const u64 beg = __ldg(&a.g.rowptr[u]);
     const u32 gs = Grp<BLK>::size(), tid = Grp<BLK>::tid();
-    if (NC && a.vec) {
+    if (a.vec) {
         // the same with the entries read as 16-byte quads
         const u64 lo = beg + from, hi = beg + len;
         u64 qi = (lo >> 2) + tid;
@@ -306,7 +298,7 @@ __device__ __forceinline__ void dtable_build_range(const JArgs &a, u32 u, s32 *t
                 const bool more = next_quad(a, qn, lo, hi, bn, wn);
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (b[j] != EMPTY) b[j] = ldj<NC>(&a.map[b[j]]);
+                    if (b[j] != EMPTY) b[j] = __ldg(&a.map[b[j]]);
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     if (b[j] != EMPTY) atomicAdd(&tv[b[j]], w[j]);
@@ -322,59 +314,39 @@ __device__ __forceinline__ void dtable_build_range(const JArgs &a, u32 u, s32 *t
         Grp<BLK>::sync();
         return;
     }
-    if (NC) {
-        // kernels that do not write labels: the next four entries are loaded
-        // while the current four labels are gathered
-        u32 t0 = from + tid;
-        if (t0 < len) {
-            u32 b[4];
-            s32 w[4];
-            load_entries<4>(a, beg, t0, len, gs, b, w);
-            for (;;) {
-                const u32 t1 = t0 + 4 * gs;
-                u32 bn[4];
-                s32 wn[4];
-                load_entries<4>(a, beg, t1, len, gs, bn, wn);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (b[j] != EMPTY) b[j] = ldj<NC>(&a.map[b[j]]);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (b[j] != EMPTY) atomicAdd(&tv[b[j]], w[j]);
-                if (t1 >= len) break;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    b[j] = bn[j];
-                    w[j] = wn[j];
-                }
-                t0 = t1;
-            }
-        }
-        Grp<BLK>::sync();
-        return;
-    }
-    for (u32 t0 = from + tid; t0 < len; t0 += 4 * gs) {
+    // the next four entries are loaded while the current four labels are
+    // gathered
+    u32 t0 = from + tid;
+    if (t0 < len) {
         u32 b[4];
         s32 w[4];
+        load_entries<4>(a, beg, t0, len, gs, b, w);
+        for (;;) {
+            const u32 t1 = t0 + 4 * gs;
+            u32 bn[4];
+            s32 wn[4];
+            load_entries<4>(a, beg, t1, len, gs, bn, wn);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const u32 t = t0 + j * gs;
-            b[j] = t < len ? __ldg(&a.g.adj[beg + t]) : EMPTY;
-            w[j] = t < len ? g_ew(a.g, beg + t) : 0;
+            for (int j = 0; j < 4; ++j)
+                if (b[j] != EMPTY) b[j] = __ldg(&a.map[b[j]]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (b[j] != EMPTY) atomicAdd(&tv[b[j]], w[j]);
+            if (t1 >= len) break;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                b[j] = bn[j];
+                w[j] = wn[j];
+            }
+            t0 = t1;
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (b[j] != EMPTY) b[j] = ldj<NC>(&a.map[b[j]]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (b[j] != EMPTY) atomicAdd(&tv[b[j]], w[j]);
     }
     Grp<BLK>::sync();
 }
 
-template<bool BLK, bool NC = true>
+template<bool BLK>
 __device__ __forceinline__ void dtable_build(const JArgs &a, u32 u, s32 *tv) {
-    dtable_build_range<BLK, NC>(a, u, tv, 0, __ldg(&a.g.rowlen[u]));
+    dtable_build_range<BLK>(a, u, tv, 0, __ldg(&a.g.rowlen[u]));
 }
 
 template<bool BLK>
@@ -385,15 +357,15 @@ __device__ __forceinline__ void dtable_clear(s32 *tv, u32 k) {
 }
 
 // Connectivity table of one row: direct-indexed (DIRECT) or hashed.
-template<bool BLK, bool DIRECT, bool NC = true>
+template<bool BLK, bool DIRECT>
 struct ConnTable {
     u32 *tk;
     s32 *tv;
     u32 mask;  // hashed: slots - 1
     u32 k;
     __device__ __forceinline__ void build(const JArgs &a, u32 u) {
-        if (DIRECT) dtable_build<BLK, NC>(a, u, tv);
-        else table_build<BLK, NC>(a, u, tk, tv, mask);
+        if (DIRECT) dtable_build<BLK>(a, u, tv);
+        else table_build<BLK>(a, u, tk, tv, mask);
     }
     __device__ __forceinline__ u32 slots() const { return DIRECT ? k : mask + 1; }
     __device__ __forceinline__ u32 key(u32 s) const { return DIRECT ? (tv[s] != 0 ? s : EMPTY) : tk[s]; }
@@ -415,7 +387,6 @@ struct TRow {
 // loads in flight instead of a chain of JT), then equal blocks are merged into
 // their first occurrence. Labels are not written by the kernels that call
 // this, so they are read through the non-coherent path.
-template<bool NC = true>
 __device__ __forceinline__ void trow_build(const JArgs &a, u32 u, TRow &r) {
     const u64 beg = __ldg(&a.g.rowptr[u]);
     const u32 len = __ldg(&a.g.rowlen[u]);
@@ -426,7 +397,7 @@ __device__ __forceinline__ void trow_build(const JArgs &a, u32 u, TRow &r) {
     }
 #pragma unroll
     for (int s = 0; s < (int) JT; ++s)
-        if (r.b[s] != EMPTY) r.b[s] = ldj<NC>(&a.map[r.b[s]]);
+        if (r.b[s] != EMPTY) r.b[s] = __ldg(&a.map[r.b[s]]);
 #pragma unroll
     for (int s = 1; s < (int) JT; ++s) {
 #pragma unroll
@@ -480,10 +451,9 @@ __device__ __forceinline__ void lp_finish_map(const JArgs &a, u32 u, unsigned lo
     lp_store(a, u, best, gain);
 }
 
-template<bool NC = true>
 __device__ __forceinline__ void lp_thread(const JArgs &a, u32 u, u32 ratio) {
     TRow r;
-    trow_build<NC>(a, u, r);
+    trow_build(a, u, r);
     const u32 o = a.map[u];
     unsigned long long bk = 0;
     if (!a.code) {
@@ -514,8 +484,8 @@ __device__ __forceinline__ void lp_thread(const JArgs &a, u32 u, u32 ratio) {
 }
 
 // Best block of u from its built connectivity table T (clears T).
-template<bool BLK, bool DIRECT, bool NC = true>
-__device__ __forceinline__ void lp_finish_group(const JArgs &a, u32 u, u32 ratio, ConnTable<BLK, DIRECT, NC> T,
+template<bool BLK, bool DIRECT>
+__device__ __forceinline__ void lp_finish_group(const JArgs &a, u32 u, u32 ratio, ConnTable<BLK, DIRECT> T,
                                                 unsigned long long *smu, long long *sms) {
     const u32 o = a.map[u];
     unsigned long long bk = 0;
@@ -550,11 +520,11 @@ __device__ __forceinline__ void lp_finish_group(const JArgs &a, u32 u, u32 ratio
     T.clear();
 }
 
-template<bool BLK, bool DIRECT, bool NC = true>
-__device__ __forceinline__ void lp_group(const JArgs &a, u32 u, u32 ratio, ConnTable<BLK, DIRECT, NC> T,
+template<bool BLK, bool DIRECT>
+__device__ __forceinline__ void lp_group(const JArgs &a, u32 u, u32 ratio, ConnTable<BLK, DIRECT> T,
                                          unsigned long long *smu, long long *sms) {
     T.build(a, u);
-    lp_finish_group<BLK, DIRECT, NC>(a, u, ratio, T, smu, sms);
+    lp_finish_group<BLK, DIRECT>(a, u, ratio, T, smu, sms);
 }
 
 // Direct-indexed tables are used when k fits the table and, for the mapping
@@ -775,7 +745,6 @@ __global__ void __launch_bounds__(BLOCK) k_lp_filter(JArgs a) {
 
 // afterburner (:269-331 / ProMap :273-320): the terms of four loaded row
 // entries of u (v = SENTINEL marks an empty slot).
-template<bool NC>
 __device__ __forceinline__ s32 ab_batch(const JArgs &a, u32 u, s32 ug, u32 ou, u32 nu, const u32 (&v)[4],
                                         const s32 (&w)[4]) {
     u32 nv[4], ov[4];
@@ -787,7 +756,7 @@ __device__ __forceinline__ s32 ab_batch(const JArgs &a, u32 u, s32 ug, u32 ou, u
     if (a.abrec) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const unsigned long long r = v[j] != SENTINEL ? ldj<NC>(&a.abrec[v[j]]) : 0ull;
+            const unsigned long long r = v[j] != SENTINEL ? __ldg(&a.abrec[v[j]]) : 0ull;
             vg[j] = (s32) (u32) r;
             nv[j] = (u32) (r >> 32) & 0xFFFFu;
             ov[j] = (u32) (r >> 48);
@@ -796,13 +765,13 @@ __device__ __forceinline__ s32 ab_batch(const JArgs &a, u32 u, s32 ug, u32 ou, u
         for (int j = 0; j < 4; ++j) first[j] = v[j] != SENTINEL && (vg[j] > ug || (vg[j] == ug && v[j] < u));
     } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) vg[j] = v[j] != SENTINEL ? ldj<NC>(&a.gain1[v[j]]) : 0;
+        for (int j = 0; j < 4; ++j) vg[j] = v[j] != SENTINEL ? __ldg(&a.gain1[v[j]]) : 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             first[j] = v[j] != SENTINEL && (vg[j] > ug || (vg[j] == ug && v[j] < u));
             if (first[j]) {
-                nv[j] = ldj<NC>(&a.dest_part[v[j]]);
-                ov[j] = ldj<NC>(&a.map[v[j]]);
+                nv[j] = __ldg(&a.dest_part[v[j]]);
+                ov[j] = __ldg(&a.map[v[j]]);
             }
         }
     }
@@ -828,7 +797,7 @@ __device__ __forceinline__ s32 ab_batch(const JArgs &a, u32 u, s32 ug, u32 ou, u
 // and labels read here are not written by the afterburner kernels, so they
 // are gathered through the non-coherent path, four entries at a time; with
 // PF the next four row entries are loaded while those are gathered.
-template<bool NC = true, bool PF = false>
+template<bool PF = false>
 __device__ __forceinline__ s32 ab_range(const JArgs &a, u32 u, s32 ug, u32 ou, u32 nu, u32 from, u32 to, u32 tid,
                                         u32 nthreads) {
     const u64 beg = __ldg(&a.g.rowptr[u]);
@@ -844,7 +813,7 @@ __device__ __forceinline__ s32 ab_range(const JArgs &a, u32 u, s32 ug, u32 ou, u
             u32 vn[4];
             s32 wn[4];
             load_entries<4>(a, beg, t1, to, nthreads, vn, wn);
-            change = wadd(change, ab_batch<NC>(a, u, ug, ou, nu, v, w));
+            change = wadd(change, ab_batch(a, u, ug, ou, nu, v, w));
             if (t1 >= to) break;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -859,13 +828,12 @@ __device__ __forceinline__ s32 ab_range(const JArgs &a, u32 u, s32 ug, u32 ou, u
         u32 v[4];
         s32 w[4];
         load_entries<4>(a, beg, t0, to, nthreads, v, w);
-        change = wadd(change, ab_batch<NC>(a, u, ug, ou, nu, v, w));
+        change = wadd(change, ab_batch(a, u, ug, ou, nu, v, w));
     }
     return change;
 }
 
 // The same with 128-bit row reads (quads tid, tid + gs, ... of the segment).
-template<bool NC = true>
 __device__ __forceinline__ s32 ab_range_quads(const JArgs &a, u32 u, s32 ug, u32 ou, u32 nu, u32 from, u32 to,
                                               u32 tid, u32 gs) {
     const u64 beg = __ldg(&a.g.rowptr[u]);
@@ -880,7 +848,7 @@ __device__ __forceinline__ s32 ab_range_quads(const JArgs &a, u32 u, s32 ug, u32
         u32 vn[4];
         s32 wn[4];
         const bool more = next_quad(a, qn, lo, hi, vn, wn);
-        change = wadd(change, ab_batch<NC>(a, u, ug, ou, nu, v, w));
+        change = wadd(change, ab_batch(a, u, ug, ou, nu, v, w));
         if (!more) break;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -938,7 +906,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_ab_chunk(JArgs a) {
         const s32 ug = __ldg(&a.gain1[u]);
         const u32 ou = __ldg(&a.map[u]), nu = __ldg(&a.dest_part[u]);
         const s32 part = VEC ? ab_range_quads(a, u, ug, ou, nu, from, to, lane_id(), 32)
-                             : ab_range<true, true>(a, u, ug, ou, nu, from, to, lane_id(), 32);
+                             : ab_range<true>(a, u, ug, ou, nu, from, to, lane_id(), 32);
         const s32 change = (s32) warp_sum<u32>((u32) part);
         if (lane_id() == 0) {
             bool decide = nch == 1;
@@ -981,7 +949,7 @@ __device__ __forceinline__ bool hub_update_now(const JArgs &a) {
     return a.hub_cur && (unsigned long long) a.st->sum[SUM_PERF_ENTRIES] <= a.hub_track_max;
 }
 
-template<int B, bool NC>
+template<int B>
 __device__ __forceinline__ long long delta_batch(const JArgs &a, u32 nu, u32 ou, bool um, const u32 (&v)[B],
                                                  const s32 (&w)[B], bool inval, bool hub_upd) {
     long long acc = 0;
@@ -992,7 +960,7 @@ __device__ __forceinline__ long long delta_batch(const JArgs &a, u32 nu, u32 ou,
         // their order)
         unsigned long long xv[B];
 #pragma unroll
-        for (int j = 0; j < B; ++j) xv[j] = v[j] != SENTINEL ? ldj<NC>(&a.dlab[v[j]]) : 0ull;
+        for (int j = 0; j < B; ++j) xv[j] = v[j] != SENTINEL ? __ldg(&a.dlab[v[j]]) : 0ull;
 #pragma unroll
         for (int j = 0; j < B; ++j) {
             if (v[j] == SENTINEL) continue;
@@ -1011,9 +979,9 @@ __device__ __forceinline__ long long delta_batch(const JArgs &a, u32 nu, u32 ou,
     } else if (um) {
         u32 xv[B], ov[B];
 #pragma unroll
-        for (int j = 0; j < B; ++j) xv[j] = v[j] != SENTINEL ? ldj<NC>(&a.map[v[j]]) : 0;
+        for (int j = 0; j < B; ++j) xv[j] = v[j] != SENTINEL ? __ldg(&a.map[v[j]]) : 0;
 #pragma unroll
-        for (int j = 0; j < B; ++j) ov[j] = (xv[j] & MOVED) ? ldj<NC>(&a.dest_part[v[j]]) : (xv[j] & ~MOVED);
+        for (int j = 0; j < B; ++j) ov[j] = (xv[j] & MOVED) ? __ldg(&a.dest_part[v[j]]) : (xv[j] & ~MOVED);
 #pragma unroll
         for (int j = 0; j < B; ++j) {
             if (v[j] == SENTINEL) continue;
@@ -1034,14 +1002,14 @@ __device__ __forceinline__ long long delta_batch(const JArgs &a, u32 nu, u32 ou,
 
 // With PF, the next batch's row entries are loaded before the current
 // batch's label gathers, so the row read and the gathers overlap.
-template<bool NC = true, int B = 4, bool PF = false>
+template<int B = 4, bool PF = false>
 __device__ __forceinline__ long long delta_range(const JArgs &a, u32 u, u32 from, u32 to, u32 tid, u32 nthreads,
                                                  bool inval, bool hub_upd = false) {
     const u64 beg = __ldg(&a.g.rowptr[u]);
-    const u32 x = ldj<NC>(&a.map[u]);
+    const u32 x = __ldg(&a.map[u]);
     const bool um = (x & MOVED) != 0;
     const u32 nu = x & ~MOVED;
-    const u32 ou = um ? ldj<NC>(&a.dest_part[u]) : nu;
+    const u32 ou = um ? __ldg(&a.dest_part[u]) : nu;
     long long acc = 0;
     if (PF) {
         u32 t0 = from + tid;
@@ -1054,7 +1022,7 @@ __device__ __forceinline__ long long delta_range(const JArgs &a, u32 u, u32 from
             u32 vn[B];
             s32 wn[B];
             load_entries<B>(a, beg, t1, to, nthreads, vn, wn);
-            acc += delta_batch<B, NC>(a, nu, ou, um, v, w, inval, hub_upd);
+            acc += delta_batch<B>(a, nu, ou, um, v, w, inval, hub_upd);
             if (t1 >= to) break;
 #pragma unroll
             for (int j = 0; j < B; ++j) {
@@ -1069,7 +1037,7 @@ __device__ __forceinline__ long long delta_range(const JArgs &a, u32 u, u32 from
         u32 v[B];
         s32 w[B];
         load_entries<B>(a, beg, t0, to, nthreads, v, w);
-        acc += delta_batch<B, NC>(a, nu, ou, um, v, w, inval, hub_upd);
+        acc += delta_batch<B>(a, nu, ou, um, v, w, inval, hub_upd);
     }
     return acc;
 }
@@ -1077,14 +1045,13 @@ __device__ __forceinline__ long long delta_range(const JArgs &a, u32 u, u32 from
 // The same with 128-bit row reads: thread tid of a group of gs takes quads
 // tid, tid + gs, ... of the row segment, the next quad loaded while the
 // current one's labels are gathered.
-template<bool NC = true>
 __device__ __forceinline__ long long delta_range_quads(const JArgs &a, u32 u, u32 from, u32 to, u32 tid, u32 gs,
                                                        bool inval, bool hub_upd) {
     const u64 beg = __ldg(&a.g.rowptr[u]);
-    const u32 x = ldj<NC>(&a.map[u]);
+    const u32 x = __ldg(&a.map[u]);
     const bool um = (x & MOVED) != 0;
     const u32 nu = x & ~MOVED;
-    const u32 ou = um ? ldj<NC>(&a.dest_part[u]) : nu;
+    const u32 ou = um ? __ldg(&a.dest_part[u]) : nu;
     const u64 lo = beg + from, hi = beg + to;
     u64 qi = (lo >> 2) + tid;
     u32 v[4];
@@ -1096,7 +1063,7 @@ __device__ __forceinline__ long long delta_range_quads(const JArgs &a, u32 u, u3
         u32 vn[4];
         s32 wn[4];
         const bool more = next_quad(a, qn, lo, hi, vn, wn);
-        acc += delta_batch<4, NC>(a, nu, ou, um, v, w, inval, hub_upd);
+        acc += delta_batch<4>(a, nu, ou, um, v, w, inval, hub_upd);
         if (!more) break;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -1126,7 +1093,7 @@ __device__ __forceinline__ long long delta_staged(const JArgs &a, u32 u, const u
             v[j] = t < len ? sadj[t] : SENTINEL;
             w[j] = t < len ? (sew ? sew[t] : 1) : 0;
         }
-        acc += delta_batch<B, true>(a, nu, ou, um, v, w, inval, hub_upd);
+        acc += delta_batch<B>(a, nu, ou, um, v, w, inval, hub_upd);
     }
     return acc;
 }
@@ -1234,7 +1201,7 @@ __global__ void __launch_bounds__(BLOCK, (B > 4 || VEC) ? 4 : 5) k_delta_chunk(J
         u32 u, from, to, nch;
         chunk_range(a, __ldg(&a.items[i]), u, from, to, nch);
         if (VEC) acc += delta_range_quads(a, u, from, to, lane_id(), 32, inval, hub_upd);
-        else acc += delta_range<true, B, B <= 4>(a, u, from, to, lane_id(), 32, inval, hub_upd);
+        else acc += delta_range<B, B <= 4>(a, u, from, to, lane_id(), 32, inval, hub_upd);
     }
     acc = warp_sum<long long>(acc);
     if (lane_id() == 0 && acc) atomicAdd((unsigned long long *) &a.st->sum[SUM_DELTA], (unsigned long long) acc);
@@ -1370,10 +1337,10 @@ __device__ __forceinline__ bool rb_qualifies(const JArgs &a, const RbArgs &r, u3
     return (s64) vw <= 2 * (s64) maxv && (s64) vw < 2 * (ow - r.opt);
 }
 
-template<bool STRONG, bool NC = true>
+template<bool STRONG>
 __device__ __forceinline__ void rb_thread(const JArgs &a, const RbArgs &r, u32 u, u32 o) {
     TRow row;
-    trow_build<NC>(a, u, row);
+    trow_build(a, u, row);
     s32 own = 0, sum = 0, count = 0;
     unsigned long long bk = 0;
 #pragma unroll
@@ -1398,9 +1365,9 @@ __device__ __forceinline__ void rb_thread(const JArgs &a, const RbArgs &r, u32 u
     else weak_finish(a, r, u, o, own, bk);
 }
 
-template<bool STRONG, bool BLK, bool DIRECT, bool NC = true>
+template<bool STRONG, bool BLK, bool DIRECT>
 __device__ __forceinline__ void rb_finish_group(const JArgs &a, const RbArgs &r, u32 u,
-                                                ConnTable<BLK, DIRECT, NC> T, unsigned long long *smu,
+                                                ConnTable<BLK, DIRECT> T, unsigned long long *smu,
                                                 long long *sms) {
     const u32 o = a.map[u];
     long long own = 0, sum = 0, count = 0;
@@ -1438,11 +1405,11 @@ __device__ __forceinline__ void rb_finish_group(const JArgs &a, const RbArgs &r,
     T.clear();
 }
 
-template<bool STRONG, bool BLK, bool DIRECT, bool NC = true>
-__device__ __forceinline__ void rb_group(const JArgs &a, const RbArgs &r, u32 u, ConnTable<BLK, DIRECT, NC> T,
+template<bool STRONG, bool BLK, bool DIRECT>
+__device__ __forceinline__ void rb_group(const JArgs &a, const RbArgs &r, u32 u, ConnTable<BLK, DIRECT> T,
                                          unsigned long long *smu, long long *sms) {
     T.build(a, u);
-    rb_finish_group<STRONG, BLK, DIRECT, NC>(a, r, u, T, smu, sms);
+    rb_finish_group<STRONG, BLK, DIRECT>(a, r, u, T, smu, sms);
 }
 
 template<bool STRONG>
