@@ -163,7 +163,8 @@ struct Ctx {
     // and kept until destroy().
     std::vector<std::unique_ptr<Ctx> > workers;
     Ctx &worker(size_t i);
-    u32 peers = 1;  // contexts that run solves on the device beside this one (itself included)
+    u32 peers = 1;          // contexts that run solves on the device beside this one (itself included) ...
+    u32 peer_blocks = 56;   // ... and then the least number of blocks a grid team may take (team_grid_blocks)
 
     void init(int dev, size_t arena_bytes);
     void destroy();

@@ -2694,11 +2694,13 @@ constexpr u32 TEAM_BLOCK_MAX_N = 4096;
 // team up to these sizes. Barriers dominate small levels whatever their
 // degree (ultra R-MAT 65k, levels of up to 600 entries per vertex: 302 ms with
 // a limit of 32, 221 ms with none); on larger dense levels the rows dominate,
-// which the per-kernel loop cuts into chunks and sums hub rows once (R-MAT 4M:
-// 278 ms with a limit of 128 entries per vertex, 293 ms with none; its top
-// level, 31 entries per vertex and 1.3e8 entries, 285 ms as a team).
+// which the per-kernel loop cuts into chunks and sums hub rows once. Limits of
+// 2^22 / 2^23 / 2^24 / 2^26 entries for up to 128 per vertex: R-MAT 18 ef 8
+// k=16 37.7 / 37.9 / 37.8 / 37.8 ms (45.0 with none), R-MAT 19 ef 16 k=128 69.4
+// / 69.6 / 89.0 / 89 ms, IM R-MAT 18 ef 16 95 / 121 / 121 / 121 ms, R-MAT 21 ef
+// 8 k=128 128 / 128 / 128 / 156 ms.
 constexpr u64 TEAM_ANY_DEG_M = 1ull << 21;
-constexpr u64 TEAM_MID_DEG_M = 1ull << 26, TEAM_MID_DEG = 128;
+constexpr u64 TEAM_MID_DEG_M = 1ull << 22, TEAM_MID_DEG = 128;
 
 template<bool HASH, bool MAP>
 static const void *team_kernel_of(int team) {

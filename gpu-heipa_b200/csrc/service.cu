@@ -58,7 +58,10 @@ Service::Service(Ctx &owner, char *base, size_t bytes, size_t workers) : device_
     regions_.reset(bytes & ~(REGION_ALIGN - 1));
     if (workers == 0) workers = 1;
     for (size_t w = 0; w < workers; ++w) ctxs_.push_back(&owner.worker(w));
-    for (Ctx *c: ctxs_) c->peers = owner.peers * (u32) workers;
+    for (Ctx *c: ctxs_) {
+        c->peers = owner.peers * (u32) workers;
+        c->peer_blocks = owner.peer_blocks;
+    }
     for (size_t w = 0; w < workers; ++w) threads_.emplace_back([this, w] { worker_main(w); });
 }
 

@@ -1,5 +1,6 @@
 #include "solver.cuh"
 #include "prims.cuh"
+#include "team.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -278,6 +279,7 @@ void run_hm_tasks(Ctx &ctx, std::vector<HmTask> &tasks, Fn fn) {
     for (size_t w = 0; w < W; ++w) {
         wc[w] = &ctx.worker(w);
         wc[w]->peers = ctx.peers * (u32) W;
+        wc[w]->peer_blocks = HM_PEER_BLOCKS;
         wc[w]->arena.attach(slab + w * slice, slice);
     }
     std::atomic<size_t> next{0};

@@ -108,11 +108,14 @@ inline u32 team_cluster_limit(const void *kernel, size_t smem, u32 most) {
 }
 
 // Blocks of a grid team for `want` of them, one SM each: at least two, at most
-// what fits on the GPU at once. Beside other solves (HM sub-solves, batch and
-// server workers) a grid takes a share of the SMs, so that grids run side by
-// side instead of one after another at full width: HM RGG 8M 403 ms uncapped,
-// 342 / 359 ms with at least 32 / 64 blocks each.
-constexpr u32 TEAM_PEER_BLOCKS = 40;
+// what fits on the GPU at once. Beside other solves a grid takes a share of the
+// SMs, so that grids run side by side instead of one after another at full
+// width (HM RGG 8M: 403 ms uncapped, 342 ms with shares of 32 blocks). The
+// sub-solves of a multisection are alike and finish together: small shares
+// serve them best (16 / 24 / 40 / 56 blocks: 244 / 251 / 264 / 294 ms). Batch
+// and server jobs differ, and often few of them run a grid at a time (146 / 135
+// / 127 / 127 ms for the batch of 32 graphs).
+constexpr u32 HM_PEER_BLOCKS = 20;
 
 inline u32 team_grid_blocks(const Ctx &ctx, const void *kernel, size_t smem, u64 want) {
     int per_sm = 0;
@@ -120,9 +123,9 @@ inline u32 team_grid_blocks(const Ctx &ctx, const void *kernel, size_t smem, u64
     if (per_sm <= 0) return 0;
     u64 cap = (u64) per_sm * ctx.sm_count;
     if (ctx.peers > 1) {
-        const u64 share = 2 * (u64) ctx.sm_count / ctx.peers;
-        cap = cap < TEAM_PEER_BLOCKS || share < TEAM_PEER_BLOCKS ? (cap < TEAM_PEER_BLOCKS ? cap : TEAM_PEER_BLOCKS)
-                                                                 : (cap < share ? cap : share);
+        u64 share = 2 * (u64) ctx.sm_count / ctx.peers;
+        if (share < ctx.peer_blocks) share = ctx.peer_blocks;
+        if (share < cap) cap = share;
     }
     want = want < cap ? want : cap;
     return (u32) (want < 2 ? 2 : want);
