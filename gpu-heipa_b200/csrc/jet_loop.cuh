@@ -570,6 +570,13 @@ __device__ __forceinline__ void peer_prefix(u32 mask, s32 v, s32 &p, s32 &t) {
     }
 }
 
+// Weight of overloaded block o above the limit (all weights together fit 31
+// bits, so a limit far below zero may be cut off there).
+__device__ __forceinline__ s32 excess_of(const TeamArgs &a, const TeamSm &S, u32 o) {
+    const s64 x = (s64) S.bw[o] - (s64) a.lmax;
+    return x > INT32_MAX ? INT32_MAX : (s32) x;
+}
+
 // Adds v over all threads to *slot with one atomic per block. No block
 // barrier follows: the team barrier does.
 __device__ __forceinline__ void team_add(long long v, long long *slot, long long *sm) {
@@ -1020,7 +1027,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                     }
                     const s32 total = __shfl_sync(FULL, inc, 7, 8) + spill;
                     s32 run = spill + inc - mine;
-                    const s32 limit = act ? S.bw[o] - a.lmax : 0;
+                    const s32 limit = act ? excess_of(a, S, o) : 0;
                     if (act && gl == 0) {
                         S.toff[o] = 0;
                         // all bins but the last one of strong keys, which the
@@ -1143,7 +1150,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                         if (cut) {
                             if ((peers & lt) == 0) S.tab[o] = before + t;
                             const s32 score = S.cutbase[o] + S.toff[o] + before + p;
-                            const s32 limit = S.bw[o] - a.lmax;
+                            const s32 limit = excess_of(a, S, o);
                             take = score < limit;
                             if (strong && take && score + vw >= limit) a.ea[o] = score + vw;
                         }

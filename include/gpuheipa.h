@@ -185,14 +185,14 @@ int hp_last_solve_level(const hp_ctx *ctx, uint32_t index, uint32_t *n, uint64_t
  * HP_DEVERR_SPIN in the kernel's error word and end. *err_bits receives that
  * word, *ms (if non-NULL) the kernel's duration. Returns HP_OK when the call
  * ran (whatever the bits), HP_ERR_ARG for a bad device or block count. The
- * cooperative Jet level loop and matching loop use the same barrier. No
- * counterpart in the reference. */
+ * grid teams of the Jet level loop and of the coarsening kernel use the same
+ * barrier. No counterpart in the reference. */
 #define HP_DEVERR_SPIN 8u
 int hp_selftest_barrier_timeout(int device, uint32_t blocks, uint32_t *err_bits, double *ms);
 
 /* Diagnostics of the cooperative-launch budget (host only, no device work).
- * Grids whose blocks wait for one another at grid barriers (the cooperative
- * Jet level loop and matching loop, and the self-test above) share a budget
+ * Grids whose blocks wait for one another at grid barriers (the grid teams of
+ * the Jet level loop and of the coarsening kernel, and the self-test above) share a budget
  * of as many blocks as the device has SMs: a grid of b blocks holds min(b,
  * budget) of it until its kernel has completed, and a larger grid holds all
  * of it. The grids running together then have at most one block per SM in

@@ -78,3 +78,18 @@ def test_team_loop_equals_oracle(name, start, team):
         dg.free()
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("lmax", [-2 ** 30, -1, 0])
+def test_limits_that_no_block_can_meet(lmax):
+    # every block is overloaded by its whole weight or more
+    g, k = weighted(H.Graph.grid(31, 29, 1, 5, seed=3), 7), 6
+    og = to_oracle(g)
+    part = np.random.default_rng(3).integers(0, k, g.n).astype(np.uint32)
+    maxw = int(np.bincount(part, weights=g.vw, minlength=k).max())
+    cut = O.edge_cut(og, part)
+    want = O.jet_refine(og, k, lmax, False, 0, part, cut, maxw)
+    with H.Context(0, 64 << 20) as c:
+        got = c.jet_refine(c.upload(g), k, lmax, part, cut, maxw)
+    assert got[1:] == want[1:]
+    np.testing.assert_array_equal(got[0], want[0])
