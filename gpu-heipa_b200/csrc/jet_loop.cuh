@@ -311,12 +311,13 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
         for (int j = 0; j < 4; ++j) {
             at[j] = b[j];
             if (HASH && b[j] != EMPTY) {  // at most 32 keys in 64 slots
-                u32 h = (b[j] * 2654435761u) >> 26;
-                for (;;) {
+                u32 h = (b[j] * 2654435761u) >> 26, probe = 0;
+                for (; probe < 64; ++probe) {
                     const u32 prev = atomicCAS((u32 *) &tv[h], 0u, b[j] + 1);
                     if (prev == 0 || prev == b[j] + 1) break;
                     h = (h + 1) & 63u;
                 }
+                if (probe == 64) set_error(&a.out->err, DEV_ERR_HASH_FULL);
                 at[j] = 64 + h;
             }
         }
@@ -324,12 +325,19 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
         for (int j = 0; j < 4; ++j)
             if (b[j] != EMPTY) atomicAdd(&tv[at[j]], w[j]);
         __syncwarp();
-        // the exchange returns a block's connection to one of its entries and
-        // clears the table
+        // an exchange returns a block's connection to one of its entries and
+        // clears the table; of a hashed table it takes the key, because a
+        // connection can be 0 (weights are added modulo 2^32) and a key that
+        // stayed behind would fill the table for the rows that follow
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            w[j] = b[j] != EMPTY ? atomicExch(&tv[at[j]], 0) : 0;
-            if (HASH && w[j] != 0) tv[at[j] - 64] = 0;
+            if (!HASH) {
+                w[j] = b[j] != EMPTY ? atomicExch(&tv[at[j]], 0) : 0;
+            } else {
+                const bool first = b[j] != EMPTY && atomicExch(&tv[at[j] - 64], 0) != 0;
+                w[j] = first ? tv[at[j]] : 0;
+                if (first) tv[at[j]] = 0;
+            }
         }
         __syncwarp();
         RowOut r{0, 0, 0, 0};
@@ -1464,6 +1472,7 @@ __global__ void __launch_bounds__(512, 1) k_jet_block(const __grid_constant__ Te
     if (tid == 0) {
         out->hubs = 0;
         out->gave_up = 0;
+        out->err = 0;
     }
     if (tid < 2 * TS_N) a.sum[tid] = 0;
     if (tid < 2 * TC_N) a.cnt[tid] = 0;
@@ -1502,6 +1511,7 @@ __global__ void __launch_bounds__(512, 1) k_jet_block(const __grid_constant__ Te
         ga.out->maxw = out->maxw;
         ga.out->iterations = out->iterations;
         ga.out->gave_up = out->gave_up;
+        ga.out->err = out->err;
         ga.out->setup_ns = out->setup_ns;
     }
 }

@@ -93,3 +93,61 @@ def test_limits_that_no_block_can_meet(lmax):
         got = c.jet_refine(c.upload(g), k, lmax, part, cut, maxw)
     assert got[1:] == want[1:]
     np.testing.assert_array_equal(got[0], want[0])
+
+
+def runs_of_four(n, seed):
+    """Runs of four vertices, each vertex joined to its run and to all of six other runs. Entries between even runs weigh
+    2^30, so that four of them add up to 0 modulo 2^32; inside an even run 100, elsewhere 1 to 5."""
+    r = n // 4
+    order = np.random.default_rng(seed).permutation(r)  # place of a run -> its id
+    place = np.argsort(order)
+    rows, cols, w = [], [], []
+    for d in (0, 1, 2, 6):
+        a, b = np.arange(r), order[(place + d) % r]
+        for i in range(4):
+            for j in range(4):
+                if d == 0 and i >= j:
+                    continue
+                rows.append(4 * a + i)
+                cols.append(4 * b + j)
+                even = (a % 2 == 0) & (b % 2 == 0)
+                w.append(np.where(even, 100 if d == 0 else 1 << 30, (a + b + i + j) % 5 + 1))
+    rows, cols, w = (np.concatenate(x) for x in (rows, cols, w))
+    rows, cols, w = np.concatenate([rows, cols]), np.concatenate([cols, rows]), np.concatenate([w, w])
+    at = np.lexsort((cols, rows))
+    xadj = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=4 * r))])
+    return H.Graph(xadj, cols[at], w[at].astype(np.int32))
+
+
+def refine_both(g, k, part, lmax, tunes, hd=None, ultra=False):
+    """jet_refine by a team and by the per-kernel loop (which has no size limits): (labels, objective, weight) of each."""
+    hier, dist = hd if hd else (None, None)
+    maxw = int(np.bincount(part, weights=g.vw, minlength=k).max())
+    out = []
+    for t in (tunes, {"jet_fused_max_n": 0, "jet_coop_max_n": 0}):
+        with H.Context(0, 256 << 20) as c:
+            for name, v in t.items():
+                c.tune(name, v)
+            dg = c.upload(g)
+            obj = c.comm_cost(dg, part, hier, dist) if hd else c.edge_cut(dg, part)
+            out.append(c.jet_refine(dg, k, lmax, part, obj, maxw, ultra=ultra, hierarchy=hier, distance=dist))
+            dg.free()
+    return out
+
+
+# team -> (vertices, blocks, settings): cluster and grid levels on few warps, so that the rows of a table meet more blocks
+# with connection 0 than the table has slots
+HASHED = {"block": (300, 257, TEAMS["cluster"]), "cluster": (40000, 1000, TEAMS["cluster"]),
+          "grid": (24000, 1000, dict(TEAMS["grid"], jet_coop_rows=1 << 20))}
+
+
+@pytest.mark.parametrize("team", sorted(HASHED))
+@pytest.mark.parametrize("ultra", [False, True])
+def test_hashed_tables_when_connections_are_zero(ultra, team):
+    n, k, tunes = HASHED[team]
+    g = runs_of_four(n, 5)
+    part = (np.arange(n) // 4 % k).astype(np.uint32)
+    got, want = refine_both(g, k, part, 2 * int(np.bincount(part).max()), tunes, ultra=ultra)
+    assert got[1:] == want[1:]
+    np.testing.assert_array_equal(got[0], want[0])
+    assert (got[0] != part).any()
