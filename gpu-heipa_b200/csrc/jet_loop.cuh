@@ -52,6 +52,7 @@ constexpr u32 TEAM_OWN = 48;           // candidates / moves of a warp kept in s
 
 enum TeamCnt { TC_HUB = 0, TC_MOVES = 1, TC_FAIL = 2, TC_N = 4 };
 enum TeamSum { TS_MOVES = 0, TS_DELTA = 1, TS_N = 2 };  // (moves << 32) + their row entries; objective change
+constexpr u32 LOCK_HUB = 2;            // lock word of a hub row that is a candidate of this iteration
 constexpr u32 TW_STILL = 0x80000000u;  // stamp flag: in the move list with an unchanged label
 
 // Vertex word: label (16 bits), previous label (16 bits), iteration that
@@ -744,7 +745,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                         const u32 sh = warp_append(&cnt[TC_HUB], hb);
                         if (hb) a.hubs[sh] = u;
                     }
-                    // a hub row's record says later whether it is a candidate
+                    // a hub row's lock word says later whether it is a candidate
                     const bool c = hb || (act && lp_filter_one(a, u, o, dest, gain, lock));
                     const u32 mask = __ballot_sync(FULL, c);
                     if (c) cl[nc + __popc(mask & lt)] = u;
@@ -769,7 +770,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                                 lp_decide<MAP>(r, ratio, dest, gain);
                                 a.dest_cache[u] = dest;
                                 a.gain_cache[u] = gain;
-                                lp_filter_one(a, u, o, dest, gain, a.lock[u]);
+                                if (lp_filter_one(a, u, o, dest, gain, a.lock[u])) a.lock[u] = LOCK_HUB;
                             }
                         }
                         __syncthreads();
@@ -786,12 +787,12 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                         u = cl[i];
                         ld_row<TEAM>(a, u, beg, len);
                         rec = a.abrec[u];
+                        if (len > TEAM_HUB && a.lock[u] != LOCK_HUB) {  // a hub row that is none
+                            act = false;
+                            len = 0;
+                        }
                     }
                     const s32 ug = (s32) (u32) rec;
-                    if (ug == GAIN_MIN) {  // a hub row that is none
-                        act = false;
-                        len = 0;
-                    }
                     const u32 nu = (u32) (rec >> 32) & 0xFFFFu, ou = (u32) (rec >> 48);
                     s32 ch = 0;
                     if (act && len <= TEAM_LONG) ch = team_ab<TEAM, MAP>(a, S, u, ug, ou, nu, beg, len, gl, 8);
@@ -799,6 +800,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
 #pragma unroll
                     for (int d = 4; d > 0; d >>= 1) ch = wadd(ch, __shfl_xor_sync(FULL, ch, d));
                     bool mine = act && gl == 0;  // decided here
+                    if (mine && len > TEAM_HUB) a.lock[u] = 0;
                     if (mine && len > TEAM_SHARE) {
                         const u32 p = atomicAdd(&c_cnt, 1u);
                         if (p < TEAM_SHARE_MAX) {

@@ -151,3 +151,30 @@ def test_hashed_tables_when_connections_are_zero(ultra, team):
     assert got[1:] == want[1:]
     np.testing.assert_array_equal(got[0], want[0])
     assert (got[0] != part).any()
+
+
+def circulant(n, reach, w):
+    """A ring in which every vertex is joined to the `reach` next and previous ones; w: weight of each ring distance."""
+    off = np.concatenate([np.arange(-reach, 0), np.arange(1, reach + 1)])
+    cols = (np.arange(n)[:, None] + off[None, :]) % n
+    at = np.argsort(cols, axis=1)
+    ew = np.asarray(w, np.int64)[np.abs(off) - 1][at]
+    return H.Graph(np.arange(n + 1) * 2 * reach, np.take_along_axis(cols, at, 1).ravel(), ew.ravel().astype(np.int32))
+
+
+@pytest.mark.parametrize("team", ["block", "cluster", "grid"])
+@pytest.mark.parametrize("k", [75, 300])
+@pytest.mark.parametrize("reach", [9, 16, 20, 600])
+def test_gains_at_the_ends_of_the_range(reach, k, team):
+    # connections and gains of -2^31 (two entries of 2^30; a connection of 0 less one of -2^31) are values as all others
+    n, k = (300, k // 4) if team == "block" else (6000, k)
+    if 2 * reach >= n:
+        pytest.skip("no such ring")
+    g = circulant(n, reach, np.full(reach, 1 << 30))
+    part = (np.arange(n) // 4 % k).astype(np.uint32)
+    part[::37] = (part[::37] + 1) % k
+    maxw = int(np.bincount(part).max())
+    for lmax in (maxw, 2 * maxw):
+        got, want = refine_both(g, k, part, lmax, TEAMS["grid" if team == "grid" else "cluster"])
+        assert got[1:] == want[1:]
+        np.testing.assert_array_equal(got[0], want[0])
