@@ -82,6 +82,14 @@ void check_hier(const uint32_t *hier, const int32_t *dist, uint32_t levels) {
     if (!hier || !dist || levels == 0) throw hp::HpError{HP_ERR_ARG, "hierarchy and distance are required"};
 }
 
+// One exit, after the loop: a loop that leaves at the first bad label took 0.29
+// or 0.57 ms for 1 M labels, by where the linker had put it, this one 0.31.
+void check_labels(const uint32_t *part, uint32_t n, uint32_t k) {
+    uint32_t largest = 0;
+    for (uint32_t u = 0; u < n; ++u) largest = part[u] > largest ? part[u] : largest;
+    if (n && largest >= k) throw hp::HpError{HP_ERR_ARG, "partition label out of range"};
+}
+
 } // namespace
 
 extern "C" {
@@ -248,8 +256,7 @@ int hp_jet_refine(hp_ctx *ctx, const hp_graph *g, uint32_t k, int32_t lmax, int 
             D = hp::make_dist_oracle(ctx->c, vec_u32(hier, levels), vec_s32(dist, levels));
             if (D.k != k) throw hp::HpError{HP_ERR_ARG, "k must equal the product of the hierarchy"};
         }
-        for (uint32_t u = 0; u < g->g.n; ++u)
-            if (part[u] >= k) throw hp::HpError{HP_ERR_ARG, "partition label out of range"};
+        check_labels(part, g->g.n, k);
         hp::u32 *d = ctx->c.balloc<hp::u32>(g->g.n);
         HP_CUDA(cudaMemcpyAsync(d, part, sizeof(hp::u32) * g->g.n, cudaMemcpyHostToDevice, ctx->c.stream));
         hp::s64 o = *obj;
@@ -279,8 +286,7 @@ int hp_jet_begin(hp_ctx *ctx, const hp_graph *g, uint32_t k, int32_t lmax, const
             j->has_D = true;
             if (j->D.k != k) throw hp::HpError{HP_ERR_ARG, "k must equal the product of the hierarchy"};
         }
-        for (uint32_t u = 0; u < g->g.n; ++u)
-            if (part[u] >= k) throw hp::HpError{HP_ERR_ARG, "partition label out of range"};
+        check_labels(part, g->g.n, k);
         hp::u32 *d = ctx->c.balloc<hp::u32>(g->g.n);
         HP_CUDA(cudaMemcpyAsync(d, part, sizeof(hp::u32) * g->g.n, cudaMemcpyHostToDevice, ctx->c.stream));
         j->L.setup(ctx->c, g->g, k, lmax, j->has_D ? &j->D : nullptr, d);
