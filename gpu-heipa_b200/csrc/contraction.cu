@@ -416,6 +416,7 @@ DGraph contract_graph(Ctx &ctx, const DGraph &g, const u32 *mapping, u32 n_c) {
     c.n = n_c;
     c.cap = g.m;
     c.total_vw = g.total_vw;
+    c.row_ew = c.all_ew = g.all_ew;
     c.rowptr = ctx.falloc<u32>((u64) n_c + 1);
     c.rowlen = ctx.falloc<u32>(n_c);
     c.vw = ctx.falloc<s32>(n_c);

@@ -33,16 +33,45 @@ __global__ void k_rows(DGraph g, u32 *err, long long *vw_sum) {
     if (lane_id() == 0) atomicAdd((unsigned long long *) vw_sum, (unsigned long long) local);
 }
 
-// Checks neighbour ids and edge weights; one warp per row.
-__global__ void k_validate_edges(DGraph g, u32 *err) {
+// Checks neighbour ids and edge weights (check), and finds the largest weight
+// of a row and the weight of all entries; one warp per row.
+__global__ void __launch_bounds__(BLOCK) k_edges(DGraph g, bool check, u32 *err, unsigned long long *row_ew,
+                                                 unsigned long long *all_ew) {
+    __shared__ unsigned long long sm[2][BLOCK / 32];
     const u32 warps = (gridDim.x * blockDim.x) >> 5;
+    unsigned long long most = 0, all = 0;
     for (u32 u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < g.n; u += warps) {
         const u64 beg = g.rowptr[u];
         const u32 len = g.rowlen[u];
+        unsigned long long row = 0;
         for (u32 t = lane_id(); t < len; t += 32) {
-            u32 v = g.adj[beg + t];
-            if (v >= g.n || v == u) set_error(err, DEV_ERR_BAD_ID);
-            if (g.ew && g.ew[beg + t] < 1) set_error(err, DEV_ERR_BAD_WEIGHT);
+            if (check) {
+                u32 v = g.adj[beg + t];
+                if (v >= g.n || v == u) set_error(err, DEV_ERR_BAD_ID);
+            }
+            if (g.ew) {
+                const s32 w = g.ew[beg + t];
+                if (check && w < 1) set_error(err, DEV_ERR_BAD_WEIGHT);
+                row += (u32) w;
+            }
+        }
+        row = warp_sum<unsigned long long>(row);
+        most = row > most ? row : most;
+        all += row;
+    }
+    if (lane_id() == 0) {
+        sm[0][warp_in_block()] = most;
+        sm[1][warp_in_block()] = all;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (u32 w = 1; w < BLOCK / 32; ++w) {
+            most = sm[0][w] > most ? sm[0][w] : most;
+            all += sm[1][w];
+        }
+        if (most) {
+            atomicMax(row_ew, most);
+            atomicAdd(all_ew, all);
         }
     }
 }
@@ -51,8 +80,10 @@ static void finish_graph(Ctx &ctx, DGraph &g, bool validate) {
     ctx.zero_status();
     k_rows<<<ctx.grid(g.n, BLOCK), BLOCK, 0, ctx.stream>>>(g, &ctx.d_status->err, &ctx.d_status->sum[0]); note_launch();
     HP_LAUNCH_CHECK();
-    if (validate && g.cap > 0) {
-        k_validate_edges<<<ctx.grid((u64) g.n * 32, BLOCK), BLOCK, 0, ctx.stream>>>(g, &ctx.d_status->err); note_launch();
+    if ((validate || g.ew) && g.cap > 0) {
+        k_edges<<<ctx.grid((u64) g.n * 32, BLOCK), BLOCK, 0, ctx.stream>>>(
+            g, validate, &ctx.d_status->err, (unsigned long long *) &ctx.d_status->sum[1],
+            (unsigned long long *) &ctx.d_status->sum[2]); note_launch();
         HP_LAUNCH_CHECK();
     }
     const DevStatus &s = ctx.read_status();
@@ -62,6 +93,8 @@ static void finish_graph(Ctx &ctx, DGraph &g, bool validate) {
     g.total_vw = s.sum[0];
     if (g.total_vw > INT32_MAX) throw HpError{HP_ERR_GRAPH, "total vertex weight exceeds the 32-bit range"};
     g.m = g.cap;
+    g.row_ew = g.ew ? (u64) s.sum[1] : g.m;
+    g.all_ew = g.ew ? (u64) s.sum[2] : g.m;
 }
 
 DGraph graph_upload(Ctx &ctx, u32 n, u64 m, const u32 *xadj, const u32 *adj, const s32 *ew, const s32 *vw) {
@@ -345,6 +378,8 @@ void graph_induced_all(Ctx &ctx, const DGraph &g, const u32 *part, u32 k, const 
         s.ew = P.ew = ctx.falloc<s32>(P.m);
         s.vw = P.vw = ctx.falloc<s32>(P.n);
         s.total_vw = (s64) hw[p];
+        s.row_ew = g.row_ew;
+        s.all_ew = g.all_ew;
         n_to_o[p] = P.n_to_o = ctx.falloc<u32>(P.n);
     }
     if (ebase > 0xFFFFFFFFull) throw HpError{HP_ERR_ARG, "induced subgraphs exceed 32-bit offsets"};

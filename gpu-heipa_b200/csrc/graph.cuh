@@ -23,6 +23,10 @@ struct DGraph {
     s32 *ew = nullptr;      // cap, or null for unit edge weights
     s32 *vw = nullptr;      // n, or null for unit vertex weights
     s64 total_vw = 0;
+    // upper bounds of the weight of a row and of all entries (~0: unknown);
+    // while a row's is below 2^32, none of its block connections is 0 modulo
+    // 2^32
+    u64 row_ew = ~0ull, all_ew = ~0ull;
 };
 
 __device__ __forceinline__ s32 g_ew(const DGraph &g, u64 j) { return g.ew ? __ldg(&g.ew[j]) : 1; }

@@ -2702,17 +2702,21 @@ constexpr u32 TEAM_BLOCK_MAX_N = 4096;
 constexpr u64 TEAM_ANY_DEG_M = 1ull << 21;
 constexpr u64 TEAM_MID_DEG_M = 1ull << 22, TEAM_MID_DEG = 128;
 
-template<bool HASH, bool MAP>
+template<int TAB, bool MAP>
 static const void *team_kernel_of(int team) {
-    return team == TEAM_BLOCK ? (const void *) k_jet_block<HASH, MAP>
-                              : (team == TEAM_CLUSTER ? (const void *) k_jet_team<TEAM_CLUSTER, HASH, MAP>
-                                                      : (const void *) k_jet_team<TEAM_GRID, HASH, MAP>);
+    return team == TEAM_BLOCK ? (const void *) k_jet_block<TAB, MAP>
+                              : (team == TEAM_CLUSTER ? (const void *) k_jet_team<TEAM_CLUSTER, TAB, MAP>
+                                                      : (const void *) k_jet_team<TEAM_GRID, TAB, MAP>);
 }
 
-static const void *team_kernel(int team, u32 k, bool promap) {
-    if (promap) return team_kernel_of<false, true>(team);
-    return k <= TEAM_DIRECT_K ? team_kernel_of<false, false>(team) : team_kernel_of<true, false>(team);
+// zero: connections of 0 can occur
+static const void *team_kernel(int team, u32 k, bool promap, bool zero) {
+    if (promap) return zero ? team_kernel_of<TAB_ZERO, true>(team) : team_kernel_of<TAB_DIRECT, true>(team);
+    if (k > TEAM_DIRECT_K) return team_kernel_of<TAB_HASH, false>(team);
+    return zero ? team_kernel_of<TAB_ZERO, false>(team) : team_kernel_of<TAB_DIRECT, false>(team);
 }
+
+static bool zero_sums(const DGraph &g) { return g.row_ew >> 32 != 0; }
 
 // Per device, once: shared-memory and cluster-size limits of the team
 // kernels; returns the largest cluster that the device can run with the
@@ -2724,15 +2728,15 @@ static u32 team_limits(int device) {
     for (const auto &d: done)
         if (d.first == device) return d.second;
     u32 best = TEAM_CLUSTER_MAX;
-    for (int i = 0; i < 3; ++i) {
-        const bool promap = i == 2;
+    for (int i = 0; i < 5; ++i) {
+        const bool promap = i >= 3, zero = i == 2 || i == 4;
         const u32 k = i == 0 ? JW_SLOTS : 256;
-        const void *kc = team_kernel(TEAM_CLUSTER, k, promap), *kg = team_kernel(TEAM_GRID, k, promap);
+        const void *kc = team_kernel(TEAM_CLUSTER, k, promap, zero), *kg = team_kernel(TEAM_GRID, k, promap, zero);
         const size_t sc = team_smem(k, TEAM_CLUSTER_THREADS / 32, promap);
         const size_t sg = team_smem(k, TEAM_GRID_THREADS / 32, promap);
         HP_CUDA(cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sg));
-        HP_CUDA(cudaFuncSetAttribute(team_kernel(TEAM_BLOCK, k, promap), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int) TEAM_SMEM_MAX));
+        HP_CUDA(cudaFuncSetAttribute(team_kernel(TEAM_BLOCK, k, promap, zero),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int) TEAM_SMEM_MAX));
         best = team_cluster_limit(kc, sc, best);
     }
     done.emplace_back(device, best);
@@ -2776,7 +2780,7 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
     ctl.obj = obj;
     ctl.maxw = maxw;
     std::optional<CoopGuard> coop;  // cooperative budget (grid blocks), until the kernel has completed
-    const void *kern = team_kernel(team, k, promap);
+    const void *kern = team_kernel(team, k, promap, zero_sums(g));
     cudaLaunchAttribute attr;
     if (team == TEAM_BLOCK) {
         a.out = ctx.balloc<TeamOut>(1);
@@ -2839,14 +2843,14 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
     if (proj.ms) *proj.ms += (double) o.setup_ns * 1e-6;
 }
 
-// Blocks of the cooperative level loop for a level of n vertices and m
-// entries (0 when it does not apply): one per Tunables::jet_coop_rows vertices
+// Blocks of the cooperative level loop of a level (0 when it does not apply): one per Tunables::jet_coop_rows vertices
 // or 16 times as many entries. 512 rows against 1024 / 2048 (one B200): ultra
 // R-MAT 65k 222 / 229 / 253 ms, RGG 200k 20.5 / 20.7 / 21.8 ms.
-static u32 coop_blocks(const Ctx &ctx, u32 n, u64 m, u32 k, bool promap) {
+static u32 coop_blocks(const Ctx &ctx, const DGraph &g, u32 k, bool promap) {
     const u64 rows = std::max<u32>(1, ctx.tune.jet_coop_rows);
-    return team_grid_blocks(ctx, team_kernel(TEAM_GRID, k, promap), team_smem(k, TEAM_GRID_THREADS / 32, promap),
-                            (std::max<u64>(n, m / 16) + rows - 1) / rows);
+    return team_grid_blocks(ctx, team_kernel(TEAM_GRID, k, promap, zero_sums(g)),
+                            team_smem(k, TEAM_GRID_THREADS / 32, promap),
+                            (std::max<u64>(g.n, g.m / 16) + rows - 1) / rows);
 }
 
 __global__ void k_project(const u32 *coarse_part, const u32 *map, u32 *fine_part, u32 n) {
@@ -2900,7 +2904,7 @@ void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultr
         } else if (g.n <= ctx.tune.jet_coop_max_n && g.m <= ctx.tune.jet_coop_max_m &&
                    (g.m <= (u64) ctx.tune.jet_coop_max_deg * g.n || g.m <= TEAM_ANY_DEG_M ||
                     (g.m <= TEAM_MID_DEG_M && g.m <= TEAM_MID_DEG * g.n))) {
-            blocks = coop_blocks(ctx, g.n, g.m, k, promap);
+            blocks = coop_blocks(ctx, g, k, promap);
         }
         if (blocks) {
             ScratchScope ss2(ctx.arena);

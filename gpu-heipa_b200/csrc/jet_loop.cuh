@@ -40,6 +40,17 @@
 // 280 us (largest two) before, now 67 us (all).
 #pragma once
 
+// Rows of up to TEAM_ZERO_ROW entries take a block whose connection is 0 for a
+// neighbour, longer ones don't (nor do the per-kernel passes, which keep
+// short rows in registers). 16 weights add up to 0 modulo 2^32 only if one of
+// them is 2^28 or more, or below 1 (a coarse weight that wrapped): weight - 1
+// then has one of the bits from TEAM_ZERO_BIT on.
+constexpr u32 TEAM_ZERO_ROW = JT;
+constexpr u32 TEAM_ZERO_BIT = 27;
+// Tables of rows of up to 32 entries: direct-indexed, direct-indexed with that
+// rule (for graphs whose rows can weigh 2^32 or more, DGraph::row_ew: looking
+// for such weights costs the others 2%), or hashed, where the rule is free.
+enum TeamTable { TAB_DIRECT = 0, TAB_ZERO = 1, TAB_HASH = 2 };
 constexpr u32 TEAM_HUB = 1024;         // rows above this length are evaluated by a whole block
 constexpr u32 TEAM_LONG = 64;          // afterburner / delta rows above this length take a whole warp ...
 constexpr u32 TEAM_SHARE = 256;        // ... and above this one the warps of the block, 128 entries at a time
@@ -275,13 +286,14 @@ __device__ __forceinline__ u32 label_of(const TeamArgs &a, u32 v) { return ((con
 
 // Evaluates the rows of the lanes in `need` (beg, len <= 32, own block o of
 // each lane's row), four rows at a time, 8 lanes per row; every lane receives
-// its row's result. HASH: 64 slots of (block + 1, connection) per row instead
+// its row's result. TAB_HASH: 64 slots of (block + 1, connection) per row instead
 // of a direct-indexed table; both are all zero between rows. All lanes of the
 // warp call this.
-template<int TEAM, int OP, bool HASH>
+template<int TEAM, int OP, int TAB>
 __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u32 need, u32 beg, u32 len, u32 o,
                                            s32 max_b_w, RowOut &out) {
     constexpr int NG = 4, GL = 8;
+    constexpr bool HASH = TAB == TAB_HASH;
     const u32 lane = lane_id(), g = lane / GL, gl = lane % GL;
     s32 *tv = S.tab + g * (HASH ? 128 : a.k);
     while (need) {
@@ -304,6 +316,11 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
             b[j] = t < rl ? ld_graph<TEAM>(&a.adj[(u64) rb + t]) : EMPTY;
             w[j] = t < rl ? ld_ew<TEAM>(a, (u64) rb + t) : 0;
         }
+        u32 bits = 0;
+        if (TAB == TAB_ZERO)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (b[j] != EMPTY) bits |= (u32) w[j] - 1u;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
             if (b[j] != EMPTY) b[j] = label_of(a, b[j]);
@@ -330,15 +347,34 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
         // clears the table; of a hashed table it takes the key, because a
         // connection can be 0 (weights are added modulo 2^32) and a key that
         // stayed behind would fill the table for the rows that follow
+        bool rep[4];  // the entry stands for its block
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (!HASH) {
                 w[j] = b[j] != EMPTY ? atomicExch(&tv[at[j]], 0) : 0;
+                rep[j] = w[j] != 0;
             } else {
-                const bool first = b[j] != EMPTY && atomicExch(&tv[at[j] - 64], 0) != 0;
-                w[j] = first ? tv[at[j]] : 0;
-                if (first) tv[at[j]] = 0;
+                rep[j] = b[j] != EMPTY && atomicExch(&tv[at[j] - 64], 0) != 0;
+                w[j] = rep[j] ? tv[at[j]] : 0;
+                if (rep[j]) tv[at[j]] = 0;
+                rep[j] = rep[j] && (w[j] != 0 || rl <= TEAM_ZERO_ROW);
             }
+        }
+        if (TAB == TAB_ZERO && __any_sync(FULL, bits >> TEAM_ZERO_BIT)) {
+            // the blocks with a connection are marked, and of
+            // the others the first exchange stands for its block
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (rep[j]) tv[at[j]] = 1;
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (b[j] != EMPTY && !rep[j] && rl <= TEAM_ZERO_ROW) rep[j] = atomicExch(&tv[at[j]], 1) == 0;
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (b[j] != EMPTY) tv[at[j]] = 0;
         }
         __syncwarp();
         RowOut r{0, 0, 0, 0};
@@ -347,8 +383,8 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
             u32 cnt = 0;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const u32 mask = (__ballot_sync(FULL, w[j] != 0) >> (g * GL)) & 0xFFu;
-                if (w[j] != 0) list[cnt + __popc(mask & ((1u << gl) - 1u))] = ((unsigned long long) b[j] << 32) | (u32) w[j];
+                const u32 mask = (__ballot_sync(FULL, rep[j]) >> (g * GL)) & 0xFFu;
+                if (rep[j]) list[cnt + __popc(mask & ((1u << gl) - 1u))] = ((unsigned long long) b[j] << 32) | (u32) w[j];
                 cnt += __popc(mask);
             }
             __syncwarp();
@@ -357,7 +393,7 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
         } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (w[j] != 0) row_take<OP>(S, ro, max_b_w, b[j], w[j], r);
+                if (rep[j]) row_take<OP>(S, ro, max_b_w, b[j], w[j], r);
         }
         row_reduce<OP, GL>(r);
         // back to the lanes that own the rows
@@ -633,10 +669,10 @@ __device__ __forceinline__ s32 team_load_bw(const TeamArgs &a, const TeamSm &S, 
         if (!team_barrier<TEAM>(a.bar, bar_target, &a.out->err)) return;     \
     } while (0)
 
-// The level loop of one team of gridDim.x blocks. HASH: hashed tables for
-// short rows (k > TEAM_DIRECT_K).
+// The level loop of one team of gridDim.x blocks. TAB: tables of short rows
+// (TeamTable; hashed above TEAM_DIRECT_K blocks).
 // MAP: process-mapping objective.
-template<int TEAM, bool HASH, bool MAP>
+template<int TEAM, int TAB, bool MAP>
 __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl, const TeamSm &S) {
     __shared__ long long sl[33];
     __shared__ u32 su[33], su2[33];
@@ -734,7 +770,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                     if (need && !small) ld_row<TEAM>(a, u, beg, len);
                     const bool hb = need && len > TEAM_HUB;
                     RowOut r{0, 0, 0, 0};
-                    rows_short<TEAM, OP, HASH>(a, S, __ballot_sync(FULL, need && len <= 32), beg, len, o, 0, r);
+                    rows_short<TEAM, OP, TAB>(a, S, __ballot_sync(FULL, need && len <= 32), beg, len, o, 0, r);
                     rows_long<TEAM, OP>(a, S, __ballot_sync(FULL, need && len > 32 && !hb), beg, len, o, 0, r);
                     if (need && !hb) {
                         lp_decide<MAP>(r, ratio, dest, gain);
@@ -953,10 +989,10 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                     const u32 ms = __ballot_sync(FULL, need && len <= 32);
                     const u32 mg = __ballot_sync(FULL, need && len > 32 && !hb);
                     if (strong) {
-                        rows_short<TEAM, OP_STRONG, HASH>(a, S, ms, beg, len, o, max_b_w, r);
+                        rows_short<TEAM, OP_STRONG, TAB>(a, S, ms, beg, len, o, max_b_w, r);
                         rows_long<TEAM, OP_STRONG>(a, S, mg, beg, len, o, max_b_w, r);
                     } else {
-                        rows_short<TEAM, OP_WEAK, HASH>(a, S, ms, beg, len, o, max_b_w, r);
+                        rows_short<TEAM, OP_WEAK, TAB>(a, S, ms, beg, len, o, max_b_w, r);
                         rows_long<TEAM, OP_WEAK>(a, S, mg, beg, len, o, max_b_w, r);
                     }
                     u32 key = NOKEY;
@@ -1424,17 +1460,17 @@ __device__ __forceinline__ TeamSm team_setup(const TeamArgs &a, unsigned char *d
 }
 
 // A cluster or a cooperative grid on a level in global memory.
-template<int TEAM, bool HASH, bool MAP>
+template<int TEAM, int TAB, bool MAP>
 __global__ void __launch_bounds__(1024, 1) k_jet_team(const __grid_constant__ TeamArgs a,
                                                         const __grid_constant__ TeamCtl ctl) {
     extern __shared__ __align__(16) unsigned char team_dsm[];
     const TeamSm S = team_setup<MAP>(a, team_dsm);
-    team_loop<TEAM, HASH, MAP>(a, ctl, S);
+    team_loop<TEAM, TAB, MAP>(a, ctl, S);
 }
 
 // One block that copies the level to shared memory first (rows made
 // contiguous). `level` is the offset of the level's arrays.
-template<bool HASH, bool MAP>
+template<int TAB, bool MAP>
 __global__ void __launch_bounds__(512, 1) k_jet_block(const __grid_constant__ TeamArgs ga,
                                                         const __grid_constant__ TeamCtl ctl, u32 m, u32 level) {
     extern __shared__ __align__(16) unsigned char team_dsm[];
@@ -1507,7 +1543,7 @@ __global__ void __launch_bounds__(512, 1) k_jet_block(const __grid_constant__ Te
     a.adj = adj;
     a.ew = ew;
     a.vw = vw;
-    team_loop<TEAM_BLOCK, HASH, MAP>(a, ctl, S);
+    team_loop<TEAM_BLOCK, TAB, MAP>(a, ctl, S);
     if (tid == 0) {
         ga.out->obj = out->obj;
         ga.out->maxw = out->maxw;

@@ -66,6 +66,7 @@ CoarsenStep coarsen_level(Ctx &ctx, const DGraph &g, u32 *mp, DGraph &c, u32 &nc
         c = DGraph{};
         c.cap = g.m;
         c.total_vw = g.total_vw;
+        c.all_ew = g.all_ew;
         // Small levels keep the row bounds where the kernel writes them, sized
         // for n (12 n bytes more, instead of three copies of a few
         // microseconds each); larger ones copy them to arrays of the coarse size.
@@ -136,6 +137,7 @@ void coarsen(Ctx &ctx, const DGraph &g, u32 k, Hierarchy &H, SolveStats *stats) 
             c = contract_graph(ctx, cur, mp, nc);
             if (stats) stats->contraction_ms += ms_since(t1);
         }
+        c.row_ew = std::min<u64>(cur.row_ew < ~0ull / 2 ? 2 * cur.row_ew : ~0ull, cur.all_ew);  // pairs at most
         H.graphs.push_back(c);
         H.maps.push_back(mp);
     }

@@ -178,3 +178,20 @@ def test_gains_at_the_ends_of_the_range(reach, k, team):
         got, want = refine_both(g, k, part, lmax, TEAMS["grid" if team == "grid" else "cluster"])
         assert got[1:] == want[1:]
         np.testing.assert_array_equal(got[0], want[0])
+
+
+@pytest.mark.parametrize("team", ["block", "cluster", "grid"])
+@pytest.mark.parametrize("kind", ["k40", "k300", "map"])
+@pytest.mark.parametrize("reach", [2, 5, 8, 9])
+def test_short_rows_with_blocks_of_connection_zero(reach, kind, team):
+    # rows of up to 16 entries take a block whose weights add up to 0 for a neighbour, longer ones don't
+    n = 300 if team == "block" else 6000
+    k, hd = {"k40": (40, None), "k300": (300, None), "map": (24, ([2, 4, 3], [1, 10, 100]))}[kind]
+    g = circulant(n, reach, np.full(reach, 1 << 30))
+    part = (np.arange(n) * k // n).astype(np.uint32)
+    part[::11] = part[::-11][:len(part[::11])]
+    maxw = int(np.bincount(part, minlength=k).max())
+    for lmax in (n // k + 1, maxw, 2 * maxw):
+        got, want = refine_both(g, k, part, lmax, TEAMS["grid" if team == "grid" else "cluster"], hd)
+        assert got[1:] == want[1:]
+        np.testing.assert_array_equal(got[0], want[0])
