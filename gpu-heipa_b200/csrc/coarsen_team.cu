@@ -91,7 +91,9 @@ struct Best {
 };
 
 // Heaviest eligible neighbour, ties by xorshift (pick_neighbor :102-188); the
-// shift values of different neighbours differ.
+// shift values of different neighbours differ. Coarse weights are sums modulo
+// 2^32: rows of up to THREAD_DEG_MAX entries start from weight 0 and never take
+// a negative one, longer ones take any but the smallest (as matching.cu).
 template<bool INITIAL>
 struct PickOp {
     u32 seed;
@@ -99,9 +101,10 @@ struct PickOp {
     __device__ __forceinline__ u32 gather(const CoarsenArgs &a, u32 v) const {
         return INITIAL ? SENTINEL : __ldcg(&a.vcmap[v]);
     }
-    __device__ __forceinline__ void add(Best &s, u32 u, u32 v, s32 w, u32 x) const {
-        if (x < RECEIVER) return;  // matched
-        const unsigned long long key = ((unsigned long long) (u32) w << 32) | xorshift32(v + xorshift32(u ^ seed));
+    __device__ __forceinline__ void add(Best &s, u32 u, u32 len, u32 v, s32 w, u32 x) const {
+        if (x < RECEIVER || w < (len <= THREAD_DEG_MAX ? 0 : -INT32_MAX)) return;  // matched, or too light
+        const unsigned long long key =
+            ((unsigned long long) ((u32) w ^ 0x80000000u) << 32) | xorshift32(v + xorshift32(u ^ seed));
         if (key > s.key) s = Best{key, v};
     }
     __device__ __forceinline__ void merge(Best &s, const Best &y) const {
@@ -113,7 +116,7 @@ struct PickOp {
 struct TwinOp {
     __device__ __forceinline__ Best init() const { return Best{0, 0}; }
     __device__ __forceinline__ u32 gather(const CoarsenArgs &, u32) const { return 0; }
-    __device__ __forceinline__ void add(Best &s, u32, u32 v, s32, u32) const {
+    __device__ __forceinline__ void add(Best &s, u32, u32, u32 v, s32, u32) const {
         const unsigned long long y = murmur3_u32(v);
         s.key += y * y + y;
     }
@@ -124,7 +127,7 @@ struct TwinOp {
 struct RelOp {
     __device__ __forceinline__ Best init() const { return Best{~0ull, SENTINEL}; }
     __device__ __forceinline__ u32 gather(const CoarsenArgs &a, u32 v) const { return __ldg(&a.rowlen[v]); }
-    __device__ __forceinline__ void add(Best &s, u32, u32 v, s32 w, u32 d) const {
+    __device__ __forceinline__ void add(Best &s, u32, u32, u32 v, s32 w, u32 d) const {
         merge(s, Best{((unsigned long long) d << 32) | (u32) (INT32_MAX - w), v});
     }
     __device__ __forceinline__ void merge(Best &s, const Best &y) const {
@@ -150,7 +153,7 @@ __device__ __forceinline__ Best row_share(const CoarsenArgs &a, const Op &op, u3
         for (int j = 0; j < 4; ++j) x[j] = v[j] != SENTINEL ? op.gather(a, v[j]) : 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (v[j] != SENTINEL) op.add(s, u, v[j], w[j], x[j]);
+            if (v[j] != SENTINEL) op.add(s, u, len, v[j], w[j], x[j]);
     }
     return s;
 }

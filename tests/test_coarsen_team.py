@@ -94,3 +94,33 @@ def test_long_coarse_rows_take_the_contraction_kernels():
     want, want_cut = O.partition(to_oracle(g), 8, 0.03, False, 5)
     assert cut == want_cut
     np.testing.assert_array_equal(part, want)
+
+
+def wrapped_coarse_graph(n, deg, seed):
+    """A graph and the mapping that pairs its vertices: the 1 to 4 entries between two pairs weigh up to 2^30 each, so
+    coarse weights are sums below and above 2^31, 2^31 itself and 0 modulo 2^32."""
+    rng = np.random.default_rng(seed)
+    ring = [rng.permutation(n) for _ in range(deg // 2)]  # all degrees on one side of 16: neighbours see an edge alike
+    a = np.concatenate([np.stack([p, np.roll(p, 1)], 1) for p in ring])
+    e = np.concatenate([2 * a + np.array(x) for x in ((0, 0), (0, 1), (1, 0), (1, 1))])
+    e = e[rng.random(len(e)) < 0.8]
+    g = from_edges(2 * n, e, 1)
+    rows = np.repeat(np.arange(g.n), np.diff(g.xadj.astype(np.int64)))
+    key = np.minimum(rows, g.adj) + np.maximum(rows, g.adj)
+    g.ew = np.array([1 << 30, 1 << 30, (1 << 29) + 1, 5, 1 << 30], np.int32)[key % 5]
+    return g, (np.arange(g.n) // 2).astype(np.uint32)
+
+
+@pytest.mark.parametrize("n,deg", [(700, 6), (700, 30), (9000, 12), (40000, 6), (40000, 26), (3000, 90)])
+def test_matching_of_weights_that_wrapped(n, deg):
+    g, mp = wrapped_coarse_graph(n, deg, n + deg)
+    out = []
+    for max_n in (1 << 20, 0):  # one launch, a launch per phase
+        with H.Context(0, 512 << 20) as c:
+            c.tune("match_coop_max_n", max_n)
+            dg = c.upload(g)
+            cg = c.contract(dg, mp, n)
+            assert (cg.download().ew < 0).any() and (cg.download().ew == 0).any()
+            out.append(c.match(cg))
+    assert out[0][1] == out[1][1]
+    np.testing.assert_array_equal(out[0][0], out[1][0])
