@@ -30,6 +30,7 @@ CANDIDATES = {
     "jet_coop_max_m": [1 << 21, 1 << 24, 1 << 27],
     "jet_coop_max_deg": [12, 24, 64],
     "jet_coop_rows": [256, 512, 1024],
+    "jet_rank_pairs": [14170, 56680, 226720],
     "jet_hub_deg": [256, 1024, 4096],
     "jet_hub_conn": [0, 1],
     "jet_hub_track_pct": [25, 50, 100],
@@ -40,7 +41,8 @@ CANDIDATES = {
 DEFAULTS = {"jet_graph_max_m": 1 << 24, "order_small_n": 16384, "match_coop_max_n": 1 << 20,
             "match_coop_max_m": 1 << 24, "jet_fused_max_n": 8192, "jet_fused_max_m": 1 << 18,
             "jet_coop_max_n": 1 << 24, "jet_coop_max_m": 1 << 27, "jet_coop_max_deg": 24, "jet_coop_rows": 512,
-            "jet_hub_deg": 1024, "jet_hub_conn": 1, "jet_hub_track_pct": 50, "jet_inval_all_pct": 5,
+            "jet_rank_pairs": 56680, "jet_hub_deg": 1024, "jet_hub_conn": 1, "jet_hub_track_pct": 50,
+            "jet_inval_all_pct": 5,
             "jet_vec_loads": 1, "jet_chunk_mode": 0}
 
 

@@ -136,6 +136,12 @@ struct Tunables {
     u64 jet_coop_max_m = 1ull << 27;   // ... and entries ...
     u32 jet_coop_max_deg = 24;         // ... and average degree (smaller levels also above it: jet.cu)
     u32 jet_coop_rows = 512;           // vertices per block of that grid
+    // Strong rebalancing ranks its evicted vertices in that loop while a warp
+    // compares at most this many pairs (16384 vertices on 148 blocks), else the
+    // per-kernel loop, which sorts, takes the level. Refining a 1M grid, k = 64,
+    // with 8000 / 16000 / 24000 / 32000 evictions a step: 4.0 / 4.9 / 7.0 / 9.9
+    // ms ranked, 4.5 to 4.9 ms when the level is left at once.
+    u32 jet_rank_pairs = 56680;
     u32 jet_hub_deg = 1024;            // Jet table passes: rows above this length are cut into chunks of it (64..4096)
     u32 jet_chunk_mode = 0;            // chunk kernels: 0 = 4 entries per lane, 1 = 8, 2 = bulk-copy staged rows
     u32 jet_hub_conn = 1;              // per-kernel Jet loop: keep hub-row connectivity up to date (1) or rescan (0)

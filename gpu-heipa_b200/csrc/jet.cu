@@ -2771,6 +2771,7 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
     a.code = promap ? D->code : nullptr;
     a.bitdist = promap ? D->bitdist : nullptr;
     a.inval_all_min = inval_all_min;
+    a.rank_pairs = ctx.tune.jet_rank_pairs;
     a.part = part;
     a.cpart = proj.coarse;
     a.cmap = proj.map;

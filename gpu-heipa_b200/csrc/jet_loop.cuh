@@ -57,9 +57,8 @@ constexpr u32 TEAM_SHARE = 256;        // ... and above this one the warps of th
 constexpr u32 TEAM_SHARE_MAX = 128;    // rows a block shares in one phase (others stay with their warp)
 constexpr u32 TEAM_DIRECT_K = 256;     // direct-indexed tables per 8 lanes up to this k, hashed ones above
 constexpr u32 TEAM_LIST = 128;         // distinct-block list slots per warp (mapping objective; at least k)
-constexpr u32 TEAM_RANK_MAX = 32768;   // evicted vertices ranked by counting; more are left to the per-kernel path
-
 constexpr u32 TEAM_OWN = 48;           // candidates / moves of a warp kept in shared memory up to this range
+static_assert(2 * TEAM_OWN >= 3 * 32, "the lists' space holds a tile of three words per thread");
 
 enum TeamCnt { TC_HUB = 0, TC_MOVES = 1, TC_FAIL = 2, TC_N = 4 };
 enum TeamSum { TS_MOVES = 0, TS_DELTA = 1, TS_N = 2 };  // (moves << 32) + their row entries; objective change
@@ -84,7 +83,7 @@ struct TeamOut {
     long long obj;   // best objective
     s32 maxw;        // its maximum block weight
     u32 iterations;
-    u32 gave_up;     // 1: more than TEAM_RANK_MAX evicted vertices in one step, nothing was decided
+    u32 gave_up;     // 1: too many evicted vertices in one step to rank (TeamArgs::rank_pairs), nothing was decided
     u32 err;         // DevErr bits
     u32 hubs;        // some row is longer than TEAM_HUB
     unsigned long long setup_ns;  // time of the set-up (projection, block weights) on block 0
@@ -104,6 +103,7 @@ struct TeamArgs {
     const u32 *code;
     const s32 *bitdist;
     unsigned long long inval_all_min;
+    u32 rank_pairs;             // pairs of evicted vertices that a warp compares at most
     u32 *part;                  // in: labels (unless projected); out: best labelling
     const u32 *cpart, *cmap;    // projection: labels of the coarse vertices, fine -> coarse map (or null)
     u32 *saved;                 // receives a copy of the input labels (or null)
@@ -135,7 +135,8 @@ struct TeamSm {
     s32 *tab0;     // the block's first table
     u32 stride;    // words between the tables of two warps
     unsigned long long *list;  // this warp's distinct-block list (mapping objective)
-    u32 *own;      // this warp's candidate and move lists (2 * TEAM_OWN)
+    u32 *own;      // this warp's candidate and move lists (2 * TEAM_OWN) ...
+    u32 *own0;     // ... and the block's first
     s32 *bw, *bd, *cutbase, *tot, *spill, *toff;
     u32 *under, *olist, *cutkey;
     long long *es, *pre;
@@ -190,7 +191,8 @@ __device__ __forceinline__ TeamSm team_carve(unsigned char *base, u32 k, u32 war
     S.cutkey = (u32 *) (p + 8 * k);
     S.code = (u32 *) (p + 9 * k);
     S.dist = p + 10 * k;
-    S.own = (u32 *) (S.dist + 32) + warp * 2 * TEAM_OWN;
+    S.own0 = (u32 *) (S.dist + 32);
+    S.own = S.own0 + warp * 2 * TEAM_OWN;
     return S;
 }
 
@@ -1226,7 +1228,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                 if (strong) {
                     TEAM_SYNC();
                     const u32 ns = ld_fresh<TEAM>(&cnt[TC_MOVES]);
-                    if (ns > TEAM_RANK_MAX) {
+                    if (TEAM != TEAM_BLOCK && (u64) ns * ns > (u64) a.rank_pairs * gwarps) {
                         if (blockIdx.x == 0 && tid == 0) a.out->gave_up = 1;
                         return;
                     }
@@ -1255,33 +1257,51 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                     if (tid == 0) S.es[0] = 0;
                     __syncthreads();
                     // exact prefix of each evicted vertex among its block's
-                    // and the first slot attempt (adjust_scores :560-584)
-                    // (8 lanes per vertex, or a warp when there are enough)
-                    const u32 lanes = ns <= gwarps ? 32 : 8, li = lane & (lanes - 1);
-                    const u32 each = 32 / lanes;
-                    for (u32 j0 = gw * each; j0 < ns; j0 += gwarps * each) {
-                        const u32 j = j0 + lane / lanes;
-                        const bool act = j < ns;
-                        unsigned long long comp = 0, ow = 0;
-                        if (act) {
-                            comp = a.mcomp[j];
-                            ow = a.mow[j];
+                    // and the first slot attempt (adjust_scores :560-584). A
+                    // warp ranks two vertices against tiles of all in shared
+                    // memory, because warps that read the list from L2
+                    // were bound by its bandwidth (8000 vertices, 148 blocks:
+                    // 211 us a step, now 46)
+                    u32 *const t_key = S.own0, *const t_u = t_key + blockDim.x;
+                    s32 *const t_vw = (s32 *) (t_u + blockDim.x);
+                    for (u32 j0 = 0; j0 < ns; j0 += 2 * gwarps) {
+                        unsigned long long comp[2], ow[2], low[2];
+                        s32 x[2] = {0, 0};
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            const u32 j = j0 + q * gwarps + gw;
+                            comp[q] = j < ns ? a.mcomp[j] : 0ull;
+                            ow[q] = j < ns ? a.mow[j] : 0ull;
+                            low[q] = (unsigned long long) ((u32) (ow[q] >> 32) * a.width + sft) << 32;
                         }
-                        const u32 o = (u32) (ow >> 32);
-                        s32 x = 0;
-                        if (act) {
-#pragma unroll 4
-                            for (u32 i = li; i < ns; i += lanes) {
-                                const unsigned long long ci = a.mcomp[i], wi = a.mow[i];
-                                if ((u32) (wi >> 32) == o && ci < comp) x += (s32) (u32) wi;
+                        for (u32 t0 = 0; t0 < ns; t0 += blockDim.x) {
+                            const u32 tn = min(ns - t0, blockDim.x);
+                            if (j0 == 0 || ns > blockDim.x) {
+                                __syncthreads();
+                                if (tid < tn) {
+                                    const unsigned long long c = a.mcomp[t0 + tid];
+                                    t_key[tid] = (u32) (c >> 32);
+                                    t_u[tid] = (u32) c;
+                                    t_vw[tid] = (s32) (u32) a.mow[t0 + tid];
+                                }
+                                __syncthreads();
+                            }
+                            for (u32 i = lane; i < tn; i += 32) {
+                                const unsigned long long c = ((unsigned long long) t_key[i] << 32) | t_u[i];
+                                const s32 vw = t_vw[i];
+#pragma unroll
+                                for (int q = 0; q < 2; ++q)  // keys of the same block that are smaller
+                                    if (c - low[q] < comp[q] - low[q]) x[q] += vw;
                             }
                         }
                         __syncwarp();
-                        for (u32 d = lanes / 2; d > 0; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
-                        if (act && li == 0) {
-                            const u32 u = (u32) comp;
-                            const s32 vw = (s32) (u32) ow;
-                            const long long tg = (long long) S.spill[o] + x + S.pre[o];
+#pragma unroll
+                        for (int q = 0; q < 2; ++q)
+                            for (int d = 16; d > 0; d >>= 1) x[q] += __shfl_xor_sync(FULL, x[q], d);
+                        if (lane < 2 && j0 + lane * gwarps + gw < ns) {
+                            const u32 u = (u32) (lane ? comp[1] : comp[0]), o = (u32) ((lane ? ow[1] : ow[0]) >> 32);
+                            const s32 vw = (s32) (u32) (lane ? ow[1] : ow[0]);
+                            const long long tg = (long long) S.spill[o] + (lane ? x[1] : x[0]) + S.pre[o];
                             const s32 id = chunk_of(S.es, k, tg);
                             const bool fits = id < (s32) k && (long long) (vw / 2) <= S.es[id + 1] - tg;
                             if (!fits && id < (s32) k) {

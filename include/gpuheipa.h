@@ -219,7 +219,10 @@ int hp_coop_slot_release(int device);
  * "jet_coop_max_deg" (likewise as one cooperative grid of 1024-thread blocks
  * for larger levels, up to this many vertices, entries and entries per vertex,
  * or denser up to fixed entry counts; 0 vertices = never), "jet_coop_rows"
- * (vertices per block of that grid),
+ * (vertices per block of that grid), "jet_rank_pairs" (that launch leaves a
+ * level to the per-kernel loop when a strong rebalancing step evicts so many
+ * vertices that ranking them takes more pairs per warp than this; levels that
+ * run in one block never do),
  * "jet_hub_deg" (Jet connectivity passes with k <= 256: rows longer than this
  * are split into chunks of this many entries, one warp each; 64..4096),
  * "jet_chunk_mode" (the Jet chunk kernels read row entries 4 (0) or 8 (1) per

@@ -195,3 +195,30 @@ def test_short_rows_with_blocks_of_connection_zero(reach, kind, team):
         got, want = refine_both(g, k, part, lmax, TEAMS["grid" if team == "grid" else "cluster"], hd)
         assert got[1:] == want[1:]
         np.testing.assert_array_equal(got[0], want[0])
+
+
+def alternating(n, k, over):
+    """Blocks that are in turn larger and smaller than the average, and a limit `over` vertices in all below it: after two
+    weak steps every second block is overloaded and strong rebalancing evicts about `over` vertices."""
+    sizes = np.full(k, n // k)
+    sizes[0::2] += n // k // 50
+    sizes[1::2] -= n // k // 50
+    return np.repeat(np.arange(k), sizes).astype(np.uint32), n // k - over // k
+
+
+@pytest.mark.parametrize("team,tunes", [("cluster", TEAMS["cluster"]), ("grid", TEAMS["grid"]),
+                                        ("two_blocks", dict(TEAMS["grid"], jet_coop_rows=1 << 20))])
+@pytest.mark.parametrize("over", [120, 512, 516, 1020, 1024, 1032, 3000])
+def test_ranks_of_evicted_vertices(over, team, tunes):
+    # below, at and above a tile (512 or 1024 vertices), and several rounds of a warp's two vertices
+    g, k = H.Graph.grid(200, 120), 4
+    part, lmax = alternating(g.n, k, over)
+    og = to_oracle(g)
+    cut, maxw = O.edge_cut(og, part), int(np.bincount(part).max())
+    want = O.jet_refine(og, k, lmax, False, 0, part, cut, maxw)
+    with H.Context(0, 256 << 20) as c:
+        for name, v in tunes.items():
+            c.tune(name, v)
+        got = c.jet_refine(c.upload(g), k, lmax, part, cut, maxw)
+    assert got[1:] == want[1:]
+    np.testing.assert_array_equal(got[0], want[0])
