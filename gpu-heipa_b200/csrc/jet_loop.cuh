@@ -331,13 +331,17 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
         for (int j = 0; j < 4; ++j) {
             at[j] = b[j];
             if (HASH && b[j] != EMPTY) {  // at most 32 keys in 64 slots
-                u32 h = (b[j] * 2654435761u) >> 26, probe = 0;
-                for (; probe < 64; ++probe) {
+                const u32 h0 = (b[j] * 2654435761u) >> 26;
+                u32 h = h0;
+                for (;;) {
                     const u32 prev = atomicCAS((u32 *) &tv[h], 0u, b[j] + 1);
                     if (prev == 0 || prev == b[j] + 1) break;
                     h = (h + 1) & 63u;
+                    if (h == h0) {  // all slots seen
+                        set_error(&a.out->err, DEV_ERR_HASH_FULL);
+                        break;
+                    }
                 }
-                if (probe == 64) set_error(&a.out->err, DEV_ERR_HASH_FULL);
                 at[j] = 64 + h;
             }
         }
@@ -356,8 +360,9 @@ __device__ __forceinline__ void rows_short(const TeamArgs &a, const TeamSm &S, u
                 w[j] = b[j] != EMPTY ? atomicExch(&tv[at[j]], 0) : 0;
                 rep[j] = w[j] != 0;
             } else {
+                // (only the entry that takes the key uses what it read)
+                if (b[j] != EMPTY) w[j] = tv[at[j]];
                 rep[j] = b[j] != EMPTY && atomicExch(&tv[at[j] - 64], 0) != 0;
-                w[j] = rep[j] ? tv[at[j]] : 0;
                 if (rep[j]) tv[at[j]] = 0;
                 rep[j] = rep[j] && (w[j] != 0 || rl <= TEAM_ZERO_ROW);
             }
