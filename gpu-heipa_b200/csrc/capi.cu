@@ -676,6 +676,7 @@ int hp_tune(hp_ctx *ctx, const char *name, int64_t value) {
     else if (nm == "jet_coop_max_deg") t.jet_coop_max_deg = (uint32_t) std::min<int64_t>(value, 0xFFFFFFFFll);
     else if (nm == "jet_coop_rows") t.jet_coop_rows = (uint32_t) std::min<int64_t>(value, 0xFFFFFFFFll);
     else if (nm == "jet_rank_pairs") t.jet_rank_pairs = (uint32_t) std::min<int64_t>(value, 0xFFFFFFFFll);
+    else if (nm == "team_give_up" && value <= 3) t.team_give_up = (uint32_t) value;
     else if (nm == "jet_hub_deg") t.jet_hub_deg = (uint32_t) std::min<int64_t>(value, 0xFFFFFFFFll);
     else if (nm == "jet_chunk_mode" && value <= 2) t.jet_chunk_mode = (uint32_t) value;
     else if (nm == "jet_hub_conn" && value <= 1) t.jet_hub_conn = (uint32_t) value;

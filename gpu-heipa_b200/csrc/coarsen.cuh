@@ -8,7 +8,8 @@ namespace hp {
 // with the deterministic commit rule (smallest proposer wins a receiver) and
 // digest grouping by exact value for the leaf/twin/relative passes. Writes the
 // fine->coarse map (device, n entries) and returns the coarse vertex count.
-u32 match_graph(Ctx &ctx, const DGraph &g, u32 *mapping);
+// one_launch: try the single launch below first, where it applies.
+u32 match_graph(Ctx &ctx, const DGraph &g, u32 *mapping, bool one_launch = true);
 
 // from_Graph_Mapping (src/datastructures/graph.h:127-390): coarse vertex
 // weights are summed members, coarse edges aggregate all fine edges between

@@ -966,7 +966,7 @@ CoarsenResult coarsen_team(Ctx &ctx, const DGraph &g, u32 *mapping, DGraph *rows
     HP_CUDA(cudaMemcpyAsync(ctx.h_status, a.out, sizeof(CoarsenOut), cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();
     const CoarsenOut o = *(const CoarsenOut *) ctx.h_status;
-    if (o.err & DEV_ERR_SPIN) throw CoopSpin{};
+    if ((o.err & DEV_ERR_SPIN) || (ctx.tune.team_give_up & 1u)) throw CoopSpin{};
     if (o.err) throw HpError{HP_ERR_DEVICE, "matching or contraction reported error bits " + std::to_string(o.err)};
     r.contract_ms = (double) o.contract_ns * 1e-6;
     r.n = o.n;

@@ -142,6 +142,7 @@ struct Tunables {
     // with 8000 / 16000 / 24000 / 32000 evictions a step: 4.0 / 4.9 / 7.0 / 9.9
     // ms ranked, 4.5 to 4.9 ms when the level is left at once.
     u32 jet_rank_pairs = 56680;
+    u32 team_give_up = 0;              // diagnostic: finished launches of 1 coarsening, 2 refinement count as given up
     u32 jet_hub_deg = 1024;            // Jet table passes: rows above this length are cut into chunks of it (64..4096)
     u32 jet_chunk_mode = 0;            // chunk kernels: 0 = 4 entries per lane, 1 = 8, 2 = bulk-copy staged rows
     u32 jet_hub_conn = 1;              // per-kernel Jet loop: keep hub-row connectivity up to date (1) or rescan (0)

@@ -2837,7 +2837,7 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
     HP_CUDA(cudaMemcpyAsync(ctx.h_status, a.out, sizeof(TeamOut), cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();
     const TeamOut o = *(const TeamOut *) ctx.h_status;
-    if ((o.err & DEV_ERR_SPIN) || o.gave_up) throw CoopSpin{};
+    if ((o.err & DEV_ERR_SPIN) || o.gave_up || (team != TEAM_BLOCK && (ctx.tune.team_give_up & 2u))) throw CoopSpin{};
     if (o.err) throw HpError{HP_ERR_DEVICE, "Jet kernel reported error bits " + std::to_string(o.err)};
     obj = o.obj;
     maxw = o.maxw;

@@ -501,10 +501,10 @@ static u32 match_graph_phases(Ctx &ctx, const DGraph &g, u32 *mapping) {
     return ctx.read_status().cnt[0];
 }
 
-u32 match_graph(Ctx &ctx, const DGraph &g, u32 *mapping) {
+u32 match_graph(Ctx &ctx, const DGraph &g, u32 *mapping, bool one_launch) {
     if (g.n == 0) return 0;
     ProfScope prof_all(ctx, "match");
-    if (coarsen_team_applies(ctx, g)) {
+    if (one_launch && coarsen_team_applies(ctx, g)) {
         // small levels: one launch (matching is a deterministic function of
         // the graph, so the phases give the same mapping)
         try {

@@ -49,12 +49,13 @@ struct Hierarchy {
 
 constexpr u32 COARSEN_DIRECT_MAX_N = 1u << 16;
 
-enum class CoarsenStep { None, Matched, Contracted };
+enum class CoarsenStep { None, GaveUp, Matched, Contracted };
 
 // One level by the single-launch kernel, where it applies: the mapping and
 // coarse size (Matched), and the coarse graph in the front of the arena
 // (Contracted) unless the level shrinks by less than 1%. None: nothing was
-// done (level too large, no room for its scratch, or the launch gave up).
+// done (level too large, or no room for its scratch). GaveUp: nor was anything
+// after a launch whose blocks waited in vain, which is not made again.
 CoarsenStep coarsen_level(Ctx &ctx, const DGraph &g, u32 *mp, DGraph &c, u32 &nc, SolveStats *stats) {
     if (!coarsen_team_applies(ctx, g)) return CoarsenStep::None;
     ProfScope prof(ctx, "coarsen_level");
@@ -102,7 +103,7 @@ CoarsenStep coarsen_level(Ctx &ctx, const DGraph &g, u32 *mp, DGraph &c, u32 &nc
         }
     } catch (const CoopSpin &) {
         ctx.arena.front_release(mark);
-        return CoarsenStep::None;
+        return CoarsenStep::GaveUp;
     } catch (const HpError &e) {
         if (e.code != HP_ERR_OOM) throw;
         ctx.arena.front_release(mark);
@@ -127,8 +128,8 @@ void coarsen(Ctx &ctx, const DGraph &g, u32 k, Hierarchy &H, SolveStats *stats) 
         DGraph c;
         u32 nc = 0;
         const CoarsenStep step = coarsen_level(ctx, cur, mp, c, nc, stats);
-        if (step == CoarsenStep::None) {
-            nc = match_graph(ctx, cur, mp);
+        if (step == CoarsenStep::None || step == CoarsenStep::GaveUp) {
+            nc = match_graph(ctx, cur, mp, step == CoarsenStep::None);
             if (stats) stats->coarsening_ms += ms_since(t0);
         }
         if ((u64) nc * 100 > (u64) cur.n * 99) break;

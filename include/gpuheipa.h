@@ -222,7 +222,9 @@ int hp_coop_slot_release(int device);
  * (vertices per block of that grid), "jet_rank_pairs" (that launch leaves a
  * level to the per-kernel loop when a strong rebalancing step evicts so many
  * vertices that ranking them takes more pairs per warp than this; levels that
- * run in one block never do),
+ * run in one block never do), "team_give_up" (diagnostic: a finished launch of
+ * a coarsening level (1), of a refinement loop in more than one block (2) or of
+ * either (3) is treated as one that gave up; 0),
  * "jet_hub_deg" (Jet connectivity passes with k <= 256: rows longer than this
  * are split into chunks of this many entries, one warp each; 64..4096),
  * "jet_chunk_mode" (the Jet chunk kernels read row entries 4 (0) or 8 (1) per
