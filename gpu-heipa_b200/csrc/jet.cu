@@ -1325,7 +1325,7 @@ __device__ __forceinline__ void strong_finish(const JArgs &a, const RbArgs &r, u
     if (count == 0) count = 1;
     const s32 gain = wsub(sum / count, own);
     const s32 vw = g_vw(a.g, u);
-    const s32 excess = a.bw[o] - a.lmax;
+    const s32 excess = wsub(a.bw[o], a.lmax);  // of 32 bits, as the reference's (:404-442)
     r.keys[u] = (MAX_BUCKETS * o + gain_bucket(gain, vw < excess ? vw : excess)) * r.sections + (u % r.sections) + 1;
 }
 

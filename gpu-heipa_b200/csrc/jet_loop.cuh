@@ -956,7 +956,7 @@ __device__ __forceinline__ void team_loop(const TeamArgs &a, const TeamCtl &ctl,
                 auto finish = [&](u32 u, u32 o, s32 vw, const RowOut &r) -> u32 {
                     if (strong) {
                         const s32 gain = wsub(r.sum / (r.count ? r.count : 1), r.own);
-                        const s32 excess = S.bw[o] - a.lmax;
+                        const s32 excess = wsub(S.bw[o], a.lmax);  // of 32 bits, as the reference's
                         return (MAX_BUCKETS * o + gain_bucket(gain, vw < excess ? vw : excess)) * a.sections +
                                (u % a.sections) + 1;
                     }

@@ -807,7 +807,7 @@ std::vector<u32> rebalance_strong(Jet &J) {
             }
             if (count == 0) count = 1;
             s32 gn = wsub(sum / count, own);
-            u32 gt = gain_bucket(gn, std::min<s32>(vw, ow - lmax));
+            u32 gt = gain_bucket(gn, std::min<s32>(vw, wsub(ow, lmax)));
             keyv[u] = (MAX_BUCKETS * o + gt) * sections + (u % sections) + 1;
             is_cand[u] = 1;
         }

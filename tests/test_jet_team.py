@@ -80,9 +80,15 @@ def test_team_loop_equals_oracle(name, start, team):
         c.close()
 
 
-@pytest.mark.parametrize("lmax", [-2 ** 30, -1, 0])
-def test_limits_that_no_block_can_meet(lmax):
-    # every block is overloaded by its whole weight or more
+LOOPS = {"block": {}, "cluster": {"jet_coop_max_n": 0}, "grid": TEAMS["grid"],
+         "kernels": {"jet_fused_max_n": 0, "jet_coop_max_n": 0}}
+
+
+@pytest.mark.parametrize("loop", sorted(LOOPS))
+@pytest.mark.parametrize("lmax", [-2147483000, -2 ** 30, -1, 0])
+def test_limits_that_no_block_can_meet(lmax, loop):
+    # every block is overloaded by its whole weight or more; block weights of about 3000 less the first limit exceed 31
+    # bits: the weight to evict is a 64-bit difference, the one in the bucket key (as in the reference) a 32-bit one
     g, k = weighted(H.Graph.grid(31, 29, 1, 5, seed=3), 7), 6
     og = to_oracle(g)
     part = np.random.default_rng(3).integers(0, k, g.n).astype(np.uint32)
@@ -90,6 +96,8 @@ def test_limits_that_no_block_can_meet(lmax):
     cut = O.edge_cut(og, part)
     want = O.jet_refine(og, k, lmax, False, 0, part, cut, maxw)
     with H.Context(0, 64 << 20) as c:
+        for name, v in LOOPS[loop].items():
+            c.tune(name, v)
         got = c.jet_refine(c.upload(g), k, lmax, part, cut, maxw)
     assert got[1:] == want[1:]
     np.testing.assert_array_equal(got[0], want[0])
