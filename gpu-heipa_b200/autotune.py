@@ -26,6 +26,7 @@ CANDIDATES = {
     "match_coop_max_m": [0, 1 << 20, 1 << 22, 1 << 24],
     "jet_fused_max_n": [0, 2048, 4096, 8192],
     "jet_fused_max_m": [1 << 16, 1 << 18, 1 << 20],
+    "jet_block_max_n": [0, 1024, 4096],
     "jet_coop_max_n": [0, 65536, 1 << 20, 1 << 24],
     "jet_coop_max_m": [1 << 21, 1 << 24, 1 << 27],
     "jet_coop_max_deg": [12, 24, 64],
@@ -39,11 +40,10 @@ CANDIDATES = {
     "jet_chunk_mode": [0, 1],
 }
 DEFAULTS = {"jet_graph_max_m": 1 << 24, "order_small_n": 16384, "match_coop_max_n": 1 << 20,
-            "match_coop_max_m": 1 << 24, "jet_fused_max_n": 8192, "jet_fused_max_m": 1 << 18,
+            "match_coop_max_m": 1 << 24, "jet_fused_max_n": 8192, "jet_fused_max_m": 1 << 18, "jet_block_max_n": 4096,
             "jet_coop_max_n": 1 << 24, "jet_coop_max_m": 1 << 27, "jet_coop_max_deg": 24, "jet_coop_rows": 512,
             "jet_rank_pairs": 56680, "jet_hub_deg": 1024, "jet_hub_conn": 1, "jet_hub_track_pct": 50,
-            "jet_inval_all_pct": 5,
-            "jet_vec_loads": 1, "jet_chunk_mode": 0}
+            "jet_inval_all_pct": 5, "jet_vec_loads": 1, "jet_chunk_mode": 0}
 
 
 def _time(ctx, graphs, ks, config, seed, repeats):

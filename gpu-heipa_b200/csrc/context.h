@@ -132,6 +132,10 @@ struct Tunables {
     u64 match_coop_max_m = 1ull << 24; // ... and entries
     u32 jet_fused_max_n = 8192;        // whole Jet level loop in one thread-block cluster up to this many vertices ...
     u64 jet_fused_max_m = 1ull << 18;  // ... and entries
+    // ... of these, in one block where its shared memory holds the level (up to
+    // 3700 vertices). The cluster took 14.7 us per iteration on the levels of up
+    // to 1700 vertices of an RGG with 3001 vertices, one block 10.5 us.
+    u32 jet_block_max_n = 4096;
     u32 jet_coop_max_n = 1u << 24;     // ... else as a cooperative grid up to this many vertices ...
     u64 jet_coop_max_m = 1ull << 27;   // ... and entries ...
     u32 jet_coop_max_deg = 24;         // ... and average degree (smaller levels also above it: jet.cu)

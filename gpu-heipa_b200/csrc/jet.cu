@@ -2686,10 +2686,6 @@ void JetLevel::run_step(int kind, u32 ratio_pct) {
 // vertices per block of a cluster team (up to its largest size): 4 rows per warp
 constexpr u32 TEAM_CLUSTER_ROWS = 64;
 constexpr u32 TEAM_CLUSTER_MAX_N = 1u << 16;  // upper bound of Tunables::jet_fused_max_n
-// Block teams: what fits in shared memory. The cluster took 14.7 us per
-// iteration on the levels of up to 1700 vertices of an RGG with 3001 vertices,
-// one block with the level in shared memory 10.5 us.
-constexpr u32 TEAM_BLOCK_MAX_N = 4096;
 // Levels above Tunables::jet_coop_max_deg entries per vertex run as a grid
 // team up to these sizes. Barriers dominate small levels whatever their
 // degree (ultra R-MAT 65k, levels of up to 600 entries per vertex: 302 ms with
@@ -2895,7 +2891,7 @@ void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultr
         sections_of(g.n, k, sections, width);
         const bool fused = g.n <= std::min<u32>(ctx.tune.jet_fused_max_n, TEAM_CLUSTER_MAX_N) &&
                            g.m <= ctx.tune.jet_fused_max_m;
-        if (fused && g.n <= TEAM_BLOCK_MAX_N &&
+        if (fused && g.n <= ctx.tune.jet_block_max_n &&
             team_level_offset(k, promap) + team_level_smem(g.n, g.m, k, width) <= TEAM_SMEM_MAX) {
             team = TEAM_BLOCK;
             blocks = 1;

@@ -215,7 +215,9 @@ int hp_coop_slot_release(int device);
  * vertices capped at 1048576; 0 = never), "jet_fused_max_n" / "jet_fused_max_m" (the whole refinement loop
  * of a level in one launch of a thread-block cluster up to these sizes,
  * vertices capped at 65536, when k <= 1024, or k <= 256 for the mapping
- * objective; 0 = never), "jet_coop_max_n" / "jet_coop_max_m" /
+ * objective; 0 = never), "jet_block_max_n" (of these, in one block up to this
+ * many vertices, at most 4096, where shared memory holds the level; 0 = never),
+ * "jet_coop_max_n" / "jet_coop_max_m" /
  * "jet_coop_max_deg" (likewise as one cooperative grid of 1024-thread blocks
  * for larger levels, up to this many vertices, entries and entries per vertex,
  * or denser up to fixed entry counts; 0 vertices = never), "jet_coop_rows"

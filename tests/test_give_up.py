@@ -7,7 +7,7 @@ import pytest
 import gpu_heipa as H
 import oracle as O
 from helpers import to_oracle
-from test_jet_team import alternating
+from test_jet_team import TEAMS, alternating
 
 pytestmark = pytest.mark.gpu
 
@@ -50,7 +50,7 @@ LOOP = ("k_lp_dispatch", "k_weak_pick", "k_strong_pick")  # passes of the per-ke
 @pytest.mark.parametrize("config", ["default", "ultra"])
 def test_levels_that_are_redone_in_a_partition(config, team, why):
     # the start labels are projected again
-    tunes = {"jet_fused_max_n": 65536, "jet_fused_max_m": 1 << 30} if team == "cluster" else {"jet_fused_max_n": 0}
+    tunes = dict(TEAMS["cluster"]) if team == "cluster" else {"jet_fused_max_n": 0}
     for g, k in ((RMAT, 48), (MESH, 300)):
         want = O.partition(to_oracle(g), k, 0.03, config == "ultra", 5)
         part, cut, names = solve(g, k, config, **tunes, **GIVE_UP[why])
@@ -83,7 +83,8 @@ def test_level_that_is_redone_in_a_refinement(team, why):
         c.tune("jet_graph_max_m", 0)
         for name, v in GIVE_UP[why].items():
             c.tune(name, v)
-        c.tune("jet_fused_max_n", 65536 if team == "cluster" else 0)
+        for name, v in TEAMS[team].items():
+            c.tune(name, v)
         dg = c.upload(g)
         c.instrument(True)
         got = c.jet_refine(dg, k, lmax, part, cut, maxw)

@@ -1,7 +1,9 @@
-"""The single-launch Jet level loop (cluster and cooperative-grid teams) against the oracle at the sizes where it can go
-wrong: levels of one to a few vertices, row lengths around the tiers (8 lanes x 4 entries, a warp, 64-entry and 1024-entry
-limits), block counts around the table layouts (256 / 257, 1024), several mini-buckets per gain bucket, one overloaded
-block, and evictions that need fallback slots. Integer results: equality."""
+"""The single-launch Jet level loop (block, cluster and cooperative-grid teams) against the oracle at the sizes where it
+can go wrong: levels of one to a few vertices, row lengths around the tiers (8 lanes x 4 entries, a warp, 64-entry and
+1024-entry limits), block counts around the table layouts (256 / 257, 1024), several mini-buckets per gain bucket, one
+overloaded block, evictions that need fallback slots, and more of them than a tile of the ranking holds. Weights whose
+sums wrap are compared with the per-kernel loop (the oracle's rules for connections of 0 or less differ). Integer results:
+equality."""
 import numpy as np
 import pytest
 
@@ -11,7 +13,9 @@ from helpers import isolated_plus_path, star, to_oracle
 
 pytestmark = pytest.mark.gpu
 
-TEAMS = {"cluster": {"jet_fused_max_n": 65536, "jet_fused_max_m": 1 << 30, "jet_coop_max_n": 0},
+# block: levels that fit its shared memory run in one block, larger ones as a cluster
+TEAMS = {"block": {"jet_fused_max_n": 65536, "jet_fused_max_m": 1 << 30, "jet_coop_max_n": 0},
+         "cluster": {"jet_fused_max_n": 65536, "jet_fused_max_m": 1 << 30, "jet_coop_max_n": 0, "jet_block_max_n": 0},
          "grid": {"jet_fused_max_n": 0, "jet_coop_max_n": 1 << 24, "jet_coop_max_deg": 1 << 20, "jet_coop_rows": 64}}
 
 
@@ -80,8 +84,7 @@ def test_team_loop_equals_oracle(name, start, team):
         c.close()
 
 
-LOOPS = {"block": {}, "cluster": {"jet_coop_max_n": 0}, "grid": TEAMS["grid"],
-         "kernels": {"jet_fused_max_n": 0, "jet_coop_max_n": 0}}
+LOOPS = dict(TEAMS, kernels={"jet_fused_max_n": 0, "jet_coop_max_n": 0})
 
 
 @pytest.mark.parametrize("loop", sorted(LOOPS))
@@ -145,7 +148,7 @@ def refine_both(g, k, part, lmax, tunes, hd=None, ultra=False):
 
 # team -> (vertices, blocks, settings): cluster and grid levels on few warps, so that the rows of a table meet more blocks
 # with connection 0 than the table has slots
-HASHED = {"block": (300, 257, TEAMS["cluster"]), "cluster": (40000, 1000, TEAMS["cluster"]),
+HASHED = {"block": (300, 257, TEAMS["block"]), "cluster": (40000, 1000, TEAMS["cluster"]),
           "grid": (24000, 1000, dict(TEAMS["grid"], jet_coop_rows=1 << 20))}
 
 
@@ -183,7 +186,7 @@ def test_gains_at_the_ends_of_the_range(reach, k, team):
     part[::37] = (part[::37] + 1) % k
     maxw = int(np.bincount(part).max())
     for lmax in (maxw, 2 * maxw):
-        got, want = refine_both(g, k, part, lmax, TEAMS["grid" if team == "grid" else "cluster"])
+        got, want = refine_both(g, k, part, lmax, TEAMS[team])
         assert got[1:] == want[1:]
         np.testing.assert_array_equal(got[0], want[0])
 
@@ -200,7 +203,7 @@ def test_short_rows_with_blocks_of_connection_zero(reach, kind, team):
     part[::11] = part[::-11][:len(part[::11])]
     maxw = int(np.bincount(part, minlength=k).max())
     for lmax in (n // k + 1, maxw, 2 * maxw):
-        got, want = refine_both(g, k, part, lmax, TEAMS["grid" if team == "grid" else "cluster"], hd)
+        got, want = refine_both(g, k, part, lmax, TEAMS[team], hd)
         assert got[1:] == want[1:]
         np.testing.assert_array_equal(got[0], want[0])
 
@@ -228,5 +231,24 @@ def test_ranks_of_evicted_vertices(over, team, tunes):
         for name, v in tunes.items():
             c.tune(name, v)
         got = c.jet_refine(c.upload(g), k, lmax, part, cut, maxw)
+    assert got[1:] == want[1:]
+    np.testing.assert_array_equal(got[0], want[0])
+
+
+@pytest.mark.parametrize("kind", ["cut", "map"])
+@pytest.mark.parametrize("tunes", [TEAMS["cluster"], dict(TEAMS["grid"], jet_coop_rows=1 << 20)], ids=["cluster", "grid"])
+def test_more_long_rows_than_a_block_shares(tunes, kind):
+    # 3000 rows of 300 entries in at most 16 blocks: more than 128 of them in each
+    g, k = circulant(3000, 150, np.arange(150) % 7 + 1), 24
+    og = to_oracle(g)
+    hier, dist = ([2, 4, 3], [1, 10, 100]) if kind == "map" else (None, None)
+    part = np.random.default_rng(8).integers(0, k, g.n).astype(np.uint32)
+    obj = O.comm_cost(og, part, hier, dist) if hier else O.edge_cut(og, part)
+    maxw, lmax = int(np.bincount(part).max()), 140
+    want = O.jet_refine(og, k, lmax, False, 0, part, obj, maxw, hier, dist)
+    with H.Context(0, 256 << 20) as c:
+        for name, v in tunes.items():
+            c.tune(name, v)
+        got = c.jet_refine(c.upload(g), k, lmax, part, obj, maxw, hierarchy=hier, distance=dist)
     assert got[1:] == want[1:]
     np.testing.assert_array_equal(got[0], want[0])
