@@ -2742,9 +2742,9 @@ static u32 team_limits(int device) {
 // Offset of a block team's level arrays in its shared memory.
 static size_t team_level_offset(u32 k, bool promap) { return team_smem(k, TEAM_BLOCK_THREADS / 32, promap); }
 
-// Runs the level loop in one launch (direct-indexed tables): part receives
-// the best labelling. `saved` receives the input labels (cluster and grid
-// teams). Throws CoopSpin when the loop gave up (barrier wait, or too many
+// Runs the level loop in one launch (tables of short rows: TeamTable): part
+// receives the best labelling. `saved` receives the input labels (cluster and
+// grid teams). Throws CoopSpin when the loop gave up (barrier wait, or too many
 // evictions to rank); part is then to be restored from saved.
 static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const std::vector<u32> &ratios,
                             const DistOracle *D, unsigned long long inval_all_min, u32 *part, u32 *saved, s64 &obj,
@@ -2784,7 +2784,7 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
         HP_CUDA(cudaMemsetAsync(a.out, 0, sizeof(TeamOut), ctx.stream));
         u32 m = (u32) g.m, level = (u32) team_level_offset(k, promap);
         const size_t smem = level + team_level_smem(n, m, k, a.width);
-        KernTimer kt(ctx, "k_jet_fused");
+        KernTimer kt(ctx, "k_jet_block");
         const cudaLaunchConfig_t cfg = team_config(1, TEAM_BLOCK_THREADS, smem, ctx.stream, attr, team);
         void *args[] = {&a, &ctl, &m, &level};
         HP_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
@@ -2822,7 +2822,7 @@ static void jet_refine_team(Ctx &ctx, const DGraph &g, u32 k, s32 lmax, const st
         const u32 threads = team_threads(team);
         const size_t smem = team_smem(k, threads / 32, promap);
         if (team == TEAM_GRID) coop.emplace(ctx.device, ctx.stream, blocks, (u32) ctx.sm_count);
-        KernTimer kt(ctx, team == TEAM_CLUSTER ? "k_jet_fused" : "k_jet_coop");
+        KernTimer kt(ctx, team == TEAM_CLUSTER ? "k_jet_team_cluster" : "k_jet_team_grid");
         const cudaLaunchConfig_t cfg = team_config(blocks, threads, smem, ctx.stream, attr, team);
         void *args[] = {&a, &ctl};
         HP_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
@@ -2911,8 +2911,8 @@ void jet_refine(Ctx &ctx, const DGraph &g, u32 *part, u32 k, s32 lmax, bool ultr
                 jet_refine_team(ctx, g, k, lmax, ratios, D, inval, part, saved, obj, maxw, team, blocks, proj);
                 return;
             } catch (const CoopSpin &) {
-                // (a block team ranks all it has) the per-kernel loop redoes
-                // the level from its input labels
+                // (a block team ranks all it has and waits for no other block)
+                // the per-kernel loop redoes the level from its input labels
                 if (!proj.map)
                     HP_CUDA(cudaMemcpyAsync(part, saved, sizeof(u32) * g.n, cudaMemcpyDeviceToDevice, ctx.stream));
                 ctx.sync();  // saved is released here

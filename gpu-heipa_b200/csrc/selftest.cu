@@ -1,11 +1,12 @@
 // Diagnostics of the bounded waits (hp_selftest_barrier_timeout, declared in
-// include/gpuheipa.h). The cooperative level loops wait for one another at
-// grid barriers whose wait is bounded (team_barrier, team.cuh): when a
-// block does not arrive, the others give up after about a second, set an
-// error bit and end, and the host reports an error instead of hanging. This
-// entry point exercises exactly that path with a block that never arrives, so
-// a test can check that the wait ends, that the error bit is reported, and
-// that the device stays usable afterwards. No fault, trap or endless loop is
+// include/gpuheipa.h). The blocks of the cooperative level loops wait for one
+// another at grid barriers whose wait is bounded (team_barrier, team.cuh): when
+// a block does not arrive, the others give up after about a second, set an
+// error bit and end, and the host redoes the level with a launch per phase
+// instead of hanging. This entry point exercises the wait with a block that
+// never arrives, so a test can check that it ends, that the error bit reaches
+// the host, and that the device stays usable afterwards (the host's part is
+// tested with the tunable team_give_up). No fault, trap or endless loop is
 // involved.
 #include "../../include/gpuheipa.h"
 #include "common.cuh"

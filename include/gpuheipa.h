@@ -169,7 +169,10 @@ int hp_map_graph(hp_ctx *ctx, const hp_graph *g, const uint32_t *hier, const int
                  double imbalance, int mode, uint64_t seed, uint32_t *part, int64_t *J);
 
 /* Phase timings (ms) of the last solve on ctx: coarsening, contraction,
- * initial partitioning, uncontraction, refinement (solver.h:319-328 keys). */
+ * initial partitioning, uncontraction, refinement (solver.h:319-328 keys).
+ * Levels that are refined in one launch project inside it: their part of
+ * uncontraction is the set-up of that launch (projection, cache resets and
+ * block weights). */
 int hp_last_solve_stats(const hp_ctx *ctx, double *phase_ms5, int64_t *initial_obj, int32_t *lmax,
                         uint32_t *levels);
 /* Maximum block weight after initial partitioning and at the end of the last
@@ -263,7 +266,9 @@ int hp_event_record(hp_ctx *ctx, int slot);
 int hp_event_elapsed(hp_ctx *ctx, int slot_a, int slot_b, float *ms);
 /* Kernels launched by this process so far. */
 uint64_t hp_kernel_launches(void);
-/* Diagnostic phase timers (synchronising; off by default). hp_profile resets
+/* Diagnostic phase timers (synchronising; off by default). While they are on,
+ * every level is refined by the per-kernel loop, so that its phases can be
+ * told apart (the kernel timers show the single launches). hp_profile resets
  * them; hp_profile_entry enumerates (name, total ms, count) by index and
  * returns HP_ERR_ARG past the last entry. */
 int hp_profile(hp_ctx *ctx, int enable);

@@ -5,9 +5,9 @@ The failure is made on the device without any fault: one block of a
 cooperative launch simply returns before the barrier (a flag that nothing
 sets), so the others' bounded wait runs out.
 
-Cooperative launches take a per-device slot first (one such grid at a time),
-so concurrent solves whose level loops all run as full-device cooperative
-grids never wait for each other's SMs.
+Cooperative launches take blocks of a per-device budget first (as many as the
+device has SMs; a larger grid takes all of it), so concurrent solves whose level
+loops all run as cooperative grids never wait for each other's SMs.
 """
 import threading
 import time
